@@ -9,11 +9,12 @@
 //                     the cell's output blocks and writes one ColumnSet record
 //                     per transverse pair plus the source permutation.
 //
-//   remap_walk_kernel (the default, fused arithmetic) or remap_kernel (the
-//                     exact mode): persistent; each half-warp takes one
-//                     ColumnSet and walks it along the sweep dimension, one
-//                     lane per transverse cell (i,j) of the 4x4 block face.
-//                     The reconstruction is built in registers from a sliding
+//   remap_pair_kernel (fused arithmetic, PPM and PLM), remap_walk_kernel
+//                     (fused, PQM) or remap_kernel (the exact mode):
+//                     persistent; eight lanes (pair) or a half-warp take one
+//                     ColumnSet and walk it along the sweep dimension, two
+//                     columns or one of the 4x4 block face per lane.  The
+//                     reconstruction is built in registers from a sliding
 //                     window of the column; each source cell's mass goes to
 //                     the Lagrangian target cells it overlaps in a per-lane
 //                     ring of 8 target blocks in shared memory, and completed
@@ -26,6 +27,7 @@
 // of cpu_face_estimates.hpp:163 and cpu_acc_map.cpp:585), so its results are
 // bit-identical to the reference's map_1d on the same inputs.
 #include <cfloat>
+#include <cmath>
 #include <cstdint>
 
 #include "fused_ppm.cuh"
@@ -326,8 +328,7 @@ __device__ __forceinline__ void columnize_cell(
       if (sets_ok) {
          ColumnSet cs;
          cs.cell = cell;
-         cs.si = si;
-         cs.sj = sj;
+         cs.sij = si | (sj << 16);
          cs.src_pos = src.off + prefix[t];
          cs.dst_pos = 0;
          cs.src_mask[0] = m[0]; cs.src_mask[1] = m[1]; cs.src_mask[2] = m[2];
@@ -449,6 +450,29 @@ __device__ __forceinline__ int cell_offset(int i, int j, int g) {
    return i + j * WID + g * WID2;
 }
 
+// How the workers of a remap launch (warps, half-warps) take the column sets.
+// A worker's first sets follow from its number, neighbours on different SMs;
+// only further ones come from the counter.  A launch with fewer sets than
+// workers touches no counter: taking every set from it made the 592 CTAs of
+// a one-cell sweep queue 9472 atomics on one address (15.3 us for 100 sets).
+struct SetClaims {
+   SweepCounters* counters;
+   uint32_t begin, n_sets, dynamic;  // the launch's first set, the end, the first set given out by the counter
+   __device__ __forceinline__ SetClaims(SweepCounters* c, uint32_t n) : counters(c), begin(c->first_set), n_sets(n), dynamic(n) {}
+   // worker w of the CTA's `workers`, `each` sets at a time
+   __device__ __forceinline__ uint32_t first(uint32_t w, uint32_t workers, uint32_t each) {
+      dynamic = begin + workers * gridDim.x * each;
+      return begin + (w * gridDim.x + blockIdx.x) * each;
+   }
+   // `leader` asks for the lanes of `mask` (aligned segments of `width` lanes)
+   __device__ __forceinline__ uint32_t next(bool leader, unsigned mask, int width, uint32_t each) {
+      if (dynamic >= n_sets) return n_sets;
+      uint32_t s = 0;
+      if (leader) s = dynamic + atomicAdd(&counters->work, each);
+      return __shfl_sync(mask, s, 0, width);
+   }
+};
+
 constexpr uint32_t NO_BLOCK = 0xffffffffu;  // a block that exists with all-zero data
 
 __device__ __forceinline__ int clampi(int x, int lo, int hi) { return x < lo ? lo : (x > hi ? hi : x); }
@@ -498,7 +522,7 @@ __device__ __forceinline__ void pass_through_set(const ColumnSet& cs, const uint
       const bool c = fmaxf(fmaxf(v[0], v[1]), fmaxf(v[2], v[3])) >= content_thr;
       const unsigned any_c = __ballot_sync(hmask, c) & hmask;
       if (lane == 0) {
-         dst_gids[o] = gid_from_swapped(cs.si, cs.sj, (uint32_t)k, mesh.len, DIM);
+         dst_gids[o] = gid_from_swapped(cs.si(), cs.sj(), (uint32_t)k, mesh.len, DIM);
          content_out[o] = any_c ? 1 : 0;
       }
    }
@@ -541,8 +565,9 @@ __global__ void __launch_bounds__(REMAP_THREADS, 3) remap_kernel(
    const unsigned hmask = 0xffffu << (threadIdx.x & 16);
    float* ring = ring_all + hw * RING_STRIDE;
    const int i = lane & 3, j = lane >> 2;
-   uint32_t n_sets = *((volatile uint32_t*)&counters->n_sets);
+   uint32_t n_sets = counters->n_sets;
    n_sets = (n_sets < set_capacity) ? n_sets : set_capacity;
+   SetClaims claims(counters, n_sets);
    const int max_len = (int)mesh.len[DIM];
    const float dv = mesh.dv[DIM], v_min = mesh.vmin[DIM];
    const double i_dv = 1.0 / (double)dv;
@@ -553,11 +578,8 @@ __global__ void __launch_bounds__(REMAP_THREADS, 3) remap_kernel(
    // zeroes the slots it reads, so the ring is empty again at each set start
 #pragma unroll
    for (int q = 0; q < RING_CELLS; ++q) ring[q * 16 + lane] = 0.0f;
-   for (;;) {
-      uint32_t sidx = 0;
-      if (lane == 0) sidx = atomicAdd(&counters->work, 1u);
-      sidx = __shfl_sync(hmask, sidx, 0, 16);
-      if (sidx >= n_sets) break;
+   for (uint32_t sidx = claims.first(hw, REMAP_THREADS / 16, 1u); sidx < n_sets;
+        sidx = claims.next(lane == 0, hmask, 16, 1u)) {
       const ColumnSet cs = sets[sidx];
       const SweepCell P = sweep_cells[cs.cell];
       if (P.flags & SWEEP_PASS) {
@@ -568,11 +590,11 @@ __global__ void __launch_bounds__(REMAP_THREADS, 3) remap_kernel(
       const float scale = __double2float_rn(1.0 / (double)threshold);
       const float dk = P.dk;
       // lane's Lagrangian starting point (cpu_acc_map.cpp:493-496)
-      const float A = fa((float)(cs.si * WID), (float)i);
-      const float B = fa((float)(cs.sj * WID), (float)j);
+      const float A = fa((float)(cs.si() * WID), (float)i);
+      const float B = fa((float)(cs.sj() * WID), (float)j);
       const float im = fa(fa(P.intersection, fm(A, P.di)), fm(B, P.dj));
       float mx, mn;
-      set_corners(P, cs.si, cs.sj, mx, mn);
+      set_corners(P, cs.si(), cs.sj(), mx, mn);
       int next_flush = mask_next_set(cs.tgt_mask, 0);
       uint32_t out_idx = 0;
       bool range_err = false;
@@ -594,7 +616,7 @@ __global__ void __launch_bounds__(REMAP_THREADS, 3) remap_kernel(
                            (v[3] >= content_thr);
             const unsigned any_c = __ballot_sync(hmask, c) & hmask;
             if (lane == 0) {
-               dst_gids[o] = gid_from_swapped(cs.si, cs.sj, (uint32_t)next_flush, mesh.len, DIM);
+               dst_gids[o] = gid_from_swapped(cs.si(), cs.sj(), (uint32_t)next_flush, mesh.len, DIM);
                content_out[o] = any_c ? 1 : 0;
             }
             ++out_idx;
@@ -709,18 +731,12 @@ __global__ void __launch_bounds__(REMAP_THREADS, 3) remap_kernel(
 }
 
 // ---------------------------------------------------------------------------
-// remap_walk: the fused arithmetic as a single-accumulator walk
+// remap_walk: the fused arithmetic as a single-accumulator walk (PQM)
 // ---------------------------------------------------------------------------
 // The same column sets, lanes, ring and flushes as remap_kernel, with the
-// reconstruction and the distribution of mass over the target cells reduced
-// to what the fused mode needs:
+// distribution of mass over the target cells reduced to what the fused mode
+// needs:
 //
-//  - PPM: each face's raw h4 value and its test "face outside the values of
-//    the two cells it separates" are evaluated once and used by both cells
-//    (the test of the left face of cell k, (v_{k-1} - f)(f - v_k) < 0, is the
-//    test of the right face of cell k-1 with the same rounded product); the two
-//    Colella-Woodward overshoot corrections are applied as alternatives (in
-//    exact arithmetic the second can no longer fire once the first has).
 //  - Distribution: each lane keeps one pending target g (the lowest target
 //    cell not yet complete), its accumulated mass and the position u of the
 //    target's right edge (g+1) dk + im relative to the current source cell,
@@ -741,8 +757,8 @@ __global__ void __launch_bounds__(REMAP_THREADS, 3) remap_kernel(
 //    which then receives all mass below its right edge, as in the reference;
 //    mass of targets above the column's highest cell is moved into it when
 //    the column ends.
-template <int DIM, int RECON>
-__global__ void __launch_bounds__(REMAP_THREADS, RECON == RECON_PQM ? 2 : 4) remap_walk_kernel(
+template <int DIM>
+__global__ void __launch_bounds__(REMAP_THREADS, 2) remap_walk_kernel(
    const ColumnSet* __restrict__ sets, SweepCounters* __restrict__ counters, const uint32_t* __restrict__ perm,
    const float* __restrict__ src_data, float* __restrict__ dst_data, uint32_t* __restrict__ dst_gids,
    const SweepCell* __restrict__ sweep_cells, uint32_t* __restrict__ status, MeshDev mesh, int wall_margin,
@@ -755,23 +771,20 @@ __global__ void __launch_bounds__(REMAP_THREADS, RECON == RECON_PQM ? 2 : 4) rem
    // that a target block's four cells are one 16-byte access
    float* ring = ring_all + (size_t)threadIdx.x * WALK_LANE_STRIDE;
    const int i = lane & 3, j = lane >> 2;
-   uint32_t n_sets = *((volatile uint32_t*)&counters->n_sets);
+   uint32_t n_sets = counters->n_sets;
    n_sets = (n_sets < set_capacity) ? n_sets : set_capacity;
+   SetClaims claims(counters, n_sets);
    const int max_len = (int)mesh.len[DIM];
    const float dv = mesh.dv[DIM], v_min = mesh.vmin[DIM];
    const float inv_dv = (float)(1.0 / (double)dv);
    const float content_thr = __double2float_ru(content_threshold);
-   constexpr float one_sixth = (float)(1.0 / 6.0);
    constexpr int RMASK = RING_CELLS - 1;
    constexpr uint32_t SMASK = RING_CELLS - 1;  // slot offsets wrap around the ring
 
 #pragma unroll
    for (int q = 0; q < RING_CELLS; ++q) ring[q] = 0.0f;
-   for (;;) {
-      uint32_t sidx = 0;
-      if (lane == 0) sidx = atomicAdd(&counters->work, 1u);
-      sidx = __shfl_sync(hmask, sidx, 0, 16);
-      if (sidx >= n_sets) break;
+   for (uint32_t sidx = claims.first(hw, REMAP_THREADS / 16, 1u); sidx < n_sets;
+        sidx = claims.next(lane == 0, hmask, 16, 1u)) {
       const ColumnSet cs = sets[sidx];
       const SweepCell P = sweep_cells[cs.cell];
       if (P.flags & SWEEP_PASS) {
@@ -779,13 +792,13 @@ __global__ void __launch_bounds__(REMAP_THREADS, RECON == RECON_PQM ? 2 : 4) rem
          continue;
       }
       const float dk = P.dk;
-      const float A = fa((float)(cs.si * WID), (float)i);
-      const float B = fa((float)(cs.sj * WID), (float)j);
+      const float A = fa((float)(cs.si() * WID), (float)i);
+      const float B = fa((float)(cs.sj() * WID), (float)j);
       const float im = fa(fa(P.intersection, fm(A, P.di)), fm(B, P.dj));
       float mx, mn;
-      set_corners(P, cs.si, cs.sj, mx, mn);
-      const uint32_t gid0 = gid_from_swapped(cs.si, cs.sj, 0u, mesh.len, DIM);
-      const uint32_t gid_step = gid_from_swapped(cs.si, cs.sj, 1u, mesh.len, DIM) - gid0;
+      set_corners(P, cs.si(), cs.sj(), mx, mn);
+      const uint32_t gid0 = gid_from_swapped(cs.si(), cs.sj(), 0u, mesh.len, DIM);
+      const uint32_t gid_step = gid_from_swapped(cs.si(), cs.sj(), 1u, mesh.len, DIM) - gid0;
       // the next target block to write and the end of the run of consecutive
       // target blocks it belongs to
       int next_flush = mask_next_set(cs.tgt_mask, 0);
@@ -864,17 +877,8 @@ __global__ void __launch_bounds__(REMAP_THREADS, RECON == RECON_PQM ? 2 : 4) rem
             nxt[0] = nxt[1] = nxt[2] = nxt[3] = 0.0f;
          }
          // face state of the column's first cell
-         float face = 0.0f, face_d = 0.0f;
-         bool face_out = false;  // PPM: the left face lies outside its two cells' values
-         float dprev = cur[0];   // v_k - v_{k-1}
-         if constexpr (RECON == RECON_PPM) {
-            face = h4_face_fused(0.0f, 0.0f, cur[0], cur[1]);
-            face_out = (0.0f - face) * (face - cur[0]) < 0.0f;
-         }
-         if constexpr (RECON == RECON_PQM) {
-            face = h8_value(0.0f, 0.0f, 0.0f, 0.0f, cur[0], cur[1], cur[2], cur[3]);
-            face_d = h7_derivative(0.0f, 0.0f, 0.0f, 0.0f, cur[0], cur[1], cur[2], cur[3]);
-         }
+         float face = h8_value(0.0f, 0.0f, 0.0f, 0.0f, cur[0], cur[1], cur[2], cur[3]);
+         float face_d = h7_derivative(0.0f, 0.0f, 0.0f, 0.0f, cur[0], cur[1], cur[2], cur[3]);
          for (int kb = col_s; kb <= col_e; ++kb) {
             float nn[4];
             if (kb + 2 <= col_e) {
@@ -886,46 +890,17 @@ __global__ void __launch_bounds__(REMAP_THREADS, RECON == RECON_PQM ? 2 : 4) rem
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                const float vm1 = w[q + 3], v0 = w[q + 4], vp1 = w[q + 5];
-               float a[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-               if constexpr (RECON == RECON_PPM) {
-                  const float fr = h4_face_fused(vm1, v0, vp1, w[q + 6]);
-                  const bool fr_out = (v0 - fr) * (fr - vp1) < 0.0f;
-                  const float dn = vp1 - v0;
-                  const bool same = dn * dprev > 0.0f;
-                  // superbee: max(min(|a|, 2|b|), min(2|a|, |b|)) = min(2 min(|a|,|b|), max(|a|,|b|))
-                  const float an = fabsf(dn), ap = fabsf(dprev);
-                  const float sl = fminf(2.0f * fminf(an, ap), fmaxf(an, ap));
-                  const float hs = copysignf(0.5f * sl, dn);
-                  float fl2 = face_out ? v0 - hs : face;
-                  float fr2 = fr_out ? v0 + hs : fr;
-                  fl2 = same ? fl2 : v0;
-                  fr2 = same ? fr2 : v0;
-                  const float d = fr2 - fl2;
-                  const float ev = fmaf(-0.5f, fl2 + fr2, v0);
-                  const float de = d * ev, dd = d * (d * one_sixth);
-                  const float v3 = 3.0f * v0;
-                  const float nfl = (de > dd) ? fmaf(-2.0f, fr2, v3) : fl2;
-                  const float nfr = (-dd > de) ? fmaf(-2.0f, fl2, v3) : fr2;
-                  a[0] = nfl;
-                  a[1] = fmaf(-2.0f, nfl, v3) - nfr;
-                  a[2] = fmaf(-2.0f, v0, nfl + nfr);
-                  face = fr;
-                  face_out = fr_out;
-                  dprev = dn;
-               } else if constexpr (RECON == RECON_PQM) {
-                  const float fr = h8_value(w[q + 1], w[q + 2], w[q + 3], w[q + 4], w[q + 5], w[q + 6], w[q + 7],
-                                            w[q + 8]);
-                  const float fdr = h7_derivative(w[q + 1], w[q + 2], w[q + 3], w[q + 4], w[q + 5], w[q + 6],
-                                                  w[q + 7], w[q + 8]);
-                  pqm_coeff_fused(vm1, v0, vp1, face, fr, face_d, fdr, a);
-                  face = fr;
-                  face_d = fdr;
-               } else {
-                  plm_coeff_fused(vm1, v0, vp1, a);
-               }
+               float a[5];
+               const float fr = h8_value(w[q + 1], w[q + 2], w[q + 3], w[q + 4], w[q + 5], w[q + 6], w[q + 7],
+                                         w[q + 8]);
+               const float fdr = h7_derivative(w[q + 1], w[q + 2], w[q + 3], w[q + 4], w[q + 5], w[q + 6], w[q + 7],
+                                               w[q + 8]);
+               pqm_coeff_fused(vm1, v0, vp1, face, fr, face_d, fdr, a);
+               face = fr;
+               face_d = fdr;
                // ---- distribute the cell over the lane's targets ----
                const bool has = u < 1.0f;  // the pending target's right edge lies inside this cell
-               float D = recon_integral<RECON>(u, a);  // used only when has
+               float D = pqm_integral(u, a);  // used only when has
                if (has) ring[soff] = D - nacc;
                nacc = (has ? D : nacc) - v0;
                {
@@ -938,7 +913,7 @@ __global__ void __launch_bounds__(REMAP_THREADS, RECON == RECON_PQM ? 2 : 4) rem
                if (u < 1.0f) {
                   // further edges inside the same source cell (dk < dv)
                   for (int guard = 0; u < 1.0f && guard < 8; ++guard) {
-                     const float D2 = recon_integral<RECON>(u, a);
+                     const float D2 = pqm_integral(u, a);
                      ring[soff] = D2 - D;
                      D = D2;
                      g1f += 1.0f;
@@ -1001,6 +976,493 @@ __global__ void __launch_bounds__(REMAP_THREADS, RECON == RECON_PQM ? 2 : 4) rem
          if (lane == 0) atomicOr(&status[cs.cell], VLGPU_CELL_RANGE);
 #pragma unroll
          for (int q = 0; q < RING_CELLS; ++q) ring[q] = 0.0f;
+      }
+   }
+}
+
+// ---------------------------------------------------------------------------
+// remap_pair: the fused arithmetic, two columns per lane
+// ---------------------------------------------------------------------------
+// The walk of remap_walk_kernel (pending target, edges, column limits, flushes)
+// with eight lanes per column set, four sets per warp, each lane walking two
+// neighbouring columns whose values sit side by side in float2 registers:
+//
+//  - The arithmetic of both columns is one packed f32x2 instruction; loads,
+//    stores and ring accesses move both columns' values at once, and the
+//    bookkeeping of a block and of a set (about 80 and 300 instructions) is
+//    shared by twice the cells.
+//  - The limiter works on magnitudes: with L = |v0 - left face|, R = |right
+//    face - v0| (a face outside the values of its two cells gives half the
+//    superbee slope h = min(|a|, |b|, max(|a|, |b|) / 2) instead) the
+//    Colella-Woodward corrections are L = min(L, 2R), R = min(R, 2L), and the
+//    reconstruction is v0 - s (L + u ((R - 2L) + u (L - R))) with s the sign of
+//    the slope, zero at an extremum.  v0 - face is the neighbour's value
+//    minus the same face for the cell on the other side, so it is carried.
+//    That takes 8 operations of the ALU pipe per cell where the selections of
+//    faces took 14.
+//  - The four sets of a warp walk in step (the loop count is the warp's), so
+//    every vote covers the whole warp.
+//  - The ring of target cells lies slot by slot in shared memory (a slot of
+//    all the CTA's lanes is contiguous): a lane's slot is always in its own
+//    banks, whatever slots the other lanes are at.
+//
+// Bound by issue and the ALU pipe (72% and 60% busy with 24 warps per SM, the
+// most the ring's 64 KB per CTA leave room for).  Measured on 4096 drifting
+// Maxwellian cells (5.8 M blocks): 1145 us per sweep, 2870 GB/s of 8 B per
+// cell, against 1415 us and 2321 GB/s with half a warp per set; 64 cells: 38
+// against 53 us; PLM on 1024 cells: 247 against 291 us.  Two CTAs per SM with
+// 100 registers take 17% longer, a loop over two blocks that loads a block
+// ahead 25% (instruction cache); prefetches to L2 change nothing.
+constexpr int PAIR_THREADS = 256;
+constexpr int PAIR_WARPS = PAIR_THREADS / 32;
+constexpr uint32_t PAIR_SLOT_BYTES = PAIR_THREADS * sizeof(float2);  // one ring slot of the CTA
+constexpr uint32_t PAIR_SLOT_MASK = (RING_CELLS - 1) * PAIR_SLOT_BYTES;
+// a b > 0 of two value differences as a factor 0 or 1: their scaled product,
+// saturated.  2^75 squared times the smallest denormal product is 1.
+constexpr float SAME_SCALE = 37778931862957161709568.0f;
+constexpr int PAIR_CTAS = 3;  // per SM: 72 to 80 registers, 192 KB of rings
+constexpr size_t PAIR_SMEM = (size_t)RING_CELLS * PAIR_SLOT_BYTES;
+
+// m >= 0 with the sign of a
+__device__ __forceinline__ float with_sign(float m, float a) {
+   return __uint_as_float(__float_as_uint(m) | (__float_as_uint(a) & 0x80000000u));
+}
+// y - x of two columns
+__device__ __forceinline__ float2 p_neg_add(float2 y, float2 x) { return __fadd2_rn(y, make_float2(-x.x, -x.y)); }
+
+// The lane's two columns of the block at `row`: cells g = 0..3 along the
+// sweep, .x and .y the two columns (zeros for a block without data).
+template <int DIM>
+__device__ __forceinline__ void load_pair(const float* __restrict__ lane_data, uint32_t row, float2 v[4]) {
+   const float* __restrict__ blk = lane_data + (size_t)row * WID3;
+   if (DIM == 0) {
+      float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a;
+      if (row != NO_BLOCK) {
+         a = __ldg(reinterpret_cast<const float4*>(blk));
+         b = __ldg(reinterpret_cast<const float4*>(blk) + 1);
+      }
+      v[0] = make_float2(a.x, b.x);
+      v[1] = make_float2(a.y, b.y);
+      v[2] = make_float2(a.z, b.z);
+      v[3] = make_float2(a.w, b.w);
+   } else {
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+         v[g] = make_float2(0.0f, 0.0f);
+         if (row != NO_BLOCK) v[g] = __ldg(reinterpret_cast<const float2*>(blk + g * (DIM == 1 ? WID : WID2)));
+      }
+   }
+}
+
+template <int DIM>
+__device__ __forceinline__ void store_pair(float* __restrict__ blk, const float2 v[4]) {
+   if (DIM == 0) {
+      reinterpret_cast<float4*>(blk)[0] = make_float4(v[0].x, v[1].x, v[2].x, v[3].x);
+      reinterpret_cast<float4*>(blk)[1] = make_float4(v[0].y, v[1].y, v[2].y, v[3].y);
+   } else {
+#pragma unroll
+      for (int g = 0; g < 4; ++g) *reinterpret_cast<float2*>(blk + g * (DIM == 1 ? WID : WID2)) = v[g];
+   }
+}
+
+// The set of a cell that is not accelerated in this step (pass_through_set)
+// by its eight lanes.
+template <int DIM>
+__device__ __forceinline__ void pass_through_pair(const ColumnSet& cs, const uint32_t* __restrict__ perm,
+                                                  const float* __restrict__ src_data, float* __restrict__ dst_data,
+                                                  uint32_t* __restrict__ dst_gids, uint8_t* __restrict__ content_out,
+                                                  const uint32_t len[3], float content_thr, int off, bool leader,
+                                                  unsigned omask) {
+   uint32_t r = 0;
+   for (int k = mask_next_set(cs.src_mask, 0); k < 96; k = mask_next_set(cs.src_mask, k + 1), ++r) {
+      float2 v[4];
+      load_pair<DIM>(src_data + off, perm[cs.src_pos + r], v);
+      const uint32_t o = cs.dst_pos + r;
+      store_pair<DIM>(dst_data + (size_t)o * WID3 + off, v);
+      bool c = false;
+#pragma unroll
+      for (int g = 0; g < 4; ++g) c |= fmaxf(v[g].x, v[g].y) >= content_thr;
+      const unsigned any_c = __ballot_sync(omask, c) & omask;
+      if (leader) {
+         dst_gids[o] = gid_from_swapped(cs.si(), cs.sj(), (uint32_t)k, len, DIM);
+         content_out[o] = any_c ? 1 : 0;
+      }
+   }
+}
+
+// First set bit of a mask (96: none) and first clear bit at or after k.
+__device__ __forceinline__ int mask_first(const uint32_t m[3]) {
+   return m[0] ? __ffs(m[0]) - 1 : (m[1] ? 31 + __ffs(m[1]) : (m[2] ? 63 + __ffs(m[2]) : 96));
+}
+__device__ __forceinline__ int mask_run_end(const uint32_t m[3], int k) {
+   uint32_t c[3];
+#pragma unroll
+   for (int w = 0; w < 3; ++w) {
+      const int s = k - 32 * w;  // bits of the word below k count as set
+      c[w] = ~m[w] & (s <= 0 ? 0xffffffffu : (s >= 32 ? 0u : 0xffffffffu << s));
+   }
+   return mask_first(c);
+}
+
+// What the sweep's kernels read of the mesh, in the walk's precision.
+struct PairMesh {
+   uint32_t len[3];
+   int wall_margin;
+   float dv, v_min, inv_dv;
+   float content_thr;  // the smallest float >= the threshold: v >= it exactly when (double)v >= the threshold
+};
+
+template <int DIM, int RECON>
+__global__ void __launch_bounds__(PAIR_THREADS, PAIR_CTAS) remap_pair_kernel(
+   const ColumnSet* __restrict__ sets, SweepCounters* __restrict__ counters, const uint32_t* __restrict__ perm,
+   const float* __restrict__ src_data, float* __restrict__ dst_data, uint32_t* __restrict__ dst_gids,
+   const SweepCell* __restrict__ sweep_cells, uint32_t* __restrict__ status, const PairMesh mesh,
+   uint32_t set_capacity, uint8_t* __restrict__ content_out) {
+   static_assert(RECON == RECON_PPM || RECON == RECON_PLM, "the quartic reconstruction runs in remap_walk_kernel");
+   extern __shared__ __align__(16) unsigned char pair_ring[];
+   constexpr unsigned FULL = 0xffffffffu;
+   const int lane = threadIdx.x & 31, l8 = threadIdx.x & 7;
+   const unsigned oshift = lane & 24;  // the octet's first lane
+   // the lane's columns (i0, j0) and its neighbour: i0 + 1, or j0 + 1 in the x
+   // sweep, whose columns are rows of the block along y
+   const int i0 = (DIM == 0) ? (l8 >> 1) : 2 * (l8 & 1);
+   const int j0 = (DIM == 0) ? 2 * (l8 & 1) : (l8 >> 1);
+   const int off = cell_offset<DIM>(i0, j0, 0);
+   // this lane's ring slot at byte s (target cell times PAIR_SLOT_BYTES, mod the ring)
+   const uint32_t lane_at = threadIdx.x * (uint32_t)sizeof(float2);
+   auto slot_x = [&](uint32_t s) -> float& {
+      return *reinterpret_cast<float*>(pair_ring + ((s & PAIR_SLOT_MASK) | lane_at));
+   };
+   auto slot_y = [&](uint32_t s) -> float& {
+      return *reinterpret_cast<float*>(pair_ring + ((s & PAIR_SLOT_MASK) | lane_at) + 4);
+   };
+   auto slot2 = [&](uint32_t s) -> float2& {
+      return *reinterpret_cast<float2*>(pair_ring + ((s & PAIR_SLOT_MASK) | lane_at));
+   };
+
+   uint32_t n_sets = counters->n_sets;
+   n_sets = (n_sets < set_capacity) ? n_sets : set_capacity;
+   SetClaims claims(counters, n_sets);
+   const float2 zero2 = make_float2(0.0f, 0.0f);
+
+   uint32_t base = claims.first(threadIdx.x >> 5, PAIR_WARPS, 4u);
+   if (base >= n_sets) return;
+#pragma unroll
+   for (int q = 0; q < RING_CELLS; ++q) slot2(q * PAIR_SLOT_BYTES) = zero2;
+   for (; base < n_sets; base = claims.next(lane == 0, FULL, 32, 4u)) {
+      const uint32_t sidx = base + (oshift >> 3);
+      float2 im = zero2;
+      float dk = 1.0f;
+      uint32_t out = 0, gid0 = 0, pos = 0;  // next output block; block ID of the set's k = 0; the set's first row
+      int n_src = 0;                        // source blocks to walk
+      int next_flush = 96, run_end = 96;    // next target block to write, end of its run of consecutive ones
+      // the current column: source blocks from this one on, highest target
+      // cell, and the next column's first target block (none: NO_COLUMN)
+      constexpr int NO_COLUMN = 1 << 20;
+      int left = 0, hi = 0, ncf = NO_COLUMN;
+      int kb = 0, lo = 0;  // first block and lowest target cell of the column about to start
+      if (sidx < n_sets) {
+         const ColumnSet cs = sets[sidx];
+         const SweepCell P = sweep_cells[cs.cell];
+         if (P.flags & SWEEP_PASS) {
+            pass_through_pair<DIM>(cs, perm, src_data, dst_data, dst_gids, content_out, mesh.len, mesh.content_thr, off,
+                                   l8 == 0, 0xffu << oshift);
+         } else {
+            dk = P.dk;
+            const float A0 = fa((float)(cs.si() * WID), (float)i0), B0 = fa((float)(cs.sj() * WID), (float)j0);
+            const float A1 = (DIM == 0) ? A0 : fa((float)(cs.si() * WID), (float)(i0 + 1));
+            const float B1 = (DIM == 0) ? fa((float)(cs.sj() * WID), (float)(j0 + 1)) : B0;
+            im.x = fa(fa(P.intersection, fm(A0, P.di)), fm(B0, P.dj));
+            im.y = fa(fa(P.intersection, fm(A1, P.di)), fm(B1, P.dj));
+            gid0 = gid_from_swapped(cs.si(), cs.sj(), 0u, mesh.len, DIM);
+            out = cs.dst_pos;
+            pos = cs.src_pos;
+            next_flush = mask_first(cs.tgt_mask);
+            run_end = mask_run_end(cs.tgt_mask, next_flush);
+            // a cell whose Lagrangian cells do not advance (flagged by
+            // columnize) gets its target blocks with zero values
+            if (dk > 0.0f) n_src = __popc(cs.src_mask[0]) + __popc(cs.src_mask[1]) + __popc(cs.src_mask[2]);
+            if (n_src > 0) {
+               kb = mask_first(cs.src_mask);
+               const int e = mask_run_end(cs.src_mask, kb);
+               left = e - kb;
+               if (left == n_src) {
+                  // one column: columnize marked exactly its targets
+                  lo = next_flush * WID;
+                  hi = run_end * WID - 1;
+               } else {
+                  float mx, mn;
+                  int cf, cl, ncl;
+                  set_corners(P, cs.si(), cs.sj(), mx, mn);
+                  column_extent(mx, mn, dk, mesh.dv, mesh.v_min, (int)mesh.len[DIM], kb, e - 1, mesh.wall_margin, cf, cl);
+                  lo = cf * WID;
+                  hi = (cl + 1) * WID - 1;
+                  const int s = mask_next_set(cs.src_mask, e);
+                  column_extent(mx, mn, dk, mesh.dv, mesh.v_min, (int)mesh.len[DIM], s,
+                                mask_run_end(cs.src_mask, s) - 1, mesh.wall_margin, ncf, ncl);
+               }
+            }
+         }
+      }
+      __syncwarp();
+      const int iters = __reduce_max_sync(FULL, n_src);
+      bool range_err = false;
+
+      // writes out the target blocks below `limit` that all the lanes of the
+      // octet have completed
+      auto flush = [&](int limit) {
+         limit = limit < 96 ? limit : 96;
+         for (;;) {
+            unsigned can = __ballot_sync(FULL, next_flush < limit);
+            can &= can >> 4;
+            can &= can >> 2;
+            can &= (can >> 1) & 0x01010101u;  // bit 8 q: all of octet q's lanes
+            if (can == 0u) break;
+            float2 v[4];
+            const uint32_t slot = (uint32_t)next_flush * (WID * PAIR_SLOT_BYTES);
+#pragma unroll
+            for (int g = 0; g < 4; ++g) v[g] = slot2(slot + g * PAIR_SLOT_BYTES);
+            const float m = fmaxf(fmaxf(fmaxf(v[0].x, v[0].y), fmaxf(v[1].x, v[1].y)),
+                                  fmaxf(fmaxf(v[2].x, v[2].y), fmaxf(v[3].x, v[3].y)));
+            const unsigned any_c = __ballot_sync(FULL, m >= mesh.content_thr) >> oshift;
+            if ((can >> oshift) & 1u) {
+#pragma unroll
+               for (int g = 0; g < 4; ++g) slot2(slot + g * PAIR_SLOT_BYTES) = zero2;
+               store_pair<DIM>(dst_data + (size_t)out * WID3 + off, v);
+               if (l8 == 0) {
+                  dst_gids[out] = gid0 + (uint32_t)next_flush *
+                                            (DIM == 0 ? 1u : (DIM == 1 ? mesh.len[0] : mesh.len[0] * mesh.len[1]));
+                  content_out[out] = (any_c & 0xffu) ? 1 : 0;
+               }
+               ++out;
+               if (++next_flush >= run_end) {
+                  const ColumnSet& cs = sets[sidx];
+                  const uint32_t tm[3] = {cs.tgt_mask[0], cs.tgt_mask[1], cs.tgt_mask[2]};
+                  next_flush = mask_next_set(tm, next_flush);
+                  run_end = mask_run_end(tm, next_flush);
+               }
+            }
+         }
+      };
+
+      // the walk's state (see remap_walk_kernel): u the pending target's right
+      // edge in the cell, g2f the index of the edge after it, nacc minus its
+      // mass so far, so its slot (target cell times PAIR_SLOT_BYTES)
+      float v_l = 0.0f;
+      float2 g2f = zero2, u = zero2, nacc = zero2;
+      uint32_t sox = 0, soy = 0;
+      float2 vm1 = zero2, b = zero2, L = zero2;
+      bool out_x = false, out_y = false;
+
+      // the state at the start of the column whose first block is c
+      auto start = [&](const float2 c[4]) {
+         v_l = fa(fm((float)(WID * kb), mesh.dv), mesh.v_min);
+         // each lane's first target: the lowest g with (g+1) dk + im > v_l,
+         // from an approximate quotient
+         auto first_target = [&](float imc, float& gf, float& uc, uint32_t& so) {
+            int g = __float2int_rz(__fdividef(fs(v_l, imc), dk));
+            float e = fa(fm((float)(g + 1), dk), imc);
+#pragma unroll 1
+            for (int q = 0; q < 3 && e <= v_l; ++q) {
+               ++g;
+               e = fa(fm((float)(g + 1), dk), imc);
+            }
+#pragma unroll 1
+            for (int q = 0; q < 3; ++q) {
+               const float ep = fa(fm((float)g, dk), imc);
+               if (!(ep > v_l)) break;
+               --g;
+               e = ep;
+            }
+            if (g < lo) {
+               g = lo;
+               e = fa(fm((float)(g + 1), dk), imc);
+            }
+            gf = (float)(g + 2);
+            uc = fs(e, v_l) * mesh.inv_dv;
+            so = (uint32_t)g * PAIR_SLOT_BYTES;
+         };
+         first_target(im.x, g2f.x, u.x, sox);
+         first_target(im.y, g2f.y, u.y, soy);
+         // what another column left in the slots
+         nacc.x = -slot_x(sox);
+         nacc.y = -slot_y(soy);
+         // zero padding below the column
+         vm1 = zero2;
+         b = c[0];
+         if constexpr (RECON == RECON_PPM) {
+            const float2 face = h4_face_x2(zero2, zero2, c[0], c[1]);
+            L = p_neg_add(c[0], face);
+            const float2 t = __fmul2_rn(face, L);
+            out_x = t.x < 0.0f;
+            out_y = t.y < 0.0f;
+         }
+      };
+
+      // one cell: v0 with its upper neighbours
+      auto cell_step = [&](const float2 v0, const float2 vp1, const float2 vp2) {
+         // ---- reconstruction ----
+         const float2 a = p_neg_add(vp1, v0);
+         const float2 aS = __fmul2_rn(a, f2(SAME_SCALE)), bS = __fmul2_rn(b, f2(SAME_SCALE));
+         const float2 s = make_float2(with_sign(__saturatef(aS.x * bS.x), a.x), with_sign(__saturatef(aS.y * bS.y), a.y));
+         const float2 mx = __fmul2_rn(make_float2(fmaxf(fabsf(a.x), fabsf(b.x)), fmaxf(fabsf(a.y), fabsf(b.y))), f2(0.5f));
+         const float2 h = make_float2(fminf(fminf(fabsf(a.x), fabsf(b.x)), mx.x),
+                                      fminf(fminf(fabsf(a.y), fabsf(b.y)), mx.y));
+         float2 l = h, r = h;
+         if constexpr (RECON == RECON_PPM) {
+            const float2 fr = h4_face_x2(vm1, v0, vp1, vp2);
+            const float2 R = p_neg_add(fr, v0), Ln = p_neg_add(vp1, fr);
+            const float2 t = __fmul2_rn(R, Ln);
+            const bool or_x = t.x < 0.0f, or_y = t.y < 0.0f;
+            const float2 lf = make_float2(out_x ? h.x : L.x, out_y ? h.y : L.y);
+            const float2 rf = make_float2(or_x ? h.x : R.x, or_y ? h.y : R.y);
+            const float2 l2 = __fmul2_rn(lf, f2(2.0f)), r2 = __fmul2_rn(rf, f2(2.0f));
+            l = make_float2(fminf(fabsf(lf.x), fabsf(r2.x)), fminf(fabsf(lf.y), fabsf(r2.y)));
+            r = make_float2(fminf(fabsf(rf.x), fabsf(l2.x)), fminf(fabsf(rf.y), fabsf(l2.y)));
+            L = Ln;
+            out_x = or_x;
+            out_y = or_y;
+         }
+         // ---- distribute the cell over the lane's targets ----
+         const float2 um = __fadd2_rn(u, f2(-1.0f));
+         const bool hx = um.x < 0.0f, hy = um.y < 0.0f;  // the pending target's right edge lies inside
+         const float2 rl = p_neg_add(r, l);
+         // used only where the edge lies inside
+         const float2 T = (RECON == RECON_PPM) ? __ffma2_rn(u, rl, l) : l;
+         const float2 D = __fmul2_rn(u, __ffma2_rn(__fmul2_rn(s, um), T, v0));
+         // without an edge the slot is written again when its target is complete
+         const float2 val = p_neg_add(D, nacc);
+         slot_x(sox) = val.x;
+         slot_y(soy) = val.y;
+         nacc = p_neg_add(make_float2(hx ? D.x : nacc.x, hy ? D.y : nacc.y), v0);
+         // the next edge, with the reference's roundings (the packed multiply
+         // and add get contracted, so these are scalar)
+         const float2 e = make_float2(fa(fm(g2f.x, dk), im.x), fa(fm(g2f.y, dk), im.y));
+         const float2 un = __ffma2_rn(make_float2(fs(e.x, v_l), fs(e.y, v_l)), f2(mesh.inv_dv), f2(-1.0f));
+         u = um;
+         if (hx) {
+            g2f.x += 1.0f;
+            u.x = un.x;
+            sox += PAIR_SLOT_BYTES;
+         }
+         if (hy) {
+            g2f.y += 1.0f;
+            u.y = un.y;
+            soy += PAIR_SLOT_BYTES;
+         }
+         if (__builtin_expect(fminf(u.x, u.y) < 0.0f, 0)) {
+            // further edges inside the same source cell (dk < dv); more than
+            // eight (dk < dv / 8) lie outside what the walk represents and
+            // are reported with the cell
+            auto more = [&](float& uc, float& gf, uint32_t& so, float imc, float vc, float sc, float lc, float rlc,
+                            float Dc, auto slot) {
+#pragma unroll 1
+               for (int guard = 0; uc < 0.0f && guard < 8; ++guard) {
+                  const float ue = uc + 1.0f;
+                  const float T2 = (RECON == RECON_PPM) ? fmaf(ue, rlc, lc) : lc;
+                  const float D2 = ue * fmaf(sc * uc, T2, vc);
+                  slot(so) = D2 - Dc;
+                  Dc = D2;
+                  so += PAIR_SLOT_BYTES;
+                  uc = fmaf(fs(fa(fm(gf, dk), imc), v_l), mesh.inv_dv, -1.0f);
+                  gf += 1.0f;
+               }
+               range_err |= uc < 0.0f;
+               return Dc - vc;
+            };
+            if (u.x < 0.0f) nacc.x = more(u.x, g2f.x, sox, im.x, v0.x, s.x, l.x, rl.x, D.x, slot_x);
+            if (u.y < 0.0f) nacc.y = more(u.y, g2f.y, soy, im.y, v0.y, s.y, l.y, rl.y, D.y, slot_y);
+         }
+         v_l = fa(v_l, mesh.dv);
+         vm1 = v0;
+         b = a;
+      };
+
+      float2 w[4], n[4];  // the values of block `it` and of the one after it
+      {
+         const uint32_t r0 = n_src > 0 ? __ldg(perm + pos) : NO_BLOCK;
+         load_pair<DIM>(src_data + off, r0, w);
+      }
+      uint32_t row = n_src > 1 ? __ldg(perm + pos + 1) : NO_BLOCK;  // data row of block it + 1
+      if (n_src > 0) start(w);
+      // (one pass at least: a set without source blocks writes its targets)
+      for (int it = 0; it == 0 || it < iters; ++it) {
+         const bool active = it < n_src, last = left == 1;
+         load_pair<DIM>(src_data + off, row, n);
+         row = (it + 2 < n_src) ? __ldg(perm + pos + it + 2) : NO_BLOCK;
+         if (active) {
+            // zero padding above the column
+            const float2 n0 = last ? zero2 : n[0], n1 = last ? zero2 : n[1];
+            cell_step(w[0], w[1], w[2]);
+            cell_step(w[1], w[2], w[3]);
+            cell_step(w[2], w[3], n0);
+            cell_step(w[3], n0, n1);
+         }
+         int limit = NO_COLUMN;  // target blocks below it are complete in this lane's columns
+         if (active) {
+            const int gx = (int)(sox / PAIR_SLOT_BYTES), gy = (int)(soy / PAIR_SLOT_BYTES);  // the pending targets
+            int top = max(gx, gy) - 1;  // the highest target this block completed
+            limit = min(min(gx, gy), min(hi, ncf * WID)) >> 2;
+            if (last) {
+               // column done: the pending targets keep the rest; targets
+               // above the column's highest cell are folded into it
+               auto close = [&](int g, uint32_t so, float rest, auto slot) {
+                  if (g > hi) {
+#pragma unroll 1
+                     for (int t = hi + 1; t < g && t <= hi + RING_CELLS / 2; ++t) {
+                        rest += slot((uint32_t)t * PAIR_SLOT_BYTES);
+                        slot((uint32_t)t * PAIR_SLOT_BYTES) = 0.0f;
+                     }
+                     range_err |= g > hi + RING_CELLS / 2;
+                     slot(so) = 0.0f;  // what was written there while it was pending
+                     slot((uint32_t)hi * PAIR_SLOT_BYTES) += rest;
+                     return hi;
+                  }
+                  slot(so) = rest;
+                  return g;
+               };
+               const int tx = close(gx, sox, -nacc.x, slot_x), ty = close(gy, soy, -nacc.y, slot_y);
+               top = max(tx, ty);
+               limit = ncf;
+            }
+            // everything this block wrote must lie inside the ring's window
+            range_err |= top >= (next_flush + RING_BLOCKS) * WID;
+            --left;
+         }
+         flush(limit);
+         if (active && last && ncf != NO_COLUMN) {
+            // the next column of the set
+            const ColumnSet& cs = sets[sidx];
+            const SweepCell P = sweep_cells[cs.cell];
+            const uint32_t sm[3] = {cs.src_mask[0], cs.src_mask[1], cs.src_mask[2]};
+            int e = 0;
+            for (int done = it + 1;; done -= left) {
+               kb = mask_next_set(sm, e);
+               e = mask_run_end(sm, kb);
+               left = e - kb;
+               if (done == 0) break;
+            }
+            float mx, mn;
+            int cf, cl;
+            set_corners(P, cs.si(), cs.sj(), mx, mn);
+            column_extent(mx, mn, dk, mesh.dv, mesh.v_min, (int)mesh.len[DIM], kb, e - 1, mesh.wall_margin, cf, cl);
+            lo = cf * WID;
+            hi = (cl + 1) * WID - 1;
+            ncf = NO_COLUMN;
+            const int s = mask_next_set(sm, e);
+            if (s < 96)
+               column_extent(mx, mn, dk, mesh.dv, mesh.v_min, (int)mesh.len[DIM], s, mask_run_end(sm, s) - 1,
+                             mesh.wall_margin, ncf, cl);
+            start(n);
+         }
+#pragma unroll
+         for (int q = 0; q < 4; ++q) w[q] = n[q];
+      }
+      if ((__ballot_sync(FULL, range_err) >> oshift) & 0xffu) {
+         // deposits past the ring's window may lie in slots no flush reads
+         if (l8 == 0) atomicOr(&status[sets[sidx].cell], VLGPU_CELL_RANGE);
+#pragma unroll
+         for (int q = 0; q < RING_CELLS; ++q) slot2(q * PAIR_SLOT_BYTES) = zero2;
       }
    }
 }
@@ -1090,39 +1552,61 @@ cudaError_t launch_remap(int dim, const ColumnSet* sets, SweepCounters* counters
                          uint32_t* status, const MeshDev& mesh, int wall_margin, uint32_t set_capacity,
                          uint8_t* content_out, double content_threshold, bool exact, int recon, int grid,
                          cudaStream_t stream) {
+   PairMesh pm;
+   for (int d = 0; d < 3; ++d) pm.len[d] = mesh.len[d];
+   pm.wall_margin = wall_margin;
+   pm.dv = mesh.dv[dim];
+   pm.v_min = mesh.vmin[dim];
+   pm.inv_dv = (float)(1.0 / (double)mesh.dv[dim]);
+   pm.content_thr = (float)content_threshold;
+   if ((double)pm.content_thr < content_threshold) pm.content_thr = std::nextafterf(pm.content_thr, FLT_MAX);
 #define VLGPU_REMAP(D)                                                                                        \
    remap_kernel<D><<<grid, REMAP_THREADS, 0, stream>>>(sets, counters, perm, src_data, dst_data, dst_gids,          \
                                                        sweep_cells, status, mesh, wall_margin, set_capacity,        \
                                                        content_out, content_threshold)
-#define VLGPU_WALK(D, R)                                                                                       \
-   remap_walk_kernel<D, R><<<grid, REMAP_THREADS, 0, stream>>>(sets, counters, perm, src_data, dst_data, dst_gids, \
+#define VLGPU_WALK(D)                                                                                          \
+   remap_walk_kernel<D><<<grid, REMAP_THREADS, 0, stream>>>(sets, counters, perm, src_data, dst_data, dst_gids, \
                                                                sweep_cells, status, mesh, wall_margin, set_capacity, \
                                                                content_out, content_threshold)
-#define VLGPU_WALK_DIMS(R)               \
-   if (dim == 0) VLGPU_WALK(0, R);       \
-   else if (dim == 1) VLGPU_WALK(1, R);  \
-   else VLGPU_WALK(2, R);
+#define VLGPU_PAIR(D, R)                                                                                       \
+   {                                                                                                           \
+      const cudaError_t e = cudaFuncSetAttribute(remap_pair_kernel<D, R>,                                      \
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PAIR_SMEM); \
+      if (e != cudaSuccess) return e;                                                                          \
+      remap_pair_kernel<D, R><<<grid, PAIR_THREADS, PAIR_SMEM, stream>>>(                                      \
+         sets, counters, perm, src_data, dst_data, dst_gids, sweep_cells, status, pm, set_capacity, content_out); \
+   }
+#define VLGPU_PAIR_DIMS(R)                 \
+   if (dim == 0) VLGPU_PAIR(0, R)          \
+   else if (dim == 1) VLGPU_PAIR(1, R)     \
+   else VLGPU_PAIR(2, R)
    if (exact) {
       if (recon != RECON_PPM) return cudaErrorInvalidValue;  // the exact mode is PPM only
       if (dim == 0) VLGPU_REMAP(0);
       else if (dim == 1) VLGPU_REMAP(1);
       else VLGPU_REMAP(2);
    } else if (recon == RECON_PLM) {
-      VLGPU_WALK_DIMS(RECON_PLM)
+      VLGPU_PAIR_DIMS(RECON_PLM)
    } else if (recon == RECON_PQM) {
-      VLGPU_WALK_DIMS(RECON_PQM)
+      if (dim == 0) VLGPU_WALK(0);
+      else if (dim == 1) VLGPU_WALK(1);
+      else VLGPU_WALK(2);
    } else {
-      VLGPU_WALK_DIMS(RECON_PPM)
+      VLGPU_PAIR_DIMS(RECON_PPM)
    }
-#undef VLGPU_WALK_DIMS
+#undef VLGPU_PAIR_DIMS
+#undef VLGPU_PAIR
 #undef VLGPU_WALK
 #undef VLGPU_REMAP
    return cudaGetLastError();
 }
 
-// Points the remap work counter at the first set the next columnize launch
-// will create (per-cell launch sequences share one set array).
-__global__ void rebase_work_kernel(SweepCounters* counters) { counters->work = counters->n_sets; }
+// Points the remap at the first set the next columnize launch will create
+// (per-cell launch sequences share one set array).
+__global__ void rebase_work_kernel(SweepCounters* counters) {
+   counters->first_set = counters->n_sets;
+   counters->work = 0u;
+}
 
 cudaError_t launch_rebase_work(SweepCounters* counters, cudaStream_t stream) {
    rebase_work_kernel<<<1, 1, 0, stream>>>(counters);
@@ -1131,7 +1615,8 @@ cudaError_t launch_rebase_work(SweepCounters* counters, cudaStream_t stream) {
 
 int remap_blocks_per_sm() {
    int n = 0;
-   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, remap_walk_kernel<2, RECON_PPM>, REMAP_THREADS, 0);
+   cudaFuncSetAttribute(remap_pair_kernel<2, RECON_PPM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PAIR_SMEM);
+   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, remap_pair_kernel<2, RECON_PPM>, PAIR_THREADS, PAIR_SMEM);
    return n > 0 ? n : 1;
 }
 

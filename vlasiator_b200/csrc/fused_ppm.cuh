@@ -14,13 +14,6 @@ __device__ __forceinline__ float superbee_fused(float l, float m, float r) {
    return same ? copysignf(fmaxf(fminf(aa, ab + ab), fminf(aa + aa, ab)), a) : 0.0f;
 }
 
-// PLM coefficients (compute_plm_coeff, cpu_1d_plm.hpp:38-49): f = a0 + 2 a1 t.
-__device__ __forceinline__ void plm_coeff_fused(float vm1, float v0, float vp1, float a[5]) {
-   const float d = superbee_fused(vm1, v0, vp1);
-   a[0] = v0 - 0.5f * d;
-   a[1] = 0.5f * d;
-}
-
 // h8 face value and h7 face derivative of the left face of the cell whose
 // stencil is w0..w7 = values k-4 .. k+3 (cpu_face_estimates.hpp:45-79).
 __device__ __forceinline__ float h8_value(float w0, float w1, float w2, float w3, float w4, float w5, float w6,
@@ -111,23 +104,15 @@ __device__ __forceinline__ void pqm_coeff_fused(float vm1, float v0, float vp1, 
 // ACC_SEMILAG_PLM / _PPM / _PQM).
 constexpr int RECON_PLM = 1, RECON_PPM = 2, RECON_PQM = 4;
 
-// Integral of the reconstruction from 0 to u (cpu_acc_map.cpp:585-601),
+// Integral of the quartic reconstruction from 0 to u (cpu_acc_map.cpp:590-601),
 // Horner form with FMA.
-template <int RECON>
-__device__ __forceinline__ float recon_integral(float u, const float a[5]) {
-   if constexpr (RECON == RECON_PLM) return u * fmaf(u, a[1], a[0]);
-   if constexpr (RECON == RECON_PPM) return u * fmaf(u, fmaf(u, a[2], a[1]), a[0]);
+__device__ __forceinline__ float pqm_integral(float u, const float a[5]) {
    return u * fmaf(u, fmaf(u, fmaf(u, fmaf(u, a[4], a[3]), a[2]), a[1]), a[0]);
 }
 
 // The h4 face of uniform cells, (-v_{-2} + 7 v_{-1} + 7 v_0 - v_1) / 12
-// (cpu_face_estimates.hpp:160-167), in single precision with FMA.
-__device__ __forceinline__ float h4_face_fused(float vm2, float vm1, float v0, float vp1) {
-   return fmaf(7.0f, vm1 + v0, -(vm2 + vp1)) * (float)(1.0 / 12.0);
-}
-
-// The same face and PPM for two independent cells at once, with the packed
-// single-precision operations of sm_100 (__fadd2_rn, __fmul2_rn, __ffma2_rn;
+// (cpu_face_estimates.hpp:160-167), and PPM for two columns at once, with the
+// packed single-precision operations of sm_100 (__fadd2_rn, __fmul2_rn, __ffma2_rn;
 // y - x as fma(x, -1, y), exact before rounding); the limiter's comparisons
 // and selections stay per component.
 __device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
@@ -231,11 +216,6 @@ __device__ __forceinline__ void ppm_walk_x2(float2 v0, float2 vp1, float2 fl, fl
    nfr.y = (-dd.y > de.y) ? alt_r.y : r.y;
    a1 = p_sub(__ffma2_rn(a0, f2(-2.0f), v3), nfr);
    a2 = __ffma2_rn(v0, f2(-2.0f), __fadd2_rn(a0, nfr));
-}
-
-// Integral of two PPM reconstructions from 0 to u (u * (a0 + u (a1 + u a2))).
-__device__ __forceinline__ float2 ppm_integral_x2(float2 u, float2 a0, float2 a1, float2 a2) {
-   return __fmul2_rn(u, __ffma2_rn(u, __ffma2_rn(u, a2, a1), a0));
 }
 
 }  // namespace vlgpu

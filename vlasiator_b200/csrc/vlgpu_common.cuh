@@ -26,19 +26,21 @@ struct CellSlot {
 
 // One column set of one sweep: all blocks of a cell that share the two
 // transverse block indices.  Built by the columnize kernel, consumed by the
-// remap kernel.
-struct ColumnSet {
+// remap kernel.  40 bytes on 8-byte boundaries: a lane reads it in five loads.
+struct alignas(8) ColumnSet {
    uint32_t cell;
-   uint32_t si, sj;     // transverse block indices in the swapped frame
+   uint32_t sij;        // transverse block indices in the swapped frame: si + (sj << 16)
    uint32_t src_pos;    // first entry in the permutation array (absolute)
    uint32_t dst_pos;    // first output block (absolute, destination pool)
    uint32_t src_mask[3];
    uint32_t tgt_mask[3];
+   __host__ __device__ uint32_t si() const { return sij & 0xffffu; }
+   __host__ __device__ uint32_t sj() const { return sij >> 16; }
 };
 
 // Per-cell sweep parameters, already converted to Realf and swapped into the
 // frame where the sweep dimension is k (cpu_acc_map.cpp:127-199).
-struct SweepCell {
+struct alignas(8) SweepCell {
    float intersection, di, dj, dk;
    float threshold;
    uint32_t flags;  // SWEEP_PASS
@@ -126,7 +128,8 @@ struct MaskRec {
 struct SweepCounters {
    uint32_t n_sets;
    uint32_t dst_top;
-   uint32_t work;
+   uint32_t work;       // remap: sets claimed beyond the warps' first ones
+   uint32_t first_set;  // remap: the first set of this launch
    uint32_t overflow;
    uint32_t cell_next;  // warp-per-cell kernels (columnize, adjustment): next cell a warp takes
    uint32_t n_wide;     // cells those kernels left to their CTA-per-cell forms
