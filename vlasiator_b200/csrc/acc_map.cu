@@ -159,7 +159,22 @@ __device__ __forceinline__ void set_corners(const SweepCell& P, uint32_t si, uin
 // ---------------------------------------------------------------------------
 // columnize: one CTA per cell
 // ---------------------------------------------------------------------------
+// Threads per CTA: COL_THREADS where the cells outnumber the SMs, so that six
+// CTAs share an SM and hide one another's barriers; COL_FEW_THREADS where a
+// CTA has an SM to itself anyway (launch_columnize_batch).
 constexpr int COL_THREADS = 256;
+constexpr int COL_FEW_THREADS = 1024;
+constexpr int COL_UNROLL = 4;  // list entries a thread has in flight
+
+// Swapped indices of a block ID, by the mesh's reciprocals.
+template <int DIM>
+__device__ __forceinline__ void swapped_of(const MeshDev& mesh, uint32_t gid, uint32_t s[3]) {
+   uint32_t x, y, z;
+   block_xyz(mesh, gid, x, y, z);
+   s[0] = (DIM == 0) ? z : x;
+   s[1] = (DIM == 1) ? z : y;
+   s[2] = (DIM == 0) ? x : (DIM == 1 ? y : z);
+}
 
 __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* warp_sums, uint32_t& total) {
    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -223,11 +238,21 @@ __device__ __forceinline__ void columnize_cell(
    // shared min/max per warp)
    {
       uint32_t a0 = 0xffffffffu, a1 = 0, b0 = 0xffffffffu, b1 = 0;
-      for (uint32_t b = threadIdx.x; b < src.count; b += blockDim.x) {
-         uint32_t s[3];
-         swapped_indices(gids[src.off + b], mesh.len, DIM, s);
-         a0 = min(a0, s[0]); a1 = max(a1, s[0]);
-         b0 = min(b0, s[1]); b1 = max(b1, s[1]);
+      for (uint32_t t = threadIdx.x; t < src.count; t += blockDim.x * COL_UNROLL) {
+         // (an entry past the end repeats the thread's first one)
+         uint32_t g[COL_UNROLL];
+#pragma unroll
+         for (int u = 0; u < COL_UNROLL; ++u) {
+            const uint32_t b = t + blockDim.x * u;
+            g[u] = gids[src.off + (b < src.count ? b : t)];
+         }
+#pragma unroll
+         for (int u = 0; u < COL_UNROLL; ++u) {
+            uint32_t s[3];
+            swapped_of<DIM>(mesh, g[u], s);
+            a0 = min(a0, s[0]); a1 = max(a1, s[0]);
+            b0 = min(b0, s[1]); b1 = max(b1, s[1]);
+         }
       }
       a0 = __reduce_min_sync(FULL, a0); a1 = __reduce_max_sync(FULL, a1);
       b0 = __reduce_min_sync(FULL, b0); b1 = __reduce_max_sync(FULL, b1);
@@ -251,26 +276,42 @@ __device__ __forceinline__ void columnize_cell(
    uint32_t* tcount = prefix + plane + (plane + 1) / 2;  // plane
    for (uint32_t q = threadIdx.x; q < 3 * plane; q += blockDim.x) mask[q] = 0;
    __syncthreads();
-   // pass 2: occupancy masks along the sweep dimension; lanes that set bits
-   // of one word (a run of the list along the sweep) combine them first
-   for (uint32_t b0 = warp * 32; b0 < src.count; b0 += blockDim.x) {
-      const uint32_t b = b0 + lane;
-      uint32_t key = 0xffffffffu, bit = 0u;
-      if (b < src.count) {
-         uint32_t s[3];
-         swapped_indices(gids[src.off + b], mesh.len, DIM, s);
-         key = 3 * ((s[0] - a_lo) * nb + (s[1] - b_lo)) + (s[2] >> 5);
-         bit = 1u << (s[2] & 31);
+   // pass 2: occupancy masks along the sweep dimension; where the list runs
+   // along the sweep (the x sweep of a list in ID order) the lanes that set
+   // bits of one word combine them first
+   for (uint32_t t = warp * 32; t < src.count; t += blockDim.x * COL_UNROLL) {
+      uint32_t g[COL_UNROLL];
+#pragma unroll
+      for (int u = 0; u < COL_UNROLL; ++u) {
+         const uint32_t b = t + blockDim.x * u + lane;
+         g[u] = (b < src.count) ? gids[src.off + b] : 0u;
       }
-      const uint32_t match = __match_any_sync(FULL, key);
-      const bool big = key != 0xffffffffu && __popc(match) >= 4;
-      if (key != 0xffffffffu && !big) atomicOr(&mask[key], bit);
-      for (uint32_t leaders = __ballot_sync(FULL, big && (int)lane == __ffs(match) - 1); leaders;
-           leaders &= leaders - 1) {
-         const int leader = __ffs(leaders) - 1;
-         const bool mine = (__shfl_sync(FULL, match, leader) >> lane) & 1u;
-         const uint32_t bits = __reduce_or_sync(FULL, mine ? bit : 0u);
-         if ((int)lane == leader) atomicOr(&mask[key], bits);
+#pragma unroll
+      for (int u = 0; u < COL_UNROLL; ++u) {
+         const uint32_t b = t + blockDim.x * u + lane;
+         uint32_t key = 0xffffffffu, bit = 0u;
+         if (b < src.count) {
+            uint32_t s[3];
+            swapped_of<DIM>(mesh, g[u], s);
+            key = 3 * ((s[0] - a_lo) * nb + (s[1] - b_lo)) + (s[2] >> 5);
+            bit = 1u << (s[2] & 31);
+         }
+         const uint32_t left = __shfl_up_sync(FULL, key, 1);
+         const bool run = __popc(__ballot_sync(FULL, lane > 0 && key == left && key != 0xffffffffu)) >= 12;
+         if (!run) {
+            if (key != 0xffffffffu) atomicOr(&mask[key], bit);
+            continue;
+         }
+         const uint32_t match = __match_any_sync(FULL, key);
+         const bool big = key != 0xffffffffu && __popc(match) >= 4;
+         if (key != 0xffffffffu && !big) atomicOr(&mask[key], bit);
+         for (uint32_t leaders = __ballot_sync(FULL, big && (int)lane == __ffs(match) - 1); leaders;
+              leaders &= leaders - 1) {
+            const int leader = __ffs(leaders) - 1;
+            const bool mine = (__shfl_sync(FULL, match, leader) >> lane) & 1u;
+            const uint32_t bits = __reduce_or_sync(FULL, mine ? bit : 0u);
+            if ((int)lane == leader) atomicOr(&mask[key], bits);
+         }
       }
    }
    __syncthreads();
@@ -320,7 +361,11 @@ __device__ __forceinline__ void columnize_cell(
             int fb, lb;
             if (column_extent(mx, mn, P.dk, mesh.dv[DIM], mesh.vmin[DIM], max_len, k, e, wall_margin, fb, lb))
                wall = 1;
-            for (int q = fb; q <= lb; ++q) tm[q >> 5] |= 1u << (q & 31);
+#pragma unroll
+            for (int w = 0; w < 3; ++w) {
+               const int q0 = max(fb - 32 * w, 0), q1 = min(lb - 32 * w, 31);
+               if (q0 <= q1) tm[w] |= (0xffffffffu << q0) & (0xffffffffu >> (31 - q1));
+            }
             k = mask_next_set(m, e + 1);
          }
       }
@@ -360,12 +405,22 @@ __device__ __forceinline__ void columnize_cell(
          tbase += tcount[s];
       }
       // source permutation in (set, k) order
-      for (uint32_t b = threadIdx.x; b < src.count; b += blockDim.x) {
-         uint32_t s[3];
-         swapped_indices(gids[src.off + b], mesh.len, DIM, s);
-         const uint32_t t = (s[0] - a_lo) * nb + (s[1] - b_lo);
-         const uint32_t pos = prefix[t] + (uint32_t)mask_popc_below(&mask[3 * t], s[2]);
-         perm[src.off + pos] = src_index ? src_index[src.off + b] : src.off + b;
+      for (uint32_t e = threadIdx.x; e < src.count; e += blockDim.x * COL_UNROLL) {
+         uint32_t g[COL_UNROLL], row[COL_UNROLL];
+#pragma unroll
+         for (int u = 0; u < COL_UNROLL; ++u) {
+            const uint32_t b = e + blockDim.x * u, at = src.off + (b < src.count ? b : e);
+            g[u] = gids[at];
+            row[u] = src_index ? src_index[at] : at;
+         }
+#pragma unroll
+         for (int u = 0; u < COL_UNROLL; ++u) {
+            if (e + blockDim.x * u >= src.count) break;
+            uint32_t s[3];
+            swapped_of<DIM>(mesh, g[u], s);
+            const uint32_t t = (s[0] - a_lo) * nb + (s[1] - b_lo);
+            perm[src.off + prefix[t] + (uint32_t)mask_popc_below(&mask[3 * t], s[2])] = row[u];
+         }
       }
    } else if (sets_ok) {
       // no room for the output: neutralise this cell's sets
@@ -391,8 +446,8 @@ __device__ __forceinline__ void columnize_cell(
 }
 
 // One CTA per cell of [cell_begin, cell_end).
-template <int DIM>
-__global__ void __launch_bounds__(COL_THREADS) columnize_kernel(
+template <int DIM, int THREADS>
+__global__ void __launch_bounds__(THREADS) columnize_kernel(
    const uint32_t* __restrict__ gids, const uint32_t* __restrict__ src_index, const CellSlot* __restrict__ src_slots,
    CellSlot* __restrict__ dst_slots, uint32_t* __restrict__ perm, ColumnSet* __restrict__ sets,
    uint32_t set_capacity, uint32_t dst_capacity,
@@ -409,7 +464,7 @@ __global__ void __launch_bounds__(COL_THREADS) columnize_kernel(
 // Persistent CTAs over the cells whose plane did not fit the capped launch
 // (wide_cells, counters->n_wide of them), with a full plane of shared memory.
 template <int DIM>
-__global__ void __launch_bounds__(COL_THREADS) columnize_wide_kernel(
+__global__ void __launch_bounds__(COL_FEW_THREADS) columnize_wide_kernel(
    const uint32_t* __restrict__ gids, const uint32_t* __restrict__ src_index, const CellSlot* __restrict__ src_slots,
    CellSlot* __restrict__ dst_slots, uint32_t* __restrict__ perm, ColumnSet* __restrict__ sets,
    uint32_t set_capacity, uint32_t dst_capacity,
@@ -1483,13 +1538,12 @@ cudaError_t launch_columnize(int dim, const uint32_t* gids, const uint32_t* src_
    if (n == 0) return cudaSuccess;
    cudaError_t e = cudaSuccess;
 #define VLGPU_COL(D)                                                                                             \
-   e = cudaFuncSetAttribute(columnize_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);      \
+   e = cudaFuncSetAttribute(columnize_kernel<D, COL_FEW_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
+                            (int)smem);                                                                         \
    if (e != cudaSuccess) return e;                                                                              \
-   columnize_kernel<D><<<n, COL_THREADS, smem, stream>>>(gids, src_index, src_slots, dst_slots, perm, sets,      \
-                                                         set_capacity,                                          \
-                                                         dst_capacity, sweep_cells, status, counters, stats, mesh, \
-                                                         wall_margin, cell_begin, cell_end, first_of_step, nullptr, \
-                                                         0xffffffffu, nullptr);
+   columnize_kernel<D, COL_FEW_THREADS><<<n, COL_FEW_THREADS, smem, stream>>>(                                  \
+      gids, src_index, src_slots, dst_slots, perm, sets, set_capacity, dst_capacity, sweep_cells, status, counters, \
+      stats, mesh, wall_margin, cell_begin, cell_end, first_of_step, nullptr, 0xffffffffu, nullptr);
    if (dim == 0) { VLGPU_COL(0) } else if (dim == 1) { VLGPU_COL(1) } else { VLGPU_COL(2) }
 #undef VLGPU_COL
    return cudaGetLastError();
@@ -1498,32 +1552,36 @@ cudaError_t launch_columnize(int dim, const uint32_t* gids, const uint32_t* src_
 // Columnize of every cell of a batch: one CTA per cell, the largest cells
 // first (order), with shared memory for planes of up to COL_CAP_PLANE entries,
 // which lets four CTAs share an SM; the cells with wider planes follow in
-// columnize_wide_kernel.  The counters' n_wide must be zero (the caller clears
-// the sweep counters before every sweep).
+// columnize_wide_kernel.  The counters are zero before every sweep.
 constexpr uint32_t COL_CAP_PLANE = 1024;
 cudaError_t launch_columnize_batch(int dim, const uint32_t* gids, const uint32_t* src_index,
                                    const CellSlot* src_slots, CellSlot* dst_slots, uint32_t* perm, ColumnSet* sets,
                                    uint32_t set_capacity, uint32_t dst_capacity, const SweepCell* sweep_cells,
                                    uint32_t* status, SweepCounters* counters, BatchStats* stats, const MeshDev& mesh,
                                    int wall_margin, uint32_t n_cells, int first_of_step, uint32_t* wide_cells,
-                                   const uint32_t* order, int wide_grid, cudaStream_t stream) {
+                                   const uint32_t* order, int wide_grid, uint32_t few_cells, cudaStream_t stream) {
    if (n_cells == 0) return cudaSuccess;
    uint32_t li, lj;
    plane_lengths(mesh.len, dim, li, lj);
+   if (n_cells <= few_cells)
+      return launch_columnize(dim, gids, src_index, src_slots, dst_slots, perm, sets, set_capacity, dst_capacity,
+                              sweep_cells, status, counters, stats, mesh, wall_margin, 0, n_cells, first_of_step,
+                              stream);
    const uint32_t cap = li * lj < COL_CAP_PLANE ? li * lj : COL_CAP_PLANE;
    const size_t smem_cap = columnize_smem_bytes(cap);
    const size_t smem = columnize_smem_bytes(li * lj);
    const uint32_t g2 = (uint32_t)wide_grid < n_cells ? (uint32_t)wide_grid : n_cells;
    cudaError_t e = cudaSuccess;
 #define VLGPU_COLB(D)                                                                                           \
-   e = cudaFuncSetAttribute(columnize_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);       \
+   e = cudaFuncSetAttribute(columnize_kernel<D, COL_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,      \
+                            (int)smem);                                                                          \
    if (e != cudaSuccess) return e;                                                                               \
    e = cudaFuncSetAttribute(columnize_wide_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
    if (e != cudaSuccess) return e;                                                                               \
-   columnize_kernel<D><<<n_cells, COL_THREADS, smem_cap, stream>>>(                                              \
+   columnize_kernel<D, COL_THREADS><<<n_cells, COL_THREADS, smem_cap, stream>>>(                                              \
       gids, src_index, src_slots, dst_slots, perm, sets, set_capacity, dst_capacity, sweep_cells, status, counters, \
       stats, mesh, wall_margin, 0, n_cells, first_of_step, order, cap, wide_cells);                              \
-   columnize_wide_kernel<D><<<g2, COL_THREADS, smem, stream>>>(gids, src_index, src_slots, dst_slots, perm, sets, \
+   columnize_wide_kernel<D><<<g2, COL_FEW_THREADS, smem, stream>>>(gids, src_index, src_slots, dst_slots, perm, sets, \
                                                                set_capacity, dst_capacity, sweep_cells, status,   \
                                                                counters, stats, mesh, wall_margin, first_of_step, \
                                                                wide_cells);
@@ -1543,7 +1601,7 @@ int columnize_wide_blocks_per_sm(const MeshDev& mesh) {
    const size_t smem = columnize_smem_bytes(best);
    int n = 0;
    cudaFuncSetAttribute(columnize_wide_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, columnize_wide_kernel<0>, COL_THREADS, smem);
+   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, columnize_wide_kernel<0>, COL_FEW_THREADS, smem);
    return n > 0 ? n : 1;
 }
 

@@ -35,7 +35,7 @@ cudaError_t launch_columnize_batch(int dim, const uint32_t* gids, const uint32_t
                                    uint32_t set_capacity, uint32_t dst_capacity, const SweepCell* sweep_cells,
                                    uint32_t* status, SweepCounters* counters, BatchStats* stats, const MeshDev& mesh,
                                    int wall_margin, uint32_t n_cells, int first_of_step, uint32_t* wide_cells,
-                                   const uint32_t* order, int wide_grid, cudaStream_t stream);
+                                   const uint32_t* order, int wide_grid, uint32_t few_cells, cudaStream_t stream);
 int columnize_wide_blocks_per_sm(const MeshDev& mesh);
 cudaError_t launch_remap(int dim, const ColumnSet* sets, SweepCounters* counters, const uint32_t* perm,
                          const float* src_data, float* dst_data, uint32_t* dst_gids, const SweepCell* sweep_cells,

@@ -93,7 +93,7 @@ int sweep_device(vlgpu_batch* b, const SweepCell* sweep_cells, uint32_t dim, boo
       VL_CHECK(launch_columnize_batch((int)dim, b->st_gids, b->st_src, b->st_slots, b->slots[dst], b->perm, b->sets,
                                       cap, cap, sweep_cells, b->status, b->counters, b->stats, b->mdev, wm,
                                       b->n_cells, first_of_step ? 1 : 0, b->wide_cells, b->cell_order,
-                                      b->col_wide_grid, b->stream));
+                                      b->col_wide_grid, (uint32_t)b->sm_count, b->stream));
       const bool prof = b->profiling && b->prof_used + 2 <= b->prof_events.size();
       if (prof) VL_CHECK(cudaEventRecord(b->prof_events[b->prof_used], b->stream));
       VL_CHECK(launch_remap((int)dim, b->sets, b->counters, b->perm, b->data[src], b->data[dst], b->gids[dst],

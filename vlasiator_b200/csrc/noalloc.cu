@@ -187,6 +187,7 @@ extern "C" int vlgpu_map_1d_noalloc(const vlgpu_mesh* mesh, const vlgpu_params* 
       mdev.dv[d] = (float)(bs / WID);
       mdev.vmin[d] = (float)mesh->vmin[d];
    }
+   set_block_reciprocals(mdev);
 
    // the previous call's counters, flags and statuses must not leak into this one
    NA_CHECK(cudaMemsetAsync(base, 0, offsetof(NoallocLayout, zeroed_end), s));
