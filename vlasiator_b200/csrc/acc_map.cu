@@ -813,7 +813,7 @@ __global__ void __launch_bounds__(REMAP_THREADS, 3) remap_kernel(
 //    mass of targets above the column's highest cell is moved into it when
 //    the column ends.
 template <int DIM>
-__global__ void __launch_bounds__(REMAP_THREADS, 2) remap_walk_kernel(
+__global__ void __launch_bounds__(REMAP_THREADS, 3) remap_walk_kernel(
    const ColumnSet* __restrict__ sets, SweepCounters* __restrict__ counters, const uint32_t* __restrict__ perm,
    const float* __restrict__ src_data, float* __restrict__ dst_data, uint32_t* __restrict__ dst_gids,
    const SweepCell* __restrict__ sweep_cells, uint32_t* __restrict__ status, MeshDev mesh, int wall_margin,
@@ -1078,10 +1078,6 @@ constexpr float SAME_SCALE = 37778931862957161709568.0f;
 constexpr int PAIR_CTAS = 3;  // per SM: 72 to 80 registers, 192 KB of rings
 constexpr size_t PAIR_SMEM = (size_t)RING_CELLS * PAIR_SLOT_BYTES;
 
-// m >= 0 with the sign of a
-__device__ __forceinline__ float with_sign(float m, float a) {
-   return __uint_as_float(__float_as_uint(m) | (__float_as_uint(a) & 0x80000000u));
-}
 // y - x of two columns
 __device__ __forceinline__ float2 p_neg_add(float2 y, float2 x) { return __fadd2_rn(y, make_float2(-x.x, -x.y)); }
 

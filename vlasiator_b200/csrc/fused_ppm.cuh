@@ -5,13 +5,9 @@
 
 namespace vlgpu {
 
-// Superbee slope of (l, m, r) on unscaled values: sign(a) * max(min(|a|, 2|b|),
-// min(2|a|, |b|)) when a b > 0 (a = r - m, b = m - l), else 0.
-__device__ __forceinline__ float superbee_fused(float l, float m, float r) {
-   const float a = r - m, b = m - l;
-   const bool same = a * b > 0.0f;
-   const float aa = fabsf(a), ab = fabsf(b);
-   return same ? copysignf(fmaxf(fminf(aa, ab + ab), fminf(aa + aa, ab)), a) : 0.0f;
+// m >= 0 with the sign of a.
+__device__ __forceinline__ float with_sign(float m, float a) {
+   return __uint_as_float(__float_as_uint(m) | (__float_as_uint(a) & 0x80000000u));
 }
 
 // h8 face value and h7 face derivative of the left face of the cell whose
@@ -32,72 +28,87 @@ __device__ __forceinline__ float h7_derivative(float w0, float w1, float w2, flo
 // compute_filtered_face_values_derivatives (cpu_face_estimates.hpp:216-275)
 // and the inflexion-point filter filter_pqm_monotonicity (cpu_1d_pqm.hpp:
 // 31-156), in single precision.
+//
+// The faces enter as their distances from the cell's value, L = v0 - left and
+// R = right - v0: the combinations of v0 and the faces in the reference's
+// formulas cancel v0 exactly, so each is two products instead of three, without
+// the rounding of 60 v0 and 360 v0.  The reconstruction's slope is a cubic with
+// the Bernstein coefficients fd_l, fd_l + b0/3, fd_l + 2 b0/3 + b1/6, fd_r on
+// the cell; where none opposes the cell's slope, neither does the slope at an
+// inflexion point, and the roots (a square root and two quotients) are not
+// needed.
+__device__ __forceinline__ float sqrt_approx(float x) {
+   float r;
+   asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+   return r;
+}
 __device__ __forceinline__ void pqm_coeff_fused(float vm1, float v0, float vp1, float fv_l, float fv_r, float fd_l,
                                                 float fd_r, float a[5]) {
-   const float slope = superbee_fused(vm1, v0, vp1);
-   const float slope_abs = fabsf(slope);
-   const float slope_sign = slope > 0.0f ? 1.0f : -1.0f;
-   if (slope_abs == 0.0f) {
-      fv_r = v0;
-      fv_l = v0;
-      fd_l = 0.0f;
-      fd_r = 0.0f;
+   const float dr = vp1 - v0, dl = v0 - vm1;
+   const bool same = dr * dl > 0.0f;
+   const float adr = fabsf(dr), adl = fabsf(dl);
+   const float slope = same ? copysignf(fminf(2.0f * fminf(adr, adl), fmaxf(adr, adl)), dr) : 0.0f;
+   float L = v0 - fv_l, R = fv_r - v0;
+   // a face outside the values of its two cells, or a derivative against the slope
+   const float sign = with_sign(1.0f, slope);
+   if (L * (dl - L) < 0.0f || sign * fd_l < 0.0f) {
+      L = 0.5f * slope;
+      fd_l = slope;
    }
-   if ((vm1 - fv_l) * (fv_l - v0) < 0.0f || slope_sign * fd_l < 0.0f) {
-      fv_l = v0 - slope_sign * 0.5f * slope_abs;
-      fd_l = slope_sign * slope_abs;
+   if (R * (dr - R) < 0.0f || sign * fd_r < 0.0f) {
+      R = 0.5f * slope;
+      fd_r = slope;
    }
-   if ((vp1 - fv_r) * (fv_r - v0) < 0.0f || slope_sign * fd_r < 0.0f) {
-      fv_r = v0 + slope_sign * 0.5f * slope_abs;
-      fd_r = slope_sign * slope_abs;
-   }
+   if (slope == 0.0f) L = R = fd_l = fd_r = 0.0f;
    // second-derivative coefficients (White and Adcroft 2008, eq. 23)
-   const float b0 = 60.0f * v0 - 24.0f * fv_r - 36.0f * fv_l + 3.0f * (fd_r - 3.0f * fd_l);
-   const float b1 = -360.0f * v0 + 36.0f * fd_l - 24.0f * fd_r + 168.0f * fv_r + 192.0f * fv_l;
-   const float b2 = 360.0f * v0 + 30.0f * (fd_r - fd_l) - 180.0f * (fv_l + fv_r);
-   const float disc = b1 * b1 - 4.0f * b0 * b2;
-   const float sq = disc < 0.0f ? b1 + 200.0f * b2 : sqrtf(disc);
-   const float root1 = (-b1 + sq) / (2.0f * b2);
-   const float root2 = (-b1 - sq) / (2.0f * b2);
-   const float plm_l = 2.0f * (v0 - vm1), plm_r = 2.0f * (vp1 - v0);
-   const float ssign = plm_l + plm_r;
-   const float c0 = fd_l, c1 = b0, c2 = 0.5f * b1, c3 = b2 * (float)(1.0 / 3.0);
-   const float r1s = (root1 >= 0.0f && root1 <= 1.0f) ? c0 + root1 * (c1 + root1 * (c2 + root1 * c3)) : ssign;
-   const float r2s = (root2 >= 0.0f && root2 <= 1.0f) ? c0 + root2 * (c1 + root2 * (c2 + root2 * c3)) : ssign;
-   if (r1s * ssign < 0.0f || r2s * ssign < 0.0f) {
-      const float third = (float)(1.0 / 3.0);
-      if (fabsf(plm_l) <= fabsf(plm_r)) {
-         // collapse to the left edge (eq. 21), then the PLM-slope checks (eqs. 28, 29)
-         fd_l = third * (10.0f * v0 - 2.0f * fv_r - 8.0f * fv_l);
-         fd_r = -10.0f * v0 + 6.0f * fv_r + 4.0f * fv_l;
-         if (ssign * fd_l < 0.0f) {
-            fd_l = 0.0f;
-            fv_r = 5.0f * v0 - 4.0f * fv_l;
-            fd_r = 20.0f * (v0 - fv_l);
-         } else if (ssign * fd_r < 0.0f) {
-            fd_r = 0.0f;
-            fv_l = 0.5f * (5.0f * v0 - 3.0f * fv_r);
-            fd_l = (float)(10.0 / 3.0) * (-v0 + fv_r);
-         }
-      } else {
-         fd_l = 10.0f * v0 - 6.0f * fv_l - 4.0f * fv_r;
-         fd_r = third * (-10.0f * v0 + 2.0f * fv_l + 8.0f * fv_r);
-         if (ssign * fd_l < 0.0f) {
-            fd_l = 0.0f;
-            fv_r = 0.5f * (5.0f * v0 - 3.0f * fv_l);
-            fd_r = (float)(10.0 / 3.0) * (v0 - fv_l);
-         } else if (ssign * fd_r < 0.0f) {
-            fd_r = 0.0f;
-            fv_l = 5.0f * v0 - 4.0f * fv_r;
-            fd_l = 20.0f * (-v0 + fv_r);
+   const float d = R - L, e = fd_r - fd_l;
+   const float b0 = fmaf(3.0f, fd_r, fmaf(-9.0f, fd_l, fmaf(36.0f, L, -24.0f * R)));
+   const float b1 = fmaf(-24.0f, fd_r, fmaf(36.0f, fd_l, fmaf(168.0f, R, -192.0f * L)));
+   const float third = (float)(1.0 / 3.0);
+   const float s1 = fmaf(b0, third, fd_l), s2 = fmaf(b1, (float)(1.0 / 6.0), fmaf(b0, 2.0f * third, fd_l));
+   if (fminf(sign * s1, sign * s2) < 0.0f) {
+      const float b2 = fmaf(30.0f, e, -180.0f * d);
+      const float disc = fmaf(b1, b1, -4.0f * b0 * b2);
+      const float sq = disc < 0.0f ? b1 + 200.0f * b2 : sqrt_approx(disc);
+      const float root1 = __fdividef(-b1 + sq, 2.0f * b2);
+      const float root2 = __fdividef(-b1 - sq, 2.0f * b2);
+      const float c2 = 0.5f * b1, c3 = b2 * third;
+      const float r1s = (root1 >= 0.0f && root1 <= 1.0f) ? fmaf(root1, fmaf(root1, fmaf(root1, c3, c2), b0), fd_l) : sign;
+      const float r2s = (root2 >= 0.0f && root2 <= 1.0f) ? fmaf(root2, fmaf(root2, fmaf(root2, c3, c2), b0), fd_l) : sign;
+      if (fminf(r1s * sign, r2s * sign) < 0.0f) {
+         if (adl <= adr) {
+            // collapse to the left edge (eq. 21), then the PLM-slope checks (eqs. 28, 29)
+            fd_l = third * fmaf(8.0f, L, -2.0f * R);
+            fd_r = fmaf(6.0f, R, -4.0f * L);
+            if (sign * fd_l < 0.0f) {
+               fd_l = 0.0f;
+               R = 4.0f * L;
+               fd_r = 20.0f * L;
+            } else if (sign * fd_r < 0.0f) {
+               fd_r = 0.0f;
+               L = 1.5f * R;
+               fd_l = (float)(10.0 / 3.0) * R;
+            }
+         } else {
+            fd_l = fmaf(6.0f, L, -4.0f * R);
+            fd_r = third * fmaf(8.0f, R, -2.0f * L);
+            if (sign * fd_l < 0.0f) {
+               fd_l = 0.0f;
+               R = 1.5f * L;
+               fd_r = (float)(10.0 / 3.0) * L;
+            } else if (sign * fd_r < 0.0f) {
+               fd_r = 0.0f;
+               L = 4.0f * R;
+               fd_l = 20.0f * R;
+            }
          }
       }
    }
-   a[0] = fv_l;
+   a[0] = v0 - L;
    a[1] = 0.5f * fd_l;
-   a[2] = 10.0f * v0 - 4.0f * fv_r - 6.0f * fv_l + 0.5f * (fd_r - 3.0f * fd_l);
-   a[3] = -15.0f * v0 + 1.5f * fd_l - fd_r + 7.0f * fv_r + 8.0f * fv_l;
-   a[4] = 6.0f * v0 + 0.5f * (fd_r - fd_l) - 3.0f * (fv_l + fv_r);
+   a[2] = fmaf(0.5f, fd_r, fmaf(-1.5f, fd_l, fmaf(6.0f, L, -4.0f * R)));
+   a[3] = fmaf(1.5f, fd_l, fmaf(7.0f, R, -8.0f * L)) - fd_r;
+   a[4] = fmaf(0.5f, fd_r - fd_l, 3.0f * (L - R));
 }
 
 // Reconstruction orders of the acceleration remap (the reference's
