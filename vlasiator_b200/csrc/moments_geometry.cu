@@ -22,7 +22,7 @@
 
 namespace vlgpu {
 
-// Each cell's blocks are split into equal parts of at least 32 blocks (at
+// Each cell's blocks are split into equal parts of about MOM_MIN_PART blocks (at
 // most MOM_PARTS_PER_CELL parts); a warp takes (part, cell) items in a fixed
 // grid-stride order (consecutive items are the same part of consecutive
 // cells, so the work of large and small cells interleaves), sums its part
@@ -49,7 +49,7 @@ constexpr int MOM_THREADS = 256;
 
 // Parts of a cell with `count` blocks: enough that a part has at least
 // MOM_MIN_PART blocks, at most MOM_PARTS_PER_CELL.
-constexpr uint32_t MOM_MIN_PART = 256;
+constexpr uint32_t MOM_MIN_PART = 64;
 constexpr uint32_t MOM_TILE = 256;  // blocks of a part staged at a time
 __device__ __forceinline__ uint32_t moment_parts(uint32_t count) {
    const uint32_t p = (count + MOM_MIN_PART - 1) / MOM_MIN_PART;
