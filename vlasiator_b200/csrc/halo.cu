@@ -10,13 +10,45 @@
 
 namespace vlgpu {
 
-// One CTA per selected cell: its blocks (IDs and 64 values) to dst_off.
-__global__ void pack_cells_kernel(const uint32_t* __restrict__ gids, const float4* __restrict__ data,
-                                  const uint32_t* __restrict__ desc, uint32_t* __restrict__ out_gids,
-                                  float4* __restrict__ out_data) {
+// Copies chunks of blocks (IDs and 64 values) to their places, a chunk (first
+// list entry, first output block, blocks) per CTA and half a warp per block.
+// The host cuts the selected cells into chunks of one size, so a large cell
+// spreads over many CTAs.  An indirect state is read through src_index (a
+// block without data gives zeros), so packing moves nothing in the batch.
+//
+// Bound by HBM reads and writes.  A CTA per cell took 561 us for 13 cells of 12000 blocks
+// and 404 us for 1024 cells of 30 to 9000 blocks (1.8 TB/s, the largest cells
+// last); in chunks the packing, adjustment and moments of the latter together
+// went from 1280 to 1036 us.
+constexpr int PACK_THREADS = 256;
+constexpr uint32_t PACK_BLOCKS = 4 * PACK_THREADS / 16;  // blocks a CTA moves per pass, four per half-warp
+constexpr uint32_t PACK_CHUNK = 4 * PACK_BLOCKS;         // largest chunk
+__global__ void __launch_bounds__(PACK_THREADS) pack_cells_kernel(const uint32_t* __restrict__ gids,
+                                                                  const uint32_t* __restrict__ src_index,
+                                                                  const float4* __restrict__ data,
+                                                                  const uint32_t* __restrict__ desc,
+                                                                  uint32_t* __restrict__ out_gids,
+                                                                  float4* __restrict__ out_data) {
    const uint32_t src = desc[3 * blockIdx.x], dst = desc[3 * blockIdx.x + 1], n = desc[3 * blockIdx.x + 2];
-   for (uint32_t b = threadIdx.x; b < n; b += blockDim.x) out_gids[dst + b] = gids[src + b];
-   for (uint32_t q = threadIdx.x; q < 16 * n; q += blockDim.x) out_data[16 * (size_t)dst + q] = data[16 * (size_t)src + q];
+   const uint32_t sub = threadIdx.x & 15, hw = threadIdx.x >> 4;
+   for (uint32_t b0 = 0; b0 < n; b0 += PACK_BLOCKS) {
+      float4 v[4];
+#pragma unroll
+      for (uint32_t u = 0; u < 4; ++u) {
+         const uint32_t b = b0 + hw + u * (PACK_THREADS / 16);
+         v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+         if (b < n) {
+            const uint32_t row = src_index ? src_index[src + b] : src + b;
+            if (row != 0xffffffffu) v[u] = __ldg(data + 16 * (size_t)row + sub);
+         }
+      }
+#pragma unroll
+      for (uint32_t u = 0; u < 4; ++u) {
+         const uint32_t b = b0 + hw + u * (PACK_THREADS / 16);
+         if (b < n) out_data[16 * ((size_t)dst + b) + sub] = v[u];
+      }
+   }
+   for (uint32_t b = threadIdx.x; b < n; b += PACK_THREADS) out_gids[dst + b] = gids[src + b];
 }
 
 // Every block ID below max_gid; a bad one sets *bad.
@@ -57,6 +89,61 @@ int halo_scratch(vlgpu_batch* b, size_t n) {
    return VLGPU_OK;
 }
 
+// Whether the selection names every cell of the batch.
+bool replaces_all(const vlgpu_batch* b, uint32_t n_sel, const uint32_t* cells) {
+   if (n_sel < b->n_cells) return false;
+   std::vector<char> seen(b->n_cells, 0);
+   uint32_t n = 0;
+   for (uint32_t i = 0; i < n_sel; ++i) {
+      n += !seen[cells[i]];
+      seen[cells[i]] = 1;
+   }
+   return n == b->n_cells;
+}
+
+// Unpacking that replaces every cell: nothing of the current state is kept,
+// so it is not made direct (a copy of the whole VDF after an adjustment), and
+// the blocks go to the start of the idle pool.  The current state stays as it
+// is until the block IDs are known to be good, so one wait serves the whole
+// call.
+int unpack_all(vlgpu_batch* b, uint32_t n_sel, const uint32_t* cells, const uint32_t* counts, const uint32_t* gids,
+               const float* data, uint64_t total) {
+   if (total > b->capacity) return VLGPU_ENOMEM;
+   const int pool = 1 - b->cur;
+   const int st = halo_scratch(b, 1);
+   if (st != VLGPU_OK) return st;
+   uint32_t bad = 0, used = 0;
+   std::vector<CellSlot> slots(b->n_cells);
+   uint32_t o = 0;
+   for (uint32_t i = 0; i < n_sel; ++i) {
+      slots[cells[i]] = CellSlot{o, counts[i]};
+      o += counts[i];
+   }
+   VL_CHECK(cudaMemcpyAsync(b->slots[pool], slots.data(), sizeof(CellSlot) * b->n_cells, cudaMemcpyHostToDevice,
+                            b->stream));
+   if (total > 0) {
+      VL_CHECK(cudaMemsetAsync(b->halo_scratch, 0, sizeof(uint32_t), b->stream));
+      const uint32_t max_gid = b->mesh.len[0] * b->mesh.len[1] * b->mesh.len[2];
+      check_gids_range_kernel<<<b->sm_count * 2, 256, 0, b->stream>>>(gids, total, max_gid, b->halo_scratch);
+      b->launches += 1;
+      VL_CHECK(cudaGetLastError());
+      VL_CHECK(cudaMemcpyAsync(b->gids[pool], gids, sizeof(uint32_t) * total, cudaMemcpyDeviceToDevice, b->stream));
+      VL_CHECK(cudaMemcpyAsync(b->data[pool], data, sizeof(float) * WID3 * total, cudaMemcpyDeviceToDevice, b->stream));
+      VL_CHECK(cudaMemcpyAsync(&bad, b->halo_scratch, sizeof(uint32_t), cudaMemcpyDeviceToHost, b->stream));
+   }
+   VL_CHECK(cudaMemcpyAsync(&used, b->rows_used + b->st_list, sizeof(uint32_t), cudaMemcpyDeviceToHost, b->stream));
+   VL_CHECK(cudaStreamSynchronize(b->stream));
+   // the same room is asked for as when some cells are replaced: behind the
+   // rows in use
+   if (used + total > b->capacity) return VLGPU_ENOMEM;
+   if (bad) return VLGPU_EINVAL;
+   const uint32_t now = (uint32_t)total;
+   VL_CHECK(cudaMemcpyAsync(b->rows_used + pool, &now, sizeof(uint32_t), cudaMemcpyHostToDevice, b->stream));
+   set_direct_state(b, pool);
+   b->content_valid = false;
+   return VLGPU_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -65,31 +152,41 @@ int vlgpu_batch_pack_cells(vlgpu_batch* b, uint32_t n_sel, const uint32_t* cells
                            float* data, uint64_t capacity, uint64_t* used) {
    if (!b || !used || (n_sel > 0 && (!cells || !counts))) return VLGPU_EINVAL;
    VL_CHECK(cudaSetDevice(b->device));
-   std::vector<CellSlot> slots;
-   uint32_t rows[4];
-   int st = direct_state_slots(b, slots, rows);
-   if (st != VLGPU_OK) return st;
-   std::vector<uint32_t> desc(3 * (size_t)n_sel);
+   std::vector<CellSlot> slots(b->n_cells);
+   VL_CHECK(cudaMemcpyAsync(slots.data(), b->st_slots, sizeof(CellSlot) * b->n_cells, cudaMemcpyDeviceToHost,
+                            b->stream));
+   VL_CHECK(cudaStreamSynchronize(b->stream));
    uint64_t total = 0;
    for (uint32_t i = 0; i < n_sel; ++i) {
       if (cells[i] >= b->n_cells) return VLGPU_EINVAL;
-      const CellSlot s = slots[cells[i]];
-      desc[3 * i] = s.off;
-      desc[3 * i + 1] = (uint32_t)total;
-      desc[3 * i + 2] = s.count;
-      counts[i] = s.count;
-      total += s.count;
+      counts[i] = slots[cells[i]].count;
+      total += counts[i];
    }
    *used = total;
    if (total > capacity) return VLGPU_ENOMEM;
    if (total > 0 && (!gids || !data)) return VLGPU_EINVAL;
    if (total == 0) return VLGPU_OK;
-   st = halo_scratch(b, desc.size());
+   // chunks small enough that a small selection still reaches every SM
+   const uint64_t even = total / (8 * (uint64_t)b->sm_count);
+   const uint32_t chunk = even <= PACK_BLOCKS ? PACK_BLOCKS : std::min<uint32_t>(PACK_CHUNK, (uint32_t)even);
+   std::vector<uint32_t> desc;
+   desc.reserve(3 * ((size_t)n_sel + total / chunk));
+   uint32_t dst = 0;
+   for (uint32_t i = 0; i < n_sel; ++i) {
+      const CellSlot s = slots[cells[i]];
+      for (uint32_t q = 0; q < s.count; q += chunk) {
+         const uint32_t n = std::min(chunk, s.count - q);
+         desc.insert(desc.end(), {s.off + q, dst, n});
+         dst += n;
+      }
+   }
+   const int st = halo_scratch(b, desc.size());
    if (st != VLGPU_OK) return st;
    VL_CHECK(cudaMemcpyAsync(b->halo_scratch, desc.data(), sizeof(uint32_t) * desc.size(), cudaMemcpyHostToDevice,
                             b->stream));
-   pack_cells_kernel<<<n_sel, 256, 0, b->stream>>>(b->st_gids, reinterpret_cast<const float4*>(b->data[b->cur]),
-                                                   b->halo_scratch, gids, reinterpret_cast<float4*>(data));
+   pack_cells_kernel<<<(unsigned)(desc.size() / 3), PACK_THREADS, 0, b->stream>>>(
+      b->st_gids, b->st_src, reinterpret_cast<const float4*>(b->data[b->cur]), b->halo_scratch, gids,
+      reinterpret_cast<float4*>(data));
    b->launches += 1;
    VL_CHECK(cudaGetLastError());
    VL_CHECK(cudaStreamSynchronize(b->stream));
@@ -106,6 +203,7 @@ int vlgpu_batch_unpack_cells(vlgpu_batch* b, uint32_t n_sel, const uint32_t* cel
       total += counts[i];
    }
    if (total > 0 && (!gids || !data)) return VLGPU_EINVAL;
+   if (replaces_all(b, n_sel, cells)) return unpack_all(b, n_sel, cells, counts, gids, data, total);
    std::vector<CellSlot> slots;
    uint32_t rows[4];
    int st = direct_state_slots(b, slots, rows);
