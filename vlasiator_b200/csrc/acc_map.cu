@@ -1072,14 +1072,8 @@ constexpr int PAIR_THREADS = 256;
 constexpr int PAIR_WARPS = PAIR_THREADS / 32;
 constexpr uint32_t PAIR_SLOT_BYTES = PAIR_THREADS * sizeof(float2);  // one ring slot of the CTA
 constexpr uint32_t PAIR_SLOT_MASK = (RING_CELLS - 1) * PAIR_SLOT_BYTES;
-// a b > 0 of two value differences as a factor 0 or 1: their scaled product,
-// saturated.  2^75 squared times the smallest denormal product is 1.
-constexpr float SAME_SCALE = 37778931862957161709568.0f;
 constexpr int PAIR_CTAS = 3;  // per SM: 72 to 80 registers, 192 KB of rings
 constexpr size_t PAIR_SMEM = (size_t)RING_CELLS * PAIR_SLOT_BYTES;
-
-// y - x of two columns
-__device__ __forceinline__ float2 p_neg_add(float2 y, float2 x) { return __fadd2_rn(y, make_float2(-x.x, -x.y)); }
 
 // The lane's two columns of the block at `row`: cells g = 0..3 along the
 // sweep, .x and .y the two columns (zeros for a block without data).
@@ -1302,8 +1296,8 @@ __global__ void __launch_bounds__(PAIR_THREADS, PAIR_CTAS) remap_pair_kernel(
       float v_l = 0.0f;
       float2 g2f = zero2, u = zero2, nacc = zero2;
       uint32_t sox = 0, soy = 0;
-      float2 vm1 = zero2, b = zero2, L = zero2;
-      bool out_x = false, out_y = false;
+      float2 vm1 = zero2;
+      PpmWalk ppm{zero2, zero2, false, false};
 
       // the state at the start of the column whose first block is c
       auto start = [&](const float2 c[4]) {
@@ -1340,52 +1334,35 @@ __global__ void __launch_bounds__(PAIR_THREADS, PAIR_CTAS) remap_pair_kernel(
          nacc.y = -slot_y(soy);
          // zero padding below the column
          vm1 = zero2;
-         b = c[0];
-         if constexpr (RECON == RECON_PPM) {
-            const float2 face = h4_face_x2(zero2, zero2, c[0], c[1]);
-            L = p_neg_add(c[0], face);
-            const float2 t = __fmul2_rn(face, L);
-            out_x = t.x < 0.0f;
-            out_y = t.y < 0.0f;
-         }
+         if constexpr (RECON == RECON_PPM) ppm.start(zero2, zero2, c[0], c[1]);
+         else ppm.b = c[0];
       };
 
       // one cell: v0 with its upper neighbours
       auto cell_step = [&](const float2 v0, const float2 vp1, const float2 vp2) {
          // ---- reconstruction ----
-         const float2 a = p_neg_add(vp1, v0);
-         const float2 aS = __fmul2_rn(a, f2(SAME_SCALE)), bS = __fmul2_rn(b, f2(SAME_SCALE));
-         const float2 s = make_float2(with_sign(__saturatef(aS.x * bS.x), a.x), with_sign(__saturatef(aS.y * bS.y), a.y));
-         const float2 mx = __fmul2_rn(make_float2(fmaxf(fabsf(a.x), fabsf(b.x)), fmaxf(fabsf(a.y), fabsf(b.y))), f2(0.5f));
-         const float2 h = make_float2(fminf(fminf(fabsf(a.x), fabsf(b.x)), mx.x),
-                                      fminf(fminf(fabsf(a.y), fabsf(b.y)), mx.y));
-         float2 l = h, r = h;
+         float2 s, l, r;
          if constexpr (RECON == RECON_PPM) {
-            const float2 fr = h4_face_x2(vm1, v0, vp1, vp2);
-            const float2 R = p_neg_add(fr, v0), Ln = p_neg_add(vp1, fr);
-            const float2 t = __fmul2_rn(R, Ln);
-            const bool or_x = t.x < 0.0f, or_y = t.y < 0.0f;
-            const float2 lf = make_float2(out_x ? h.x : L.x, out_y ? h.y : L.y);
-            const float2 rf = make_float2(or_x ? h.x : R.x, or_y ? h.y : R.y);
-            const float2 l2 = __fmul2_rn(lf, f2(2.0f)), r2 = __fmul2_rn(rf, f2(2.0f));
-            l = make_float2(fminf(fabsf(lf.x), fabsf(r2.x)), fminf(fabsf(lf.y), fabsf(r2.y)));
-            r = make_float2(fminf(fabsf(rf.x), fabsf(l2.x)), fminf(fabsf(rf.y), fabsf(l2.y)));
-            L = Ln;
-            out_x = or_x;
-            out_y = or_y;
+            ppm_magnitudes_x2(ppm, vm1, v0, vp1, vp2, s, l, r);
+            vm1 = v0;
+         } else {
+            const float2 a = p_minus(vp1, v0);
+            half_slope_x2(a, ppm.b, l, s);
+            r = l;
+            ppm.b = a;
          }
          // ---- distribute the cell over the lane's targets ----
          const float2 um = __fadd2_rn(u, f2(-1.0f));
          const bool hx = um.x < 0.0f, hy = um.y < 0.0f;  // the pending target's right edge lies inside
-         const float2 rl = p_neg_add(r, l);
+         const float2 rl = p_minus(r, l);
          // used only where the edge lies inside
          const float2 T = (RECON == RECON_PPM) ? __ffma2_rn(u, rl, l) : l;
          const float2 D = __fmul2_rn(u, __ffma2_rn(__fmul2_rn(s, um), T, v0));
          // without an edge the slot is written again when its target is complete
-         const float2 val = p_neg_add(D, nacc);
+         const float2 val = p_minus(D, nacc);
          slot_x(sox) = val.x;
          slot_y(soy) = val.y;
-         nacc = p_neg_add(make_float2(hx ? D.x : nacc.x, hy ? D.y : nacc.y), v0);
+         nacc = p_minus(make_float2(hx ? D.x : nacc.x, hy ? D.y : nacc.y), v0);
          // the next edge, with the reference's roundings (the packed multiply
          // and add get contracted, so these are scalar)
          const float2 e = make_float2(fa(fm(g2f.x, dk), im.x), fa(fm(g2f.y, dk), im.y));
@@ -1425,8 +1402,6 @@ __global__ void __launch_bounds__(PAIR_THREADS, PAIR_CTAS) remap_pair_kernel(
             if (u.y < 0.0f) nacc.y = more(u.y, g2f.y, soy, im.y, v0.y, s.y, l.y, rl.y, D.y, slot_y);
          }
          v_l = fa(v_l, mesh.dv);
-         vm1 = v0;
-         b = a;
       };
 
       float2 w[4], n[4];  // the values of block `it` and of the one after it

@@ -134,99 +134,65 @@ __device__ __forceinline__ float2 h4_face_x2(float2 vm2, float2 vm1, float2 v0, 
                      __fmul2_rn(__fadd2_rn(vm2, vp1), f2((float)(-1.0 / 12.0))));
 }
 
-// Superbee slope magnitude of one cell (zero at an extremum), the faces
-// flattened to v0 where it is zero, and half the signed slope.
-__device__ __forceinline__ float half_slope(float a, float b, float v0, float& fl, float& fr) {
-   const bool same = a * b > 0.0f;
-   const float aa = fabsf(a), ab = fabsf(b);
-   const float sl = same ? fmaxf(fminf(aa, ab + ab), fminf(aa + aa, ab)) : 0.0f;
-   if (sl == 0.0f) {
-      fl = v0;
-      fr = v0;
-   }
-   return copysignf(0.5f * sl, a);
+// y - x of two columns.
+__device__ __forceinline__ float2 p_minus(float2 y, float2 x) { return __fadd2_rn(y, make_float2(-x.x, -x.y)); }
+
+// a b > 0 of two value differences as a factor 0 or 1: their scaled product,
+// saturated.  2^75 squared times the smallest denormal product is 1.
+constexpr float SAME_SCALE = 37778931862957161709568.0f;
+
+// Half the superbee slope of two columns, h = min(|a|, |b|, max(|a|, |b|) / 2)
+// for the differences a, b to the right and left, and its sign s (zero at an
+// extremum).
+__device__ __forceinline__ void half_slope_x2(float2 a, float2 b, float2& h, float2& s) {
+   const float2 aS = __fmul2_rn(a, f2(SAME_SCALE)), bS = __fmul2_rn(b, f2(SAME_SCALE));
+   s = make_float2(with_sign(__saturatef(aS.x * bS.x), a.x), with_sign(__saturatef(aS.y * bS.y), a.y));
+   const float2 mx =
+      __fmul2_rn(make_float2(fmaxf(fabsf(a.x), fabsf(b.x)), fmaxf(fabsf(a.y), fabsf(b.y))), f2(0.5f));
+   h = make_float2(fminf(fminf(fabsf(a.x), fabsf(b.x)), mx.x), fminf(fminf(fabsf(a.y), fabsf(b.y)), mx.y));
 }
 
-// PPM coefficients of two cells at once (cpu_1d_ppm.hpp:35-54 in plain single
-// precision: superbee slope, faces outside their cells' values reset to
-// v0 -/+ slope/2, Colella-Woodward overshoot corrections): f(t) = a0 + a1 t +
-// a2 t^2 on each.
-__device__ __forceinline__ void ppm_coeff_x2(float2 vm1, float2 v0, float2 vp1, float2 fl, float2 fr, float2& a0,
-                                             float2& a1, float2& a2) {
-   const float2 a = p_sub(vp1, v0), b = p_sub(v0, vm1);
-   float2 hs;
-   hs.x = half_slope(a.x, b.x, v0.x, fl.x, fr.x);
-   hs.y = half_slope(a.y, b.y, v0.y, fl.y, fr.y);
-   {
-      const float2 tl = __fmul2_rn(p_sub(vm1, fl), p_sub(fl, v0));
-      const float2 tr = __fmul2_rn(p_sub(vp1, fr), p_sub(fr, v0));
-      const float2 nl = p_sub(v0, hs), nr = __fadd2_rn(v0, hs);
-      if (tl.x < 0.0f) fl.x = nl.x;
-      if (tl.y < 0.0f) fl.y = nl.y;
-      if (tr.x < 0.0f) fr.x = nr.x;
-      if (tr.y < 0.0f) fr.y = nr.y;
+// What a walk along the cells carries from one cell to the next: v - left
+// face, whether that face lies outside the values of its two cells, and the
+// difference to the cell below.
+struct PpmWalk {
+   float2 left, b;
+   bool out_x, out_y;
+   // before the cell v0 with the cells vm2, vm1 below it and vp1 above
+   __device__ __forceinline__ void start(float2 vm2, float2 vm1, float2 v0, float2 vp1) {
+      const float2 face = h4_face_x2(vm2, vm1, v0, vp1);
+      left = p_minus(v0, face);
+      b = p_minus(v0, vm1);
+      const float2 t = __fmul2_rn(p_minus(face, vm1), left);
+      out_x = t.x < 0.0f;
+      out_y = t.y < 0.0f;
    }
-   const float2 sixth = f2((float)(1.0 / 6.0));
-   const float2 v3 = __fmul2_rn(v0, f2(3.0f));
-   {
-      const float2 d = p_sub(fr, fl), e = __ffma2_rn(__fadd2_rn(fl, fr), f2(-0.5f), v0);
-      const float2 de = __fmul2_rn(d, e), dd = __fmul2_rn(__fmul2_rn(d, d), sixth);
-      const float2 alt = __ffma2_rn(fr, f2(-2.0f), v3);
-      if (de.x > dd.x) fl.x = alt.x;
-      if (de.y > dd.y) fl.y = alt.y;
-   }
-   {
-      const float2 d = p_sub(fr, fl), e = __ffma2_rn(__fadd2_rn(fl, fr), f2(-0.5f), v0);
-      const float2 de = __fmul2_rn(d, e), dd = __fmul2_rn(__fmul2_rn(d, d), sixth);
-      const float2 alt = __ffma2_rn(fl, f2(-2.0f), v3);
-      if (-dd.x > de.x) fr.x = alt.x;
-      if (-dd.y > de.y) fr.y = alt.y;
-   }
-   a0 = fl;
-   a1 = p_sub(__ffma2_rn(fl, f2(-2.0f), v3), fr);
-   a2 = __ffma2_rn(v0, f2(-2.0f), __fadd2_rn(fl, fr));
-}
+};
 
-// The same PPM in the walk form (that of the acceleration's
-// remap_walk_kernel), for a walk along the cells: what a cell shares with its
-// left neighbour comes in from it instead of being recomputed.
-//  - tl: the left face's test (vm1 - fl)(fl - v0), which is the left
-//    neighbour's right-face test (v0' - fr')(fr' - vp1') with the same
-//    rounded factors; tr returns this cell's, for the next cell.
-//  - dprev: v0 - vm1, the left neighbour's vp1 - v0; dn returns this cell's.
-//  - The superbee slope in closed form, min(2 min(|a|,|b|), max(|a|,|b|)).
-//  - The two Colella-Woodward corrections taken as alternatives: in exact
-//    arithmetic the second cannot fire once the first has.
-// Its limiter decisions are the reference's, up to rounding in the
-// corrections; the fused tolerances cover it.
-__device__ __forceinline__ void ppm_walk_x2(float2 v0, float2 vp1, float2 fl, float2 fr, float2 tl, float2 dprev,
-                                            float2& tr, float2& dn, float2& a0, float2& a1, float2& a2) {
-   dn = p_sub(vp1, v0);
-   tr = __fmul2_rn(p_sub(v0, fr), p_sub(fr, vp1));
-   float2 hs;
-   {
-      const float anx = fabsf(dn.x), apx = fabsf(dprev.x), any = fabsf(dn.y), apy = fabsf(dprev.y);
-      hs.x = copysignf(0.5f * fminf(2.0f * fminf(anx, apx), fmaxf(anx, apx)), dn.x);
-      hs.y = copysignf(0.5f * fminf(2.0f * fminf(any, apy), fmaxf(any, apy)), dn.y);
-   }
-   const float2 nl = p_sub(v0, hs), nr = __fadd2_rn(v0, hs);
-   const bool sx = dn.x * dprev.x > 0.0f, sy = dn.y * dprev.y > 0.0f;
-   float2 l, r;
-   l.x = sx ? (tl.x < 0.0f ? nl.x : fl.x) : v0.x;
-   l.y = sy ? (tl.y < 0.0f ? nl.y : fl.y) : v0.y;
-   r.x = sx ? (tr.x < 0.0f ? nr.x : fr.x) : v0.x;
-   r.y = sy ? (tr.y < 0.0f ? nr.y : fr.y) : v0.y;
-   const float2 d = p_sub(r, l), e = __ffma2_rn(__fadd2_rn(l, r), f2(-0.5f), v0);
-   const float2 de = __fmul2_rn(d, e), dd = __fmul2_rn(d, __fmul2_rn(d, f2((float)(1.0 / 6.0))));
-   const float2 v3 = __fmul2_rn(v0, f2(3.0f));
-   const float2 alt_l = __ffma2_rn(r, f2(-2.0f), v3), alt_r = __ffma2_rn(l, f2(-2.0f), v3);
-   a0.x = (de.x > dd.x) ? alt_l.x : l.x;
-   a0.y = (de.y > dd.y) ? alt_l.y : l.y;
-   float2 nfr;
-   nfr.x = (-dd.x > de.x) ? alt_r.x : r.x;
-   nfr.y = (-dd.y > de.y) ? alt_r.y : r.y;
-   a1 = p_sub(__ffma2_rn(a0, f2(-2.0f), v3), nfr);
-   a2 = __ffma2_rn(v0, f2(-2.0f), __fadd2_rn(a0, nfr));
+// PPM of two columns in magnitudes (cpu_1d_ppm.hpp:35-54): l = |v0 - left
+// face|, r = |right face - v0| after the limiters; with the slope's sign s the
+// integral of the reconstruction from 0 to u is u (v0 + s (u-1) (l + u (r-l))).
+// A face outside its two cells' values gives half the superbee slope instead;
+// the Colella-Woodward corrections are l = min(l, 2r), r = min(r, 2l), of
+// which at most one acts; at an extremum s = 0 flattens the cell.
+__device__ __forceinline__ void ppm_magnitudes_x2(PpmWalk& c, float2 vm1, float2 v0, float2 vp1, float2 vp2, float2& s,
+                                                  float2& l, float2& r) {
+   const float2 a = p_minus(vp1, v0);
+   float2 h;
+   half_slope_x2(a, c.b, h, s);
+   const float2 fr = h4_face_x2(vm1, v0, vp1, vp2);
+   const float2 right = p_minus(fr, v0), next = p_minus(vp1, fr);
+   const float2 t = __fmul2_rn(right, next);
+   const bool or_x = t.x < 0.0f, or_y = t.y < 0.0f;
+   const float2 lf = make_float2(c.out_x ? h.x : c.left.x, c.out_y ? h.y : c.left.y);
+   const float2 rf = make_float2(or_x ? h.x : right.x, or_y ? h.y : right.y);
+   const float2 l2 = __fmul2_rn(lf, f2(2.0f)), r2 = __fmul2_rn(rf, f2(2.0f));
+   l = make_float2(fminf(fabsf(lf.x), fabsf(r2.x)), fminf(fabsf(lf.y), fabsf(r2.y)));
+   r = make_float2(fminf(fabsf(rf.x), fabsf(l2.x)), fminf(fabsf(rf.y), fabsf(l2.y)));
+   c.left = next;
+   c.b = a;
+   c.out_x = or_x;
+   c.out_y = or_y;
 }
 
 }  // namespace vlgpu

@@ -48,6 +48,7 @@
 // fused mode, FMA for the outgoing integral, and no h/h ratio for equal cell
 // widths.
 #include <cstdint>
+#include <type_traits>
 
 #include "fused_ppm.cuh"
 #include "vlgpu_common.cuh"
@@ -58,6 +59,7 @@ constexpr uint32_t NO_ROW = 0xffffffffu;
 constexpr uint32_t NO_DATA = 0xffffffffu;    // an added (all-zero) block of an adjusted list
 constexpr uint32_t BAD_ITEM = 0xffffffffu;   // item slot of a pencil that did not fit
 constexpr int UNION_THREADS = 512;
+constexpr uint32_t UNION_UNROLL = 4;         // pencil cells whose lists a thread reads at once
 constexpr int TR_THREADS = 256;
 constexpr uint32_t TR_MAX_N = 128;           // cells per pencil
 
@@ -192,13 +194,28 @@ __global__ void __launch_bounds__(UNION_THREADS) pencil_union_kernel(
    const uint32_t p = blockIdx.x;
    for (uint32_t w = threadIdx.x; w < n_words; w += blockDim.x) bm[w] = 0u;
    __syncthreads();
-   for (uint32_t x = 0; x < N; ++x) {
-      const CellSlot s = slots[pencil_cell(p, x, dim, nx, ny)];
-      for (uint32_t b = threadIdx.x; b < s.count; b += blockDim.x) {
-         const uint32_t g = gids[s.off + b];
-         atomicOr(&bm[g >> 5], 1u << (g & 31));
+   // the pencil's lists, UNION_UNROLL cells at a time so that their slots and
+   // IDs are on their way together: visit(x, list position, block ID)
+   auto for_blocks = [&](auto visit) {
+      for (uint32_t x0 = 0; x0 < N; x0 += UNION_UNROLL) {
+         CellSlot s[UNION_UNROLL];
+         uint32_t most = 0;
+#pragma unroll
+         for (uint32_t u = 0; u < UNION_UNROLL; ++u) {
+            s[u] = (x0 + u < N) ? slots[pencil_cell(p, x0 + u, dim, nx, ny)] : CellSlot{0u, 0u};
+            most = max(most, s[u].count);
+         }
+         for (uint32_t b = threadIdx.x; b < most; b += blockDim.x) {
+            uint32_t g[UNION_UNROLL];
+#pragma unroll
+            for (uint32_t u = 0; u < UNION_UNROLL; ++u) g[u] = (b < s[u].count) ? gids[s[u].off + b] : 0u;
+#pragma unroll
+            for (uint32_t u = 0; u < UNION_UNROLL; ++u)
+               if (b < s[u].count) visit(x0 + u, s[u].off + b, g[u]);
+         }
       }
-   }
+   };
+   for_blocks([&](uint32_t, uint32_t, uint32_t g) { atomicOr(&bm[g >> 5], 1u << (g & 31)); });
    __syncthreads();
    const uint32_t chunk = (n_words + blockDim.x - 1) / blockDim.x;
    const uint32_t w0 = min(n_words, threadIdx.x * chunk), w1 = min(n_words, w0 + chunk);
@@ -245,16 +262,12 @@ __global__ void __launch_bounds__(UNION_THREADS) pencil_union_kernel(
       srcs[row0 + e] = NO_DATA;
    }
    __syncthreads();
-   for (uint32_t x = 0; x < N; ++x) {
-      const CellSlot s = slots[pencil_cell(p, x, dim, nx, ny)];
-      for (uint32_t b = threadIdx.x; b < s.count; b += blockDim.x) {
-         const uint32_t g = gids[s.off + b];
-         const uint32_t w = g >> 5;
-         const uint32_t r = pre[w] + __popc(bm[w] & ((1u << (g & 31)) - 1u));
-         rows[row0 + (uint64_t)r * N + x] = s.off + b;
-         srcs[row0 + (uint64_t)r * N + x] = src_index ? src_index[s.off + b] : s.off + b;
-      }
-   }
+   for_blocks([&](uint32_t x, uint32_t at, uint32_t g) {
+      const uint32_t w = g >> 5;
+      const uint32_t r = pre[w] + __popc(bm[w] & ((1u << (g & 31)) - 1u));
+      rows[row0 + (uint64_t)r * N + x] = at;
+      srcs[row0 + (uint64_t)r * N + x] = src_index ? src_index[at] : at;
+   });
 }
 
 // ---------------------------------------------------------------------------
@@ -385,7 +398,8 @@ __global__ void __launch_bounds__(TR_THREADS) trans_remap_kernel(
 // fused translation remap: one warp per item (pencil, block ID)
 // ---------------------------------------------------------------------------
 constexpr int TF_THREADS = 256;
-constexpr int TF_BATCH = 8;  // cells per batch of the walk (16 measured slower)
+constexpr int TF_CTAS = 2;   // per SM
+constexpr int TF_BATCH = 8;   // cells per batch of the walk (16 measured slower)
 
 // Lanes whose columns share the plane (index along the sweep dimension) of
 // this lane's first column; a lane owns columns 2 lane and 2 lane + 1.  For
@@ -404,43 +418,16 @@ __device__ __forceinline__ int lane_plane(int lane) {
 }
 
 // Shift of plane k of the block at swapped index sw2 along the sweep
-// dimension, as fractions of the cell: outgoing integral over [z1, z2]
-// (cpu_trans_map_amr.cpp:60-80; fused arithmetic).
-__device__ __forceinline__ void plane_shift(uint32_t sw2, int k, float dvz, float vz_min, float dt, float h,
-                                            float& z1, float& z2, bool& up) {
+// dimension, as a fraction of the cell (cpu_trans_map_amr.cpp:60-80).  The
+// part that leaves a cell is the one above the edge w = 1 - z where the plane
+// moves up, the one below w = -z where it moves down; wm = w - 1.
+__device__ __forceinline__ void plane_shift(uint32_t sw2, int k, float dvz, float vz_min, float dt, float h, float& w,
+                                            float& wm, bool& up) {
    const float cell_vz = __double2float_rn(((double)(sw2 * WID + k) + 0.5) * (double)dvz + (double)vz_min);
    const float zt = __fdiv_rn(__fmul_rn(cell_vz, dt), h);
    up = zt > 0.0f;
-   z1 = up ? 1.0f - zt : 0.0f;
-   z2 = up ? 1.0f : -zt;
-}
-
-// The PPM (ppm_coeff_x2) and the outgoing integral over [z1, z2] of two
-// columns given their left and right faces; zero for a column whose plane is
-// skipped.
-__device__ __forceinline__ float2 outgoing_x2(float2 vm1, float2 v0, float2 vp1, float2 fl, float2 fr, float2 z1,
-                                              float2 z2, uint32_t act_x, uint32_t act_y) {
-   float2 a0, a1, a2;
-   ppm_coeff_x2(vm1, v0, vp1, fl, fr, a0, a1, a2);
-   const float2 t2 = __ffma2_rn(z2, __ffma2_rn(z2, a2, a1), a0);
-   const float2 t1 = __ffma2_rn(z1, __ffma2_rn(z1, a2, a1), a0);
-   const float2 ngbr = p_sub(__fmul2_rn(z2, t2), __fmul2_rn(z1, t1));
-   return make_float2(act_x ? ngbr.x : 0.0f, act_y ? ngbr.y : 0.0f);
-}
-
-// The same in the walk form (ppm_walk_x2): the left-face test and v0 - vm1
-// come in from the cell to the left, and this cell's go out in tl and dprev.
-__device__ __forceinline__ float2 outgoing_walk_x2(float2 v0, float2 vp1, float2 fl, float2 fr, float2& tl,
-                                                   float2& dprev, float2 z1, float2 z2, uint32_t act_x,
-                                                   uint32_t act_y) {
-   float2 a0, a1, a2, tr, dn;
-   ppm_walk_x2(v0, vp1, fl, fr, tl, dprev, tr, dn, a0, a1, a2);
-   tl = tr;
-   dprev = dn;
-   const float2 t2 = __ffma2_rn(z2, __ffma2_rn(z2, a2, a1), a0);
-   const float2 t1 = __ffma2_rn(z1, __ffma2_rn(z1, a2, a1), a0);
-   const float2 ngbr = p_sub(__fmul2_rn(z2, t2), __fmul2_rn(z1, t1));
-   return make_float2(act_x ? ngbr.x : 0.0f, act_y ? ngbr.y : 0.0f);
+   w = up ? 1.0f - zt : -zt;
+   wm = up ? -zt : -zt - 1.0f;
 }
 
 // This lane's two columns of the block at data index idx (zeros where the
@@ -466,9 +453,26 @@ __device__ __forceinline__ void plane_positive(float2 v, uint32_t pmask, uint32_
 // One warp per item walks the whole (periodic) pencil, L cells per batch.
 // Window index of cell c in the batch that outputs cells s0 .. s0+L-1 is
 // c - s0 + 3; the window holds cells s0-3 .. s0+L+2, the first six carried
-// over from the previous batch.  Carried along the walk: the left face fl of
-// the next cell and the outgoing integrals nb_m1, nb_0 of the two cells before
-// it, so every face and PPM is evaluated once per cell (plus two at the start).
+// over from the previous batch, and the next batch's L cells are on their way
+// while a batch is computed.  Carried along the walk: v - left face of the
+// next cell and its test, v0 - vm1, and the outgoing integrals nb_m1, nb_0 of
+// the two cells before it, so every face and PPM is evaluated once per cell
+// (plus two at the start).
+//
+// The reconstruction is the magnitude form of remap_pair_kernel (fused_ppm.cuh,
+// ppm_magnitudes_x2), whose integral from 0 to w, w (v0 + s (w-1) (l + w (r-l))),
+// gives the outgoing part either way: it, or v0 minus it, as its value at 1 is
+// v0 exactly.
+//
+// A plane is left out (check_skip_remapping) where no value of the five cells
+// around is positive.  Nearly every value is positive, so a batch whose whole
+// window is skips the tests: one vote instead of a ballot per cell and plane.
+//
+// Bound by issue and latency (56% of issue slots, 16 warps per SM): 126 to
+// 190 instructions per block at pencils of 7 to 21 cells against 210 with a
+// ballot per cell and the faces selected; the three sweeps of a 21 x 9 x 7 grid,
+// packing included, 1076 -> 892 us.  Batches of 4 cells at 3 or 4 CTAs per SM
+// take the same time.
 //
 // The item's header and tables live in the warp's slice of shared memory,
 // double-buffered: [0] pencil, [1] block ID, tsrc[m] (m = 0 .. N+5) = data
@@ -489,7 +493,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 __host__ __device__ constexpr uint32_t tf_slice_words(uint32_t N) { return 2 * N + 8; }
 
 template <int DIM, int L>
-__global__ void __launch_bounds__(TF_THREADS, 3) trans_fused_kernel(
+__global__ void __launch_bounds__(TF_THREADS, TF_CTAS) trans_fused_kernel(
    const uint32_t* __restrict__ item_gid, const uint32_t* __restrict__ item_pencil, const uint32_t* __restrict__ rows,
    const uint32_t* __restrict__ srcs, const TransCounters* __restrict__ tc, uint32_t item_cap, uint64_t row_cap,
    const float* __restrict__ src, float* __restrict__ dst, uint32_t* __restrict__ dst_gids, MeshDev mesh,
@@ -544,83 +548,115 @@ __global__ void __launch_bounds__(TF_THREADS, 3) trans_fused_kernel(
 
       uint32_t sw[3];
       swapped_indices(gid, mesh.len, DIM, sw);
-      float2 z1, z2;
+      float2 we, wm;
       bool upx, upy;
-      plane_shift(sw[2], kx, dvz, vz_min, dt, h, z1.x, z2.x, upx);
-      plane_shift(sw[2], ky, dvz, vz_min, dt, h, z1.y, z2.y, upy);
+      plane_shift(sw[2], kx, dvz, vz_min, dt, h, we.x, wm.x, upx);
+      plane_shift(sw[2], ky, dvz, vz_min, dt, h, we.y, wm.y, upy);
+      // outgoing = share v0 + turn I(we)
+      const float2 share = make_float2(upx ? 1.0f : 0.0f, upy ? 1.0f : 0.0f);
+      const float2 turn = make_float2(upx ? -1.0f : 1.0f, upy ? -1.0f : 1.0f);
 
-      // window cells -3 .. L+2 of the first batch (past N+2: not needed)
+      // window cells -3 .. L+2 of the first batch (past N+2: not needed, any
+      // positive value)
       float2 w[W];
-      uint32_t posx = 0u, posy = 0u;  // bit j: positive value in window cell j
+      auto window_cell = [&](uint32_t m) {
+         return (m < N + 6) ? load_column_pair(src, tsrc[m], lane) : make_float2(1.0f, 1.0f);
+      };
 #pragma unroll
-      for (int j = 0; j < W; ++j) w[j] = load_column_pair(src, ((uint32_t)j < N + 6) ? tsrc[j] : NO_DATA, lane);
+      for (int j = 0; j < W; ++j) w[j] = window_cell((uint32_t)j);
+      // every value of the window's first six cells positive / of the others
+      auto positive = [&](int j0, int j1) {
+         float m = 1.0f;
 #pragma unroll
-      for (int j = 0; j < W; ++j) {
-         uint32_t px, py;
-         plane_positive<DIM>(w[j], pmask, px, py);
-         posx |= px << j;
-         posy |= py << j;
-      }
-      // the outgoing integrals of cells -1 and 0, the left face of cell 1
-      // and, carried along the walk, its left-face test and v0 - vm1
-      float2 nb_m1, nb_0, fl, tl, dprev;
+         for (int j = j0; j < j1; ++j) m = fminf(m, fminf(w[j].x, w[j].y));
+         return (bool)__all_sync(0xffffffffu, m > 0.0f);
+      };
+      // (columns of a plane in other lanes: bit j, some positive value in window cell j)
+      auto plane_bits = [&](uint32_t& posx, uint32_t& posy) {
+         posx = posy = 0u;
+#pragma unroll
+         for (int j = 0; j < W; ++j) {
+            uint32_t px, py;
+            plane_positive<DIM>(w[j], pmask, px, py);
+            posx |= px << j;
+            posy |= py << j;
+         }
+      };
+      PpmWalk walk;
+      float2 nb_m1, nb_0;
+      // the outgoing integral of the cell v0 with neighbours vm1, vp1, vp2
+      auto outgoing = [&](float2 vm1, float2 v0, float2 vp1, float2 vp2) {
+         float2 s, l, r;
+         ppm_magnitudes_x2(walk, vm1, v0, vp1, vp2, s, l, r);
+         const float2 T = __ffma2_rn(we, p_minus(r, l), l);
+         const float2 I = __fmul2_rn(we, __ffma2_rn(__fmul2_rn(s, wm), T, v0));
+         return __ffma2_rn(turn, I, __fmul2_rn(share, v0));
+      };
+      bool head = positive(0, 6);
       {
-         const uint32_t ax = posx | (posx << 1) | (posx << 2) | (posx >> 1) | (posx >> 2);
-         const uint32_t ay = posy | (posy << 1) | (posy << 2) | (posy >> 1) | (posy >> 2);
-         const float2 fm1 = h4_face_x2(w[0], w[1], w[2], w[3]);
-         const float2 f0 = h4_face_x2(w[1], w[2], w[3], w[4]);
-         fl = h4_face_x2(w[2], w[3], w[4], w[5]);
-         tl = __fmul2_rn(p_sub(w[1], fm1), p_sub(fm1, w[2]));
-         dprev = p_sub(w[2], w[1]);
-         nb_m1 = outgoing_walk_x2(w[2], w[3], fm1, f0, tl, dprev, z1, z2, (ax >> 2) & 1u, (ay >> 2) & 1u);
-         nb_0 = outgoing_walk_x2(w[3], w[4], f0, fl, tl, dprev, z1, z2, (ax >> 3) & 1u, (ay >> 3) & 1u);
+         // cells -1 and 0
+         walk.start(w[0], w[1], w[2], w[3]);
+         nb_m1 = outgoing(w[1], w[2], w[3], w[4]);
+         nb_0 = outgoing(w[2], w[3], w[4], w[5]);
+         if (!head) {
+            uint32_t posx, posy;
+            plane_bits(posx, posy);
+            const uint32_t ax = posx | (posx << 1) | (posx << 2) | (posx >> 1) | (posx >> 2);
+            const uint32_t ay = posy | (posy << 1) | (posy << 2) | (posy >> 1) | (posy >> 2);
+            if (!((ax >> 2) & 1u)) nb_m1.x = 0.0f;
+            if (!((ay >> 2) & 1u)) nb_m1.y = 0.0f;
+            if (!((ax >> 3) & 1u)) nb_0.x = 0.0f;
+            if (!((ay >> 3) & 1u)) nb_0.y = 0.0f;
+         }
       }
 
       for (uint32_t s0 = 0;;) {
-         // bit j: some positive value in window cells j-2 .. j+2 (the plane is
-         // remapped for that cell; check_skip_remapping)
-         const uint32_t ax = posx | (posx << 1) | (posx << 2) | (posx >> 1) | (posx >> 2);
-         const uint32_t ay = posy | (posy << 1) | (posy << 2) | (posy >> 1) | (posy >> 2);
+         float2 nx[L];  // the next batch's new cells s0+L+3 .. s0+2L+2
 #pragma unroll
-         for (int i = 0; i < L; ++i) {
-            // cell y = s0+1+i (window i+4): its right face and outgoing integral;
-            // then the new value of cell y-1 = s0+i (window i+3)
-            const float2 fr = h4_face_x2(w[i + 3], w[i + 4], w[i + 5], w[i + 6]);
-            const float2 nb = outgoing_walk_x2(w[i + 4], w[i + 5], fl, fr, tl, dprev, z1, z2, (ax >> (i + 4)) & 1u,
-                                               (ay >> (i + 4)) & 1u);
-            fl = fr;
-            const uint32_t r = (s0 + (uint32_t)i < N) ? trow[s0 + i] : NO_ROW;
-            if (r != NO_ROW) {
-               float2 out;
-               out.x = ((ax >> (i + 3)) & 1u) ? w[i + 3].x - nb_0.x : 0.0f;
-               out.y = ((ay >> (i + 3)) & 1u) ? w[i + 3].y - nb_0.y : 0.0f;
-               out.x = out.x + (upx ? nb_m1.x : nb.x);
-               out.y = out.y + (upy ? nb_m1.y : nb.y);
-               reinterpret_cast<float2*>(dst + (size_t)r * WID3)[lane] = out;
-               if (lane == 0) dst_gids[r] = gid;
+         for (int j = 0; j < L; ++j) nx[j] = window_cell(s0 + (uint32_t)(L + 6 + j));
+         // cell y = s0+1+i (window i+4): its outgoing integral; then the new
+         // value of cell y-1 = s0+i (window i+3)
+         auto batch = [&](auto test, uint32_t ax, uint32_t ay) {
+#pragma unroll
+            for (int i = 0; i < L; ++i) {
+               if (s0 + (uint32_t)i >= N) break;  // the last batch of a pencil may be short
+               float2 nb = outgoing(w[i + 3], w[i + 4], w[i + 5], w[(i + 6 < W) ? i + 6 : W - 1]);
+               if constexpr (decltype(test)::value) {
+                  if (!((ax >> (i + 4)) & 1u)) nb.x = 0.0f;
+                  if (!((ay >> (i + 4)) & 1u)) nb.y = 0.0f;
+               }
+               const uint32_t r = trow[s0 + i];
+               if (r != NO_ROW) {
+                  float2 own = p_minus(w[i + 3], nb_0);
+                  if constexpr (decltype(test)::value) {
+                     if (!((ax >> (i + 3)) & 1u)) own.x = 0.0f;
+                     if (!((ay >> (i + 3)) & 1u)) own.y = 0.0f;
+                  }
+                  const float2 out = __fadd2_rn(own, make_float2(upx ? nb_m1.x : nb.x, upy ? nb_m1.y : nb.y));
+                  reinterpret_cast<float2*>(dst + (size_t)r * WID3)[lane] = out;
+                  if (lane == 0) dst_gids[r] = gid;
+               }
+               nb_m1 = nb_0;
+               nb_0 = nb;
             }
-            nb_m1 = nb_0;
-            nb_0 = nb;
+         };
+         const bool tail = positive(6, W);
+         if (head && tail) {
+            batch(std::false_type{}, 0u, 0u);
+         } else {
+            // bit j: some positive value in window cells j-2 .. j+2
+            uint32_t posx, posy;
+            plane_bits(posx, posy);
+            batch(std::true_type{}, posx | (posx << 1) | (posx << 2) | (posx >> 1) | (posx >> 2),
+                  posy | (posy << 1) | (posy << 2) | (posy >> 1) | (posy >> 2));
          }
+         head = tail;
          s0 += L;
          if (s0 >= N) break;
-         // next batch: carry six cells, load cells s0+3 .. s0+L+2
 #pragma unroll
          for (int j = 0; j < 6; ++j) w[j] = w[L + j];
-         posx >>= L;
-         posy >>= L;
 #pragma unroll
-         for (int j = 0; j < L; ++j) {
-            const uint32_t m = s0 + 6u + (uint32_t)j;
-            w[6 + j] = load_column_pair(src, (m < N + 6) ? tsrc[m] : NO_DATA, lane);
-         }
-#pragma unroll
-         for (int j = 0; j < L; ++j) {
-            uint32_t px, py;
-            plane_positive<DIM>(w[6 + j], pmask, px, py);
-            posx |= px << (6 + j);
-            posy |= py << (6 + j);
-         }
+         for (int j = 0; j < L; ++j) w[6 + j] = nx[j];
       }
    }
 }
