@@ -1,11 +1,12 @@
-"""Columnize takes a cell per CTA, with larger CTAs where the cells are few.  A
-cell's step must not depend on that: the same cells alone, beside a few and
-beside many others come out bit-identical, and their adjustment and moments
-equal the oracle's.
+"""The kernels that take a cell per CTA (columnize, the adjustment's lists)
+run with larger CTAs where the cells are few, and the adjustment's values are
+summed in parts of about 128 blocks.  A cell's step must not depend on any of
+that: the same cells alone, beside a few and beside many others come out
+bit-identical, and equal to the oracle's adjustment and moments.
 
-Sizes: no block, one block, the edges of a CTA's passes (127 to 129, 255 to
-257 blocks), a cell of 9000 blocks, and a cell whose transverse plane exceeds
-the capped columnize launch (1024 entries)."""
+Sizes: no block, one block, the edges of a staged tile and of a part (127 to
+129, 255 to 257 blocks), more blocks than 64 parts of 128, and a cell whose
+transverse plane exceeds the capped columnize launch (1024 entries)."""
 import numpy as np
 import pytest
 

@@ -11,18 +11,22 @@
 // in H are removed and their mass sum(f)*dv^3 is added to RHOLOSSADJUST,
 // blocks of H that did not exist are added with zero data.
 //
-// Persistent CTAs of 256 threads, one cell at a time, the largest cells
-// first.  The content set and H live in shared memory as 96-bit x-masks over
-// the (y,z) rows of the cell's dilated bounding box.  The output
+// adjust_kernel makes the lists: persistent CTAs, one cell at a time, the
+// largest cells first.  The content set and H live in shared memory as 96-bit
+// x-masks over the (y,z) rows of the cell's dilated bounding box.  The output
 // is a new block list sorted by global ID plus, per block, the index of its
 // data in the current pool (or none for an added block): no VDF value is
 // copied, the next sweep reads the kept blocks where they are.
+// adjust_values_kernel then reads the old blocks' values once, in parts of
+// about 128 blocks over all SMs: RHOLOSSADJUST and the "_V" moments.
 //
 // On a grid, content_mask_kernel first writes every cell's content mask once
 // (its content bounding box and the x-mask rows over it, in a pool), so that
 // a cell ORs its 26 neighbours' mask rows instead of walking their block
 // lists; a cell whose mask did not fit (box too large, pool full) is read from
 // its list as before.
+#include <cfloat>
+#include <cmath>
 #include <cstdint>
 
 #include "moments_record.cuh"
@@ -31,11 +35,20 @@
 namespace vlgpu {
 
 constexpr int ADJ_THREADS = 256;
-constexpr int ADJ_MIN_CTAS = 3;   // CTAs per SM the register budget is set for
-constexpr int ADJ_UNROLL = 4;     // list entries per thread in flight
-constexpr uint32_t ADJ_QUEUE = 32 * ADJ_UNROLL;  // old blocks a warp queues per pass
-constexpr uint32_t ADJ_KEPT = 0x80000000u;       // queue flag: the block stays
+constexpr int ADJ_FEW_THREADS = 1024;  // list CTAs where the cells do not outnumber the SMs
+constexpr int ADJ_ROWS = 2;           // rows a lane has in flight, and as many on their way
+constexpr int ADJ_VALUE_CTAS = 3;         // CTAs per SM of the pass over the values
+constexpr int ADJ_UNROLL = 4;          // list entries per thread in flight
+constexpr uint32_t ADJ_TILE = 128;     // old blocks of a part staged at a time
+constexpr uint32_t ADJ_KEPT = 0x80000000u;  // staged positions: the block stays
 constexpr uint32_t NO_BLOCK = 0xffffffffu;
+
+// Parts of the pass over the values of a cell with `count` old blocks: about
+// ADJ_TILE blocks each, at most MOM_PARTS_PER_CELL.
+__host__ __device__ __forceinline__ uint32_t value_parts(uint32_t count) {
+   const uint32_t p = (count + ADJ_TILE - 1) / ADJ_TILE;
+   return p < (uint32_t)MOM_PARTS_PER_CELL ? p : (uint32_t)MOM_PARTS_PER_CELL;
+}
 
 __device__ __forceinline__ uint32_t adj_exclusive_scan(uint32_t v, uint32_t* warp_sums, uint32_t& total) {
    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -64,17 +77,39 @@ __device__ __forceinline__ uint32_t adj_exclusive_scan(uint32_t v, uint32_t* war
    return before + x - v;
 }
 
-// Content of one block: any of its 64 values >= min_value (compared in
-// double, as the reference compares Realf data with the Real threshold).
-__device__ __forceinline__ bool block_has_content(const float* __restrict__ blk, double min_value) {
-   const float4* q = reinterpret_cast<const float4*>(blk);
-   bool c = false;
-   for (int i = 0; i < 16; ++i) {
-      const float4 v = __ldg(q + i);
-      c |= ((double)v.x >= min_value) | ((double)v.y >= min_value) | ((double)v.z >= min_value) |
-           ((double)v.w >= min_value);
+// Content flags of a list whose values no sweep has just written
+// (compute_block_has_content: any of a block's 64 values >= the threshold; an
+// added block has none), one byte per row.  Half a warp per block, four blocks
+// in flight, the blocks of a cell over the gridDim.y CTAs of its column: one
+// coalesced read of the VDF, where the list CTAs read it twice with a thread
+// per block.
+// Adjustment, moments and packing of 1024 cells (1.45 M blocks): 1446 -> 1279 us.
+constexpr int FLAG_THREADS = 256;
+constexpr uint32_t FLAG_BLOCKS = 4 * FLAG_THREADS / 16;  // blocks a CTA reads per pass
+__global__ void __launch_bounds__(FLAG_THREADS) content_flags_kernel(const uint32_t* __restrict__ src_index,
+                                                                     const CellSlot* __restrict__ slots,
+                                                                     const float* __restrict__ data, float threshold,
+                                                                     uint8_t* __restrict__ content) {
+   const CellSlot s = slots[blockIdx.x];
+   const uint32_t sub = threadIdx.x & 15, hw = threadIdx.x >> 4, half = (threadIdx.x >> 4) & 1;
+   for (uint32_t b0 = blockIdx.y * FLAG_BLOCKS; b0 < s.count; b0 += gridDim.y * FLAG_BLOCKS) {
+      float4 v[4];
+#pragma unroll
+      for (uint32_t u = 0; u < 4; ++u) {
+         const uint32_t b = b0 + hw + u * (FLAG_THREADS / 16);
+         v[u] = make_float4(-1.f, -1.f, -1.f, -1.f);  // the threshold is positive
+         if (b < s.count) {
+            const uint32_t row = src_index ? src_index[s.off + b] : s.off + b;
+            if (row != NO_BLOCK) v[u] = __ldg(reinterpret_cast<const float4*>(data + (size_t)row * WID3) + sub);
+         }
+      }
+#pragma unroll
+      for (uint32_t u = 0; u < 4; ++u) {
+         const uint32_t b = b0 + hw + u * (FLAG_THREADS / 16);
+         const unsigned any = __ballot_sync(0xffffffffu, fmaxf(fmaxf(v[u].x, v[u].y), fmaxf(v[u].z, v[u].w)) >= threshold);
+         if (sub == 0 && b < s.count) content[s.off + b] = ((any >> (16 * half)) & 0xffffu) ? 1 : 0;
+      }
    }
-   return c;
 }
 
 __device__ __forceinline__ uint32_t shl96(uint32_t w0, uint32_t w1, uint32_t w2, int word, int s) {
@@ -91,15 +126,6 @@ __device__ __forceinline__ uint32_t shr96(uint32_t w0, uint32_t w1, uint32_t w2,
    return w2 >> s;
 }
 
-__device__ __forceinline__ bool list_block_content(const uint32_t* __restrict__ src_index,
-                                                   const uint8_t* __restrict__ content,
-                                                   const float* __restrict__ data, uint32_t pos, double min_value) {
-   const uint32_t idx = src_index ? src_index[pos] : pos;
-   if (idx == NO_BLOCK) return false;
-   if (content) return content[pos] != 0;
-   return block_has_content(data + (size_t)idx * WID3, min_value);
-}
-
 constexpr uint32_t NO_MASK = 0xffffffffu;
 constexpr int MASK_THREADS = 256;
 constexpr uint32_t MASK_SMEM_ROWS = 1600;
@@ -108,9 +134,8 @@ constexpr uint32_t MASK_SMEM_ROWS = 1600;
 // the content x-mask rows, copied to the pool at an offset taken from
 // pool_top.
 __global__ void __launch_bounds__(MASK_THREADS) content_mask_kernel(
-   const uint32_t* __restrict__ gids, const uint32_t* __restrict__ src_index, const CellSlot* __restrict__ slots,
-   const uint8_t* __restrict__ content, const float* __restrict__ data, MeshDev mesh, double min_value,
-   MaskRec* __restrict__ recs, uint32_t* __restrict__ pool, uint32_t* __restrict__ pool_top, uint32_t pool_cap) {
+   const uint32_t* __restrict__ gids, const CellSlot* __restrict__ slots, const uint8_t* __restrict__ content,
+   MeshDev mesh, MaskRec* __restrict__ recs, uint32_t* __restrict__ pool, uint32_t* __restrict__ pool_top, uint32_t pool_cap) {
    __shared__ uint32_t C[3 * MASK_SMEM_ROWS];
    __shared__ int s_box[4];
    __shared__ uint32_t s_off;
@@ -126,7 +151,7 @@ __global__ void __launch_bounds__(MASK_THREADS) content_mask_kernel(
    {
       int y0 = 1 << 20, y1 = -1, z0 = 1 << 20, z1 = -1;
       for (uint32_t b = threadIdx.x; b < s.count; b += blockDim.x) {
-         if (list_block_content(src_index, content, data, s.off + b, min_value)) {
+         if (content[s.off + b] != 0) {
             const uint32_t g = gids[s.off + b];
             uint32_t bx, by, bz;
             block_xyz(mesh, g, bx, by, bz);
@@ -148,7 +173,7 @@ __global__ void __launch_bounds__(MASK_THREADS) content_mask_kernel(
    for (uint32_t q = threadIdx.x; q < 3 * rows; q += blockDim.x) C[q] = 0u;
    __syncthreads();
    for (uint32_t b = threadIdx.x; b < s.count; b += blockDim.x) {
-      if (list_block_content(src_index, content, data, s.off + b, min_value)) {
+      if (content[s.off + b] != 0) {
          const uint32_t g = gids[s.off + b];
          uint32_t x, by, bz;
          block_xyz(mesh, g, x, by, bz);
@@ -171,32 +196,30 @@ __global__ void __launch_bounds__(MASK_THREADS) content_mask_kernel(
       for (uint32_t q = threadIdx.x; q < 3 * rows; q += blockDim.x) pool[off + q] = C[q];
 }
 
-// One cell at a time per CTA of ADJ_THREADS threads; persistent CTAs take
-// the cells from a counter in the order `order` gives (largest first), so
+// The lists.  One cell at a time per CTA of THREADS threads; persistent CTAs
+// take the cells from a counter in the order `order` gives (largest first), so
 // the longest cells start first and the rest balance over the CTAs.  Per
 // cell: the content bounding box, the content mask C (one shared-memory OR
 // per content block, after the lanes of a warp that set bits of the same
 // word combine them), the dilated set H row by row, the neighbours' content,
 // an exclusive scan of the row counts, the GID-sorted output list, and a pass
-// over the old blocks that points kept entries at their data and sums the
-// removed ones (a half-warp per removed block, float4 rows).
-__global__ void __launch_bounds__(ADJ_THREADS, ADJ_MIN_CTAS) adjust_kernel(
+// over the old list that points kept entries at their data and marks them in
+// `kept`.  The values are read by adjust_values_kernel, in the parts this
+// kernel appends to `items`.
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS) adjust_kernel(
    const uint32_t* __restrict__ gids, const uint32_t* __restrict__ src_index, const CellSlot* __restrict__ slots,
-   const uint8_t* __restrict__ content, const float* __restrict__ data, const int32_t* __restrict__ neighbors,
+   const uint8_t* __restrict__ content, const int32_t* __restrict__ neighbors,
    uint32_t* __restrict__ out_gids, uint32_t* __restrict__ out_src, CellSlot* __restrict__ out_slots,
-   double* __restrict__ loss, uint32_t* __restrict__ status, SweepCounters* __restrict__ counters,
-   uint32_t out_capacity, MeshDev mesh, double min_value, int add_width, double dv3, uint32_t n_cells,
+   uint32_t* __restrict__ status, SweepCounters* __restrict__ counters,
+   uint32_t out_capacity, MeshDev mesh, int add_width, uint32_t n_cells,
    uint32_t smem_rows, uint32_t* __restrict__ scratch, const MaskRec* __restrict__ masks,
-   const uint32_t* __restrict__ pool, const uint32_t* __restrict__ order, double* __restrict__ mom_record,
-   double* __restrict__ pivot, int write_pivot, MomentFrame fr) {
+   const uint32_t* __restrict__ pool, const uint32_t* __restrict__ order, uint8_t* __restrict__ kept,
+   AdjustItem* __restrict__ items, double* __restrict__ mom_record, double* __restrict__ pivot, int write_pivot) {
    extern __shared__ uint32_t smem[];
    __shared__ uint32_t warp_sums[32];
    __shared__ int s_box[8];
-   __shared__ uint32_t s_base, s_flags, s_item;
-   __shared__ double s_loss[ADJ_THREADS / 32];
-   __shared__ double s_mom[ADJ_THREADS / 32][10];            // the warps' moment sums
-   __shared__ uint32_t s_qidx[ADJ_THREADS / 32][ADJ_QUEUE];  // a warp's queue of old blocks: data row
-   __shared__ uint32_t s_qgid[ADJ_THREADS / 32][ADJ_QUEUE];  // and block ID (| ADJ_KEPT when kept)
+   __shared__ uint32_t s_base, s_flags, s_item, s_part;
    __shared__ MaskRec s_rec[27];     // the neighbours' content masks (26: the cell's own)
    __shared__ uint32_t s_first[27];  // first mask-row item of each neighbour
    constexpr uint32_t FULL = 0xffffffffu;
@@ -244,13 +267,13 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_MIN_CTAS) adjust_kernel(
          }
       } else {
          int y0 = 1 << 20, y1 = -1, z0 = 1 << 20, z1 = -1;
-         for (uint32_t b0 = threadIdx.x; b0 < s.count; b0 += ADJ_THREADS * ADJ_UNROLL) {
+         for (uint32_t b0 = threadIdx.x; b0 < s.count; b0 += THREADS * ADJ_UNROLL) {
             bool c[ADJ_UNROLL];
             uint32_t g[ADJ_UNROLL];
 #pragma unroll
             for (int u = 0; u < ADJ_UNROLL; ++u) {
-               const uint32_t b = b0 + ADJ_THREADS * u;
-               c[u] = b < s.count && list_block_content(src_index, content, data, s.off + b, min_value);
+               const uint32_t b = b0 + THREADS * u;
+               c[u] = b < s.count && content[s.off + b] != 0;
                g[u] = b < s.count ? gids[s.off + b] : 0u;
             }
 #pragma unroll
@@ -279,8 +302,8 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_MIN_CTAS) adjust_kernel(
             const int32_t nc = neighbors[(size_t)cell * 26 + q];
             if (nc < 0 || s_rec[q].off != NO_MASK) continue;
             const CellSlot ns = slots[nc];
-            for (uint32_t b = threadIdx.x; b < ns.count; b += ADJ_THREADS) {
-               if (list_block_content(src_index, content, data, ns.off + b, min_value)) {
+            for (uint32_t b = threadIdx.x; b < ns.count; b += THREADS) {
+               if (content[ns.off + b] != 0) {
                   uint32_t bx, by, bz;
                   block_xyz(mesh, gids[ns.off + b], bx, by, bz);
                   ny0 = min(ny0, (int)by); ny1 = max(ny1, (int)by);
@@ -317,7 +340,7 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_MIN_CTAS) adjust_kernel(
    uint32_t* C = base;              // 3 * rows
    uint32_t* H = base + 3 * rows;   // 3 * rows
    uint32_t* prefix = base + 6 * rows;  // rows
-   for (uint32_t q = threadIdx.x; q < 3 * rows; q += ADJ_THREADS) C[q] = 0;
+   for (uint32_t q = threadIdx.x; q < 3 * rows; q += THREADS) C[q] = 0;
    __syncthreads();
    // pass 2: content mask rows (copied from the cell's own mask when it has one)
    if (s_rec[26].off != NO_MASK) {
@@ -325,20 +348,20 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_MIN_CTAS) adjust_kernel(
       if (m.y1 >= 0) {
          const int my = m.y1 - m.y0 + 1;
          const uint32_t mrows = (uint32_t)(my * (m.z1 - m.z0 + 1));
-         for (uint32_t q = threadIdx.x; q < 3 * mrows; q += ADJ_THREADS) {
+         for (uint32_t q = threadIdx.x; q < 3 * mrows; q += THREADS) {
             const uint32_t mr = q / 3, w = q - 3 * mr;
             const int y = m.y0 + (int)(mr % my), z = m.z0 + (int)(mr / my);
             C[3 * (uint32_t)((z - z0) * ny + (y - y0)) + w] = pool[m.off + q];
          }
       }
    } else if (own_any) {
-      for (uint32_t b0 = warp * 32; b0 < s.count; b0 += ADJ_THREADS * ADJ_UNROLL) {
+      for (uint32_t b0 = warp * 32; b0 < s.count; b0 += THREADS * ADJ_UNROLL) {
          bool cc[ADJ_UNROLL];
          uint32_t gg[ADJ_UNROLL];
 #pragma unroll
          for (int u = 0; u < ADJ_UNROLL; ++u) {
-            const uint32_t b = b0 + ADJ_THREADS * u + lane;
-            cc[u] = b < s.count && list_block_content(src_index, content, data, s.off + b, min_value);
+            const uint32_t b = b0 + THREADS * u + lane;
+            cc[u] = b < s.count && content[s.off + b] != 0;
             gg[u] = b < s.count ? gids[s.off + b] : 0u;
          }
 #pragma unroll
@@ -367,7 +390,7 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_MIN_CTAS) adjust_kernel(
    }
    __syncthreads();
    // dilation: H(y,z) = OR over |dy|,|dz| <= w of the row dilated along x
-   const uint32_t chunk = (rows + ADJ_THREADS - 1) / ADJ_THREADS;
+   const uint32_t chunk = (rows + THREADS - 1) / THREADS;
    const uint32_t r0 = min(rows, threadIdx.x * chunk), r1 = min(rows, r0 + chunk);
    for (uint32_t r = r0; r < r1; ++r) {
       const int yy = y0 + (int)(r % ny), zz = z0 + (int)(r / ny);
@@ -410,7 +433,7 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_MIN_CTAS) adjust_kernel(
          __syncthreads();
          const uint32_t items = s_first[26];
          int q = 0;
-         for (uint32_t it = threadIdx.x; it < items; it += ADJ_THREADS) {
+         for (uint32_t it = threadIdx.x; it < items; it += THREADS) {
             while (it >= s_first[q + 1]) ++q;
             const MaskRec& m = s_rec[q];
             const uint32_t mr = it - s_first[q];
@@ -429,8 +452,8 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_MIN_CTAS) adjust_kernel(
          const int32_t nc = neighbors[(size_t)cell * 26 + q];
          if (nc < 0 || s_rec[q].off != NO_MASK) continue;
          const CellSlot ns = slots[nc];
-         for (uint32_t b = threadIdx.x; b < ns.count; b += ADJ_THREADS) {
-            if (list_block_content(src_index, content, data, ns.off + b, min_value)) {
+         for (uint32_t b = threadIdx.x; b < ns.count; b += THREADS) {
+            if (content[ns.off + b] != 0) {
                uint32_t x, by, bz;
                block_xyz(mesh, gids[ns.off + b], x, by, bz);
                const uint32_t r = (uint32_t)(((int)bz - z0) * ny + ((int)by - y0));
@@ -475,155 +498,230 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_MIN_CTAS) adjust_kernel(
       }
    }
    __syncthreads();
-   // old blocks: kept ones point the new entry at their data, removed ones
-   // feed the density loss; with the moments fused, the kept blocks' values
-   // also give the cell's "_V" moments (MOM_BOTH: the first sums about 0, the
-   // second about the pivot's bulk velocity U)
-   const bool fuse = mom_record != nullptr;
-   double U0 = 0.0, U1 = 0.0, U2 = 0.0;
-   if (fuse) {
-      const double* pv = pivot + (size_t)cell * MOM_COUNT;
-      U0 = pv[MOM_VX]; U1 = pv[MOM_VY]; U2 = pv[MOM_VZ];
-   }
-   // half a warp per queued block, one x-row of four cells per lane
-   const uint32_t half = lane >> 4, sub = lane & 15;
-   const double ox = 0.5 * fr.dv[0], oy = ((sub & 3) + 0.5) * fr.dv[1], oz = ((sub >> 2) + 0.5) * fr.dv[2];
-   const double dv0s = fr.dv[0] * fr.dv[0];
-   double t[10];
-#pragma unroll
-   for (int q = 0; q < 10; ++q) t[q] = 0.0;
-   double lsum = 0.0;  // sum f of the removed blocks (times dv3 below)
-   uint32_t* const qidx = s_qidx[warp];
-   uint32_t* const qgid = s_qgid[warp];
-   const uint32_t lanes_below = (1u << lane) - 1u;
-   for (uint32_t b0 = warp * 32; b0 < s.count; b0 += ADJ_THREADS * ADJ_UNROLL) {
-      uint32_t qn = 0;
+   // old blocks: kept ones point the new entry at their data; marked for the
+   // pass over the values
+   for (uint32_t b0 = threadIdx.x; b0 < s.count; b0 += THREADS * ADJ_UNROLL) {
       uint32_t gg[ADJ_UNROLL], ii[ADJ_UNROLL];
 #pragma unroll
       for (int u = 0; u < ADJ_UNROLL; ++u) {
-         const uint32_t b = b0 + ADJ_THREADS * u + lane;
-         gg[u] = b < s.count ? gids[s.off + b] : 0u;
-         ii[u] = b < s.count ? (src_index ? src_index[s.off + b] : s.off + b) : NO_BLOCK;
+         const uint32_t b = b0 + THREADS * u, at = s.off + (b < s.count ? b : b0);
+         gg[u] = gids[at];
+         ii[u] = src_index ? src_index[at] : at;
       }
 #pragma unroll
       for (int u = 0; u < ADJ_UNROLL; ++u) {
-         const bool valid = b0 + ADJ_THREADS * u + lane < s.count;
+         const uint32_t b = b0 + THREADS * u;
+         if (b >= s.count) break;
          uint32_t x, by, bz;
          block_xyz(mesh, gg[u], x, by, bz);
          const int y = (int)by, z = (int)bz;
          bool inH = false;
-         uint32_t pos = 0;
-         if (valid && any && y >= y0 && y <= y1 && z >= z0 && z <= z1) {
+         if (any && y >= y0 && y <= y1 && z >= z0 && z <= z1) {
             const uint32_t r = (uint32_t)((z - z0) * ny + (y - y0));
             inH = (H[3 * r + (x >> 5)] >> (x & 31)) & 1u;
-            pos = prefix[r] + (uint32_t)mask_popc_below(&H[3 * r], x);
+            if (inH && ok) out_src[obase + prefix[r] + (uint32_t)mask_popc_below(&H[3 * r], x)] = ii[u];
          }
-         if (inH && ok) out_src[obase + pos] = ii[u];
-         // queue the blocks whose values are read: the removed ones, and with
-         // the moments fused the kept ones too
-         const bool read = valid && ii[u] != NO_BLOCK && (fuse || !inH);
-         const uint32_t bal = __ballot_sync(FULL, read);
-         if (read) {
-            const uint32_t q = qn + __popc(bal & lanes_below);
-            qidx[q] = ii[u];
-            qgid[q] = gg[u] | (inH ? ADJ_KEPT : 0u);
-         }
-         qn += __popc(bal);
-      }
-      __syncwarp();
-      // the queue, eight blocks at a time: half-warp h reads blocks
-      // h, h + 2, h + 4, h + 6; the next eight blocks' rows are in flight
-      // while these are summed
-      auto fetch = [&](uint32_t q0, float4* f, uint32_t* gq) {
-#pragma unroll
-         for (int v = 0; v < 4; ++v) {
-            const uint32_t e = q0 + half + 2 * v;
-            gq[v] = e < qn ? qgid[e] : 0xffffffffu;
-            f[v] = e < qn ? __ldg(reinterpret_cast<const float4*>(data + (size_t)qidx[e] * WID3) + sub)
-                          : make_float4(0.f, 0.f, 0.f, 0.f);
-         }
-      };
-      float4 fc[4], fn[4];
-      uint32_t gc[4], gn[4];
-      fetch(0, fc, gc);
-      for (uint32_t q0 = 0; q0 < qn; q0 += 8) {
-         fetch(q0 + 8, fn, gn);
-#pragma unroll
-         for (int v = 0; v < 4; ++v) {
-            if (gc[v] == 0xffffffffu) continue;
-            // the row's sums of f, i f and i^2 f (i = 0..3 along x)
-            const double d0 = fc[v].x, d1 = fc[v].y, d2 = fc[v].z, d3 = fc[v].w;
-            const double s0 = (d0 + d1) + (d2 + d3);
-            if (!(gc[v] & ADJ_KEPT)) {
-               lsum += s0;
-               continue;
-            }
-            const double s1 = fma(3.0, d3, fma(2.0, d2, d1));
-            const double s2 = fma(9.0, d3, fma(4.0, d2, d1));
-            uint32_t bi, bj, bk;
-            block_xyz(mesh, gc[v] & ~ADJ_KEPT, bi, bj, bk);
-            const double x0 = (fr.vmin[0] + bi * fr.bs[0]) + ox;
-            const double uy = (fr.vmin[1] + bj * fr.bs[1]) + oy;
-            const double uz = (fr.vmin[2] + bk * fr.bs[2]) + oz;
-            const double ds1 = fr.dv[0] * s1;
-            const double sfx = fma(x0, s0, ds1);  // sum f x over the row
-            t[0] += s0;
-            t[1] += sfx;
-            t[2] = fma(s0, uy, t[2]);
-            t[3] = fma(s0, uz, t[3]);
-            // the same row relative to U
-            const double y0 = x0 - U0, vy = uy - U1, vz = uz - U2;
-            const double sfy = fma(y0, s0, ds1);
-            t[4] += fma(y0, fma(y0, s0, 2.0 * ds1), dv0s * s2);
-            const double s0y = s0 * vy;
-            t[5] = fma(s0y, vy, t[5]);
-            t[6] = fma(s0 * vz, vz, t[6]);
-            t[7] = fma(s0y, vz, t[7]);
-            t[8] = fma(sfy, vz, t[8]);
-            t[9] = fma(sfy, vy, t[9]);
-         }
-#pragma unroll
-         for (int v = 0; v < 4; ++v) {
-            fc[v] = fn[v];
-            gc[v] = gn[v];
-         }
-      }
-      __syncwarp();  // the queue is refilled
-   }
-   // CTA sums of the removed mass and of the moments (fixed order)
-#pragma unroll
-   for (int o = 16; o >= 1; o >>= 1) lsum += __shfl_xor_sync(FULL, lsum, o);
-   if (lane == 0) s_loss[warp] = lsum;
-   if (fuse) {
-#pragma unroll
-      for (int q = 0; q < 10; ++q) {
-         double v = t[q];
-#pragma unroll
-         for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
-         if (lane == 0) s_mom[warp][q] = v;
+         kept[s.off + b] = inH ? 1 : 0;
       }
    }
-   __syncthreads();
+   // the parts of the pass over the values; a cell without old blocks has none
+   const uint32_t parts = value_parts(s.count);
    if (threadIdx.x == 0) {
-      double tl = 0.0;
-      for (int w = 0; w < ADJ_THREADS / 32; ++w) tl += s_loss[w];
-      loss[cell] += dv3 * tl;
+      s_part = parts ? atomicAdd(&counters->n_items, parts) : 0u;
       out_slots[cell] = ok ? CellSlot{obase, total} : CellSlot{0u, 0u};
       if (s_flags) atomicOr(&status[cell], s_flags);
       if (!ok) atomicOr(&counters->overflow, 1u);
-      if (fuse) {
-         double S[10];
-         for (int q = 0; q < 10; ++q) {
-            double v = 0.0;
-            for (int w = 0; w < ADJ_THREADS / 32; ++w) v += s_mom[w][q];
-            S[q] = v;
-         }
-         moments_record<MOM_BOTH>(S, 0.0, 0.0, 0.0, U0, U1, U2, fr.dv[0], fr.dv[1], fr.dv[2], fr.mass, fr.charge,
-                                  mom_record + (size_t)cell * MOM_COUNT,
-                                  write_pivot ? pivot + (size_t)cell * MOM_COUNT : nullptr);
-      }
+   }
+   __syncthreads();
+   for (uint32_t p = threadIdx.x; p < parts; p += THREADS) items[s_part + p] = AdjustItem{cell, p};
+   if (parts == 0 && mom_record && threadIdx.x < MOM_COUNT) {
+      mom_record[(size_t)cell * MOM_COUNT + threadIdx.x] = 0.0;
+      if (write_pivot) pivot[(size_t)cell * MOM_COUNT + threadIdx.x] = 0.0;
    }
    __syncthreads();  // the next cell reuses the shared state
+   }
+}
+
+// The values.  A warp takes one part of a cell's old blocks at a time: the
+// removed blocks' values give the density loss, and with the moments wanted
+// (FUSE) the kept blocks' give the adjusted VDF's "_V" moments (MOM_BOTH: the
+// first sums about 0, the second about the pivot's bulk velocity U).  Half a
+// warp per block, one x-row of four cells per lane, eight blocks of the part's
+// staged list in flight.  The last part of a cell to finish adds the parts in
+// part order, so the result does not depend on which warp took which part.
+//
+// Bound by the FP64 and conversion pipes and the latency of a part's first
+// rows: 166 us for 1024 drifting cells (1.45 M blocks) in the first form, two
+// CTAs per SM with eight rows of a lane in flight.
+template <bool FUSE>
+__global__ void __launch_bounds__(ADJ_THREADS, ADJ_VALUE_CTAS) adjust_values_kernel(
+   const uint32_t* __restrict__ gids, const uint32_t* __restrict__ src_index, const CellSlot* __restrict__ slots,
+   const float* __restrict__ data, const uint8_t* __restrict__ kept, const AdjustItem* __restrict__ items,
+   const SweepCounters* __restrict__ counters, MeshDev mesh, double dv3, double* __restrict__ part_sums,
+   uint32_t* __restrict__ done, double* __restrict__ loss, double* __restrict__ mom_record,
+   double* pivot, int write_pivot, MomentFrame fr) {
+   constexpr int NS = FUSE ? 11 : 1;  // the loss and the ten moment sums
+   constexpr int WARPS = ADJ_THREADS / 32;
+   // a tile's data rows and its blocks' positions: x + (y << 8) + (z << 16)
+   // (| ADJ_KEPT)
+   __shared__ uint32_t s_idx[WARPS][ADJ_TILE], s_at[WARPS][ADJ_TILE];
+   __shared__ double s_sum[WARPS][NS][33];
+   __shared__ double s_corner[3][MAX_LEN];  // the blocks' lower corners along each axis
+   constexpr uint32_t FULL = 0xffffffffu;
+   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+   const uint32_t half = lane >> 4, sub = lane & 15;
+   if (FUSE) {
+      for (uint32_t i = threadIdx.x; i < MAX_LEN; i += ADJ_THREADS) {
+         s_corner[0][i] = fr.vmin[0] + i * fr.bs[0];
+         s_corner[1][i] = fr.vmin[1] + i * fr.bs[1];
+         s_corner[2][i] = fr.vmin[2] + i * fr.bs[2];
+      }
+      __syncthreads();
+   }
+   const double ox = 0.5 * fr.dv[0], oy = ((sub & 3) + 0.5) * fr.dv[1], oz = ((sub >> 2) + 0.5) * fr.dv[2];
+   const double dv0s = fr.dv[0] * fr.dv[0];
+   const uint32_t n_items = counters->n_items;
+   for (uint32_t it = warp * gridDim.x + blockIdx.x; it < n_items; it += WARPS * gridDim.x) {
+      const AdjustItem item = items[it];
+      const uint32_t cell = item.cell;
+      const CellSlot s = slots[cell];
+      const uint32_t parts = value_parts(s.count);
+      const uint32_t b0 = (uint32_t)(((uint64_t)s.count * item.part) / parts);
+      const uint32_t b1 = (uint32_t)(((uint64_t)s.count * (item.part + 1)) / parts);
+      double U0 = 0.0, U1 = 0.0, U2 = 0.0;
+      if (FUSE) {
+         const double* pv = pivot + (size_t)cell * MOM_COUNT;
+         U0 = pv[MOM_VX]; U1 = pv[MOM_VY]; U2 = pv[MOM_VZ];
+      }
+      double t[NS];
+#pragma unroll
+      for (int q = 0; q < NS; ++q) t[q] = 0.0;
+      for (uint32_t t0 = b0; t0 < b1; t0 += ADJ_TILE) {
+         // the tile's blocks that are read: the removed ones, and the kept
+         // ones where their moments are wanted
+         uint32_t n = 0;
+#pragma unroll
+         for (uint32_t q0 = 0; q0 < ADJ_TILE; q0 += 32) {
+            const uint32_t b = t0 + q0 + lane;
+            bool read = false;
+            uint32_t at = 0, idx = NO_BLOCK;
+            if (b < b1) {
+               const bool k = kept[s.off + b] != 0;
+               if (FUSE && k) {
+                  uint32_t x, y, z;
+                  block_xyz(mesh, gids[s.off + b], x, y, z);
+                  at = x | (y << 8) | (z << 16) | ADJ_KEPT;
+               }
+               idx = src_index ? src_index[s.off + b] : s.off + b;
+               read = idx != NO_BLOCK && (FUSE || !k);
+            }
+            const uint32_t bal = __ballot_sync(FULL, read);
+            if (read) {
+               const uint32_t q = n + __popc(bal & ((1u << lane) - 1u));
+               s_idx[warp][q] = idx;
+               s_at[warp][q] = at;
+            }
+            n += __popc(bal);
+         }
+         __syncwarp();
+         // half-warp h reads blocks h, h + 2, .. of every 2 ADJ_ROWS, the next
+         // ones on their way while these are summed
+         auto fetch = [&](uint32_t q0, float4* f) {
+#pragma unroll
+            for (int v = 0; v < ADJ_ROWS; ++v) {
+               const uint32_t e = q0 + half + 2 * v;
+               f[v] = make_float4(0.f, 0.f, 0.f, 0.f);
+               if (e < n) f[v] = __ldg(reinterpret_cast<const float4*>(data + (size_t)s_idx[warp][e] * WID3) + sub);
+            }
+         };
+         float4 fc[ADJ_ROWS], fn[ADJ_ROWS];
+         fetch(0, fc);
+         for (uint32_t q0 = 0; q0 < n; q0 += 2 * ADJ_ROWS) {
+            fetch(q0 + 2 * ADJ_ROWS, fn);
+#pragma unroll
+            for (int v = 0; v < ADJ_ROWS; ++v) {
+               const uint32_t e = q0 + half + 2 * v;
+               if (e >= n) continue;
+               const uint32_t at = s_at[warp][e];
+               // the row's sums of f, i f and i^2 f (i = 0..3 along x)
+               const double d0 = fc[v].x, d1 = fc[v].y, d2 = fc[v].z, d3 = fc[v].w;
+               const double s0 = (d0 + d1) + (d2 + d3);
+               if (!(at & ADJ_KEPT)) {
+                  t[0] += s0;
+                  continue;
+               }
+               if constexpr (FUSE) {
+                  const double s1 = fma(3.0, d3, fma(2.0, d2, d1));
+                  const double s2 = fma(9.0, d3, fma(4.0, d2, d1));
+                  const double x0 = s_corner[0][at & 0xffu] + ox;
+                  const double uy = s_corner[1][(at >> 8) & 0xffu] + oy;
+                  const double uz = s_corner[2][(at >> 16) & 0xffu] + oz;
+                  const double ds1 = fr.dv[0] * s1;
+                  const double sfx = fma(x0, s0, ds1);  // sum f x over the row
+                  t[1] += s0;
+                  t[2] += sfx;
+                  t[3] = fma(s0, uy, t[3]);
+                  t[4] = fma(s0, uz, t[4]);
+                  // the same row relative to U
+                  const double y0 = x0 - U0, vy = uy - U1, vz = uz - U2;
+                  const double sfy = fma(y0, s0, ds1);
+                  t[5] += fma(y0, sfy + ds1, dv0s * s2);
+                  const double s0y = s0 * vy;
+                  t[6] = fma(s0y, vy, t[6]);
+                  t[7] = fma(s0 * vz, vz, t[7]);
+                  t[8] = fma(s0y, vz, t[8]);
+                  t[9] = fma(sfy, vz, t[9]);
+                  t[10] = fma(sfy, vy, t[10]);
+               }
+            }
+#pragma unroll
+            for (int v = 0; v < ADJ_ROWS; ++v) fc[v] = fn[v];
+         }
+         __syncwarp();  // the tile is refilled
+      }
+      // the part's sums, the lanes added in order
+#pragma unroll
+      for (int q = 0; q < NS; ++q) s_sum[warp][q][lane] = t[q];
+      __syncwarp();
+      double* ps = part_sums + ((size_t)cell * MOM_PARTS_PER_CELL + item.part) * MOM_SUMS_PER_PART;
+      if (lane < NS) {
+         double v = 0.0;
+         for (int l = 0; l < 32; ++l) v += s_sum[warp][lane][l];
+         ps[lane] = v;
+      }
+      __syncwarp();
+      __threadfence();
+      uint32_t prev = 0;
+      if (lane == 0) prev = atomicAdd(&done[cell], 1u);
+      prev = __shfl_sync(FULL, prev, 0);
+      if (prev + 1 != parts) continue;
+      // the cell's last part: all parts in part order, compensated
+      __threadfence();
+      double S = 0.0;
+      if (lane < NS) {
+         double sum = 0.0, comp = 0.0;
+         const double* base = part_sums + (size_t)cell * MOM_PARTS_PER_CELL * MOM_SUMS_PER_PART + lane;
+         for (uint32_t p = 0; p < parts; ++p) {
+            const double y = __ldcg(base + (size_t)p * MOM_SUMS_PER_PART) - comp;
+            const double tt = sum + y;
+            comp = (tt - sum) - y;
+            sum = tt;
+         }
+         S = sum - comp;
+      }
+      if constexpr (FUSE) {
+         double Sv[10];
+#pragma unroll
+         for (int q = 0; q < 10; ++q) Sv[q] = __shfl_sync(FULL, S, q + 1);
+         if (lane == 0)
+            moments_record<MOM_BOTH>(Sv, 0.0, 0.0, 0.0, U0, U1, U2, fr.dv[0], fr.dv[1], fr.dv[2], fr.mass, fr.charge,
+                                     mom_record + (size_t)cell * MOM_COUNT,
+                                     write_pivot ? pivot + (size_t)cell * MOM_COUNT : nullptr);
+      }
+      if (lane == 0) {
+         loss[cell] += dv3 * S;
+         done[cell] = 0;  // ready for the next pass
+      }
    }
 }
 
@@ -636,39 +734,70 @@ size_t adjust_scratch_words(const MeshDev& mesh) { return (size_t)7 * mesh.len[1
 
 int adjust_blocks_per_sm() {
    int n = 0;
-   cudaFuncSetAttribute(adjust_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)adjust_smem_bytes());
-   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, adjust_kernel, ADJ_THREADS, adjust_smem_bytes());
+   cudaFuncSetAttribute(adjust_kernel<ADJ_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)adjust_smem_bytes());
+   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, adjust_kernel<ADJ_THREADS>, ADJ_THREADS, adjust_smem_bytes());
    return n > 0 ? n : 1;
 }
 
+// `kept`: a byte per row of the old list; `items`: at most one per ADJ_TILE
+// old blocks and one per cell.  The caller lends the sweeps' work arrays.
 cudaError_t launch_adjust(const uint32_t* gids, const uint32_t* src_index, const CellSlot* slots,
-                          const uint8_t* content, const float* data, const int32_t* neighbors, uint32_t* out_gids,
-                          uint32_t* out_src,
-                          CellSlot* out_slots, double* loss, uint32_t* status, SweepCounters* counters,
+                          uint8_t* content, bool content_valid, const float* data, const int32_t* neighbors,
+                          uint32_t* out_gids, uint32_t* out_src, CellSlot* out_slots, double* loss, uint32_t* status, SweepCounters* counters,
                           uint32_t out_capacity, const MeshDev& mesh, double min_value, int add_width, double dv3,
                           uint32_t n_cells, uint32_t* scratch, int grid, const uint32_t* order, MaskRec* masks,
-                          uint32_t* pool, uint32_t* pool_top, uint32_t pool_cap, double* mom_record,
+                          uint32_t* pool, uint32_t* pool_top, uint32_t pool_cap, uint8_t* kept, AdjustItem* items,
+                          double* part_sums, uint32_t* done, int value_grid, uint32_t few_cells, double* mom_record,
                           double* pivot, int write_pivot, const MomentFrame& frame, cudaStream_t stream) {
    if (n_cells == 0) return cudaSuccess;
    const size_t smem = adjust_smem_bytes();
-   cudaError_t e = cudaFuncSetAttribute(adjust_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+   const bool few = n_cells <= few_cells;
+   cudaError_t e = few ? cudaFuncSetAttribute(adjust_kernel<ADJ_FEW_THREADS>,
+                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+                       : cudaFuncSetAttribute(adjust_kernel<ADJ_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)smem);
    if (e != cudaSuccess) return e;
+   if (!content_valid) {
+      float threshold = (float)min_value;  // the smallest float >= min_value
+      if ((double)threshold < min_value) threshold = std::nextafterf(threshold, FLT_MAX);
+      const uint32_t spread = 8u * few_cells / n_cells;
+      content_flags_kernel<<<dim3(n_cells, spread > 1 ? (spread < 64 ? spread : 64) : 1), FLAG_THREADS, 0, stream>>>(
+         src_index, slots, data, threshold, content);
+   }
    const bool use_masks = neighbors && masks && pool && pool_top;
    if (use_masks) {
       e = cudaMemsetAsync(pool_top, 0, sizeof(uint32_t), stream);
       if (e != cudaSuccess) return e;
-      content_mask_kernel<<<n_cells, MASK_THREADS, 0, stream>>>(gids, src_index, slots, content, data, mesh,
-                                                                 min_value, masks, pool, pool_top, pool_cap);
+      content_mask_kernel<<<n_cells, MASK_THREADS, 0, stream>>>(gids, slots, content, mesh, masks, pool, pool_top,
+                                                                 pool_cap);
    }
-   // the counters' cell_next is zero here (the caller clears the sweep
-   // counters before every adjustment)
+   // the counters are zero here
    const uint32_t g = (uint32_t)grid < n_cells ? (uint32_t)grid : n_cells;
-   adjust_kernel<<<g, ADJ_THREADS, smem, stream>>>(gids, src_index, slots, content, data, neighbors, out_gids,
-                                                    out_src, out_slots, loss, status, counters, out_capacity, mesh,
-                                                    min_value, add_width, dv3, n_cells, ADJ_SMEM_ROWS, scratch,
-                                                    use_masks ? masks : nullptr, pool, order, mom_record, pivot,
-                                                    write_pivot, frame);
+#define VLGPU_ADJ(T)                                                                                               \
+   adjust_kernel<T><<<g, T, smem, stream>>>(gids, src_index, slots, content, neighbors, out_gids, out_src,        \
+                                            out_slots, status, counters, out_capacity, mesh, add_width,            \
+                                            n_cells, ADJ_SMEM_ROWS, scratch, use_masks ? masks : nullptr, pool,    \
+                                            order, kept, items, mom_record, pivot, write_pivot)
+   if (few) VLGPU_ADJ(ADJ_FEW_THREADS);
+   else VLGPU_ADJ(ADJ_THREADS);
+#undef VLGPU_ADJ
+   if ((e = cudaGetLastError()) != cudaSuccess) return e;
+   if (mom_record)
+      adjust_values_kernel<true><<<value_grid, ADJ_THREADS, 0, stream>>>(
+         gids, src_index, slots, data, kept, items, counters, mesh, dv3, part_sums, done, loss, mom_record, pivot,
+         write_pivot, frame);
+   else
+      adjust_values_kernel<false><<<value_grid, ADJ_THREADS, 0, stream>>>(
+         gids, src_index, slots, data, kept, items, counters, mesh, dv3, part_sums, done, loss, mom_record, pivot,
+         write_pivot, frame);
    return cudaGetLastError();
+}
+
+// CTAs per SM of the pass over the values.
+int adjust_values_blocks_per_sm() {
+   int n = 0;
+   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, adjust_values_kernel<true>, ADJ_THREADS, 0);
+   return n > 0 ? n : 1;
 }
 
 }  // namespace vlgpu

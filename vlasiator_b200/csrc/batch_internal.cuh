@@ -64,14 +64,15 @@ cudaError_t launch_geometry(const CellAccelInputs* in, const double* moments, do
                             const double vmin[3], const double dv[3], uint32_t map_order, float threshold,
                             cudaStream_t stream);
 cudaError_t launch_adjust(const uint32_t* gids, const uint32_t* src_index, const CellSlot* slots,
-                          const uint8_t* content, const float* data, const int32_t* neighbors, uint32_t* out_gids,
-                          uint32_t* out_src,
-                          CellSlot* out_slots, double* loss, uint32_t* status, SweepCounters* counters,
+                          uint8_t* content, bool content_valid, const float* data, const int32_t* neighbors,
+                          uint32_t* out_gids, uint32_t* out_src, CellSlot* out_slots, double* loss, uint32_t* status, SweepCounters* counters,
                           uint32_t out_capacity, const MeshDev& mesh, double min_value, int add_width, double dv3,
                           uint32_t n_cells, uint32_t* scratch, int grid, const uint32_t* order, MaskRec* masks,
-                          uint32_t* pool, uint32_t* pool_top, uint32_t pool_cap, double* mom_record,
+                          uint32_t* pool, uint32_t* pool_top, uint32_t pool_cap, uint8_t* kept, AdjustItem* items,
+                          double* part_sums, uint32_t* done, int value_grid, uint32_t few_cells, double* mom_record,
                           double* pivot, int write_pivot, const MomentFrame& frame, cudaStream_t stream);
 int adjust_blocks_per_sm();
+int adjust_values_blocks_per_sm();
 size_t adjust_scratch_words(const MeshDev& mesh);
 cudaError_t launch_max_dt(const uint32_t* gids, const CellSlot* slots, const CellAccelInputs* in, const MeshDev& mesh,
                           const double vmin[3], const double bs[3], const double dv[3], const double dx[3], double q,
@@ -198,6 +199,8 @@ struct vlgpu_batch {
    uint32_t* mask_top = nullptr;         // grid: words of the pool in use
    uint32_t mask_cap = 0;
    int adj_grid = 0;
+   AdjustItem* adj_items = nullptr;  // the parts of the adjustment's pass over the values
+   int adj_value_grid = 0;  // CTAs of the adjustment's pass over the values
    int col_wide_grid = 0;  // CTAs of the wide-plane columnize
    double* moments_r = nullptr;   // MOM_COUNT per cell: the moments after translation (the "_R" set)
    // pinned staging; each buffer's event marks when its last copy was read

@@ -49,6 +49,7 @@ void free_batch(vlgpu_batch* b) {
    cudaFree(b->neighbors);
    cudaFree(b->dt_buf);
    cudaFree(b->adj_scratch);
+   cudaFree(b->adj_items);
    cudaFree(b->wide_cells);
    cudaFree(b->halo_scratch);
    cudaFree(b->cell_order);
@@ -175,14 +176,17 @@ int adjust_device(vlgpu_batch* b, double* record, bool write_pivot) {
    }
    frame.mass = b->params.mass;
    frame.charge = b->params.charge;
-   VL_CHECK(launch_adjust(b->st_gids, b->st_src, b->st_slots, b->content_valid ? b->content : nullptr,
+   VL_CHECK(launch_adjust(b->st_gids, b->st_src, b->st_slots, b->content, b->content_valid,
                           b->data[b->cur], b->neighbors, b->adj_gids[a], b->adj_src[a], b->adj_slots[a], b->loss,
                           b->status,
                           b->counters, (uint32_t)b->capacity, b->mdev, b->params.min_value,
                           (int)b->params.add_width_v, dv3, b->n_cells, b->adj_scratch, b->adj_grid,
-                          b->cell_order, b->mask_recs, b->mask_pool, b->mask_top, b->mask_cap, record, b->pivot,
+                          b->cell_order, b->mask_recs, b->mask_pool, b->mask_top, b->mask_cap,
+                          reinterpret_cast<uint8_t*>(b->perm), b->adj_items,
+                          b->mom_parts, b->mom_done, b->adj_value_grid, (uint32_t)b->sm_count, record, b->pivot,
                           write_pivot ? 1 : 0, frame, b->stream));
-   b->launches += (b->neighbors && b->mask_recs) ? 2 : 1;  // content masks first on a grid
+   // content flags first unless a sweep left them, content masks on a grid
+   b->launches += 2 + (b->content_valid ? 0 : 1) + (b->neighbors && b->mask_recs ? 1 : 0);
    VL_CHECK(cudaMemcpyAsync(b->rows_used + 2 + a, &b->counters->dst_top, sizeof(uint32_t), cudaMemcpyDeviceToDevice,
                             b->stream));
    b->st_gids = b->adj_gids[a];
@@ -373,6 +377,7 @@ int vlgpu_batch_create(const vlgpu_mesh* mesh, const vlgpu_params* params, uint3
    b->cps_max[0] = remap_blocks_per_sm();
    b->cps_max[1] = moments_blocks_per_sm();
    b->cps_max[2] = adjust_blocks_per_sm();
+   b->adj_value_grid = b->sm_count * adjust_values_blocks_per_sm();
    b->col_wide_grid = b->sm_count * columnize_wide_blocks_per_sm(b->mdev);
    apply_launch(b);
    const uint64_t cap = block_capacity;
@@ -417,6 +422,9 @@ int vlgpu_batch_create(const vlgpu_mesh* mesh, const vlgpu_params* params, uint3
                                             (size_t)std::min<uint32_t>((uint32_t)b->adj_grid, n_cells))) !=
        cudaSuccess)
       return fail(e, "adjust scratch");
+   // a part per 128 old blocks and one per cell, at most
+   if ((e = cudaMalloc(&b->adj_items, sizeof(AdjustItem) * (cap / 128 + n_cells))) != cudaSuccess)
+      return fail(e, "adjust items");
    if ((e = cudaMalloc(&b->wide_cells, sizeof(uint32_t) * n_cells)) != cudaSuccess) return fail(e, "wide");
    if ((e = cudaMalloc(&b->cell_order, sizeof(uint32_t) * n_cells)) != cudaSuccess) return fail(e, "order");
    if ((e = cudaMallocHost(&b->h_order, sizeof(uint32_t) * n_cells)) != cudaSuccess) return fail(e, "order");

@@ -16,7 +16,7 @@ constexpr int MAX_PLANE = 96 * 96;  // transverse plane entries
 // The moments split a cell's blocks into at most this many parts, each
 // summed by one warp into MOM_SUMS_PER_PART doubles of a work array.
 constexpr int MOM_PARTS_PER_CELL = 64;
-constexpr int MOM_SUMS_PER_PART = 10;
+constexpr int MOM_SUMS_PER_PART = 11;  // the adjustment's parts add the removed mass
 
 // Per-cell state of one batch, indexed by cell.
 struct CellSlot {
@@ -133,6 +133,12 @@ struct SweepCounters {
    uint32_t overflow;
    uint32_t cell_next;  // warp-per-cell kernels (columnize, adjustment): next cell a warp takes
    uint32_t n_wide;     // cells those kernels left to their CTA-per-cell forms
+   uint32_t n_items;    // adjustment: parts of the pass over the values
+};
+
+// One part of the adjustment's pass over a cell's values.
+struct AdjustItem {
+   uint32_t cell, part;
 };
 
 // Running totals kept on the device across sweeps (never reset by a sweep).
