@@ -613,7 +613,8 @@ __global__ void __launch_bounds__(REMAP_THREADS, 3) remap_kernel(
    const ColumnSet* __restrict__ sets, SweepCounters* __restrict__ counters, const uint32_t* __restrict__ perm,
    const float* __restrict__ src_data, float* __restrict__ dst_data, uint32_t* __restrict__ dst_gids,
    const SweepCell* __restrict__ sweep_cells, uint32_t* __restrict__ status, MeshDev mesh, int wall_margin,
-   uint32_t set_capacity, uint8_t* __restrict__ content_out, double content_threshold) {
+   uint32_t set_capacity, uint8_t* __restrict__ content_out, double content_threshold, const HandOver after) {
+   hand_over(after, counters);
    __shared__ float ring_all[(REMAP_THREADS / 16) * RING_STRIDE];
    const int hw = threadIdx.x >> 4;
    const int lane = threadIdx.x & 15;
@@ -817,7 +818,8 @@ __global__ void __launch_bounds__(REMAP_THREADS, 3) remap_walk_kernel(
    const ColumnSet* __restrict__ sets, SweepCounters* __restrict__ counters, const uint32_t* __restrict__ perm,
    const float* __restrict__ src_data, float* __restrict__ dst_data, uint32_t* __restrict__ dst_gids,
    const SweepCell* __restrict__ sweep_cells, uint32_t* __restrict__ status, MeshDev mesh, int wall_margin,
-   uint32_t set_capacity, uint8_t* __restrict__ content_out, double content_threshold) {
+   uint32_t set_capacity, uint8_t* __restrict__ content_out, double content_threshold, const HandOver after) {
+   hand_over(after, counters);
    __shared__ __align__(16) float ring_all[REMAP_THREADS * WALK_LANE_STRIDE];
    const int hw = threadIdx.x >> 4;
    const int lane = threadIdx.x & 15;
@@ -1162,7 +1164,8 @@ __global__ void __launch_bounds__(PAIR_THREADS, PAIR_CTAS) remap_pair_kernel(
    const ColumnSet* __restrict__ sets, SweepCounters* __restrict__ counters, const uint32_t* __restrict__ perm,
    const float* __restrict__ src_data, float* __restrict__ dst_data, uint32_t* __restrict__ dst_gids,
    const SweepCell* __restrict__ sweep_cells, uint32_t* __restrict__ status, const PairMesh mesh,
-   uint32_t set_capacity, uint8_t* __restrict__ content_out) {
+   uint32_t set_capacity, uint8_t* __restrict__ content_out, const HandOver after) {
+   hand_over(after, counters);
    static_assert(RECON == RECON_PPM || RECON == RECON_PLM, "the quartic reconstruction runs in remap_walk_kernel");
    extern __shared__ __align__(16) unsigned char pair_ring[];
    constexpr unsigned FULL = 0xffffffffu;
@@ -1580,7 +1583,7 @@ cudaError_t launch_remap(int dim, const ColumnSet* sets, SweepCounters* counters
                          const float* src_data, float* dst_data, uint32_t* dst_gids, const SweepCell* sweep_cells,
                          uint32_t* status, const MeshDev& mesh, int wall_margin, uint32_t set_capacity,
                          uint8_t* content_out, double content_threshold, bool exact, int recon, int grid,
-                         cudaStream_t stream) {
+                         const HandOver& after, cudaStream_t stream) {
    PairMesh pm;
    for (int d = 0; d < 3; ++d) pm.len[d] = mesh.len[d];
    pm.wall_margin = wall_margin;
@@ -1592,18 +1595,18 @@ cudaError_t launch_remap(int dim, const ColumnSet* sets, SweepCounters* counters
 #define VLGPU_REMAP(D)                                                                                        \
    remap_kernel<D><<<grid, REMAP_THREADS, 0, stream>>>(sets, counters, perm, src_data, dst_data, dst_gids,          \
                                                        sweep_cells, status, mesh, wall_margin, set_capacity,        \
-                                                       content_out, content_threshold)
+                                                       content_out, content_threshold, after)
 #define VLGPU_WALK(D)                                                                                          \
    remap_walk_kernel<D><<<grid, REMAP_THREADS, 0, stream>>>(sets, counters, perm, src_data, dst_data, dst_gids, \
                                                                sweep_cells, status, mesh, wall_margin, set_capacity, \
-                                                               content_out, content_threshold)
+                                                               content_out, content_threshold, after)
 #define VLGPU_PAIR(D, R)                                                                                       \
    {                                                                                                           \
       const cudaError_t e = cudaFuncSetAttribute(remap_pair_kernel<D, R>,                                      \
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PAIR_SMEM); \
       if (e != cudaSuccess) return e;                                                                          \
       remap_pair_kernel<D, R><<<grid, PAIR_THREADS, PAIR_SMEM, stream>>>(                                      \
-         sets, counters, perm, src_data, dst_data, dst_gids, sweep_cells, status, pm, set_capacity, content_out); \
+         sets, counters, perm, src_data, dst_data, dst_gids, sweep_cells, status, pm, set_capacity, content_out, after); \
    }
 #define VLGPU_PAIR_DIMS(R)                 \
    if (dim == 0) VLGPU_PAIR(0, R)          \

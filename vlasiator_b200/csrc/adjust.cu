@@ -559,7 +559,8 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_VALUE_CTAS) adjust_values_ker
    const float* __restrict__ data, const uint8_t* __restrict__ kept, const AdjustItem* __restrict__ items,
    const SweepCounters* __restrict__ counters, MeshDev mesh, double dv3, double* __restrict__ part_sums,
    uint32_t* __restrict__ done, double* __restrict__ loss, double* __restrict__ mom_record,
-   double* pivot, int write_pivot, MomentFrame fr) {
+   double* pivot, int write_pivot, MomentFrame fr, const HandOver after) {
+   hand_over(after, counters);
    constexpr int NS = FUSE ? 11 : 1;  // the loss and the ten moment sums
    constexpr int WARPS = ADJ_THREADS / 32;
    // a tile's data rows and its blocks' positions: x + (y << 8) + (z << 16)
@@ -748,7 +749,8 @@ cudaError_t launch_adjust(const uint32_t* gids, const uint32_t* src_index, const
                           uint32_t n_cells, uint32_t* scratch, int grid, const uint32_t* order, MaskRec* masks,
                           uint32_t* pool, uint32_t* pool_top, uint32_t pool_cap, uint8_t* kept, AdjustItem* items,
                           double* part_sums, uint32_t* done, int value_grid, uint32_t few_cells, double* mom_record,
-                          double* pivot, int write_pivot, const MomentFrame& frame, cudaStream_t stream) {
+                          double* pivot, int write_pivot, const MomentFrame& frame, const HandOver& after,
+                          cudaStream_t stream) {
    if (n_cells == 0) return cudaSuccess;
    const size_t smem = adjust_smem_bytes();
    const bool few = n_cells <= few_cells;
@@ -785,11 +787,11 @@ cudaError_t launch_adjust(const uint32_t* gids, const uint32_t* src_index, const
    if (mom_record)
       adjust_values_kernel<true><<<value_grid, ADJ_THREADS, 0, stream>>>(
          gids, src_index, slots, data, kept, items, counters, mesh, dv3, part_sums, done, loss, mom_record, pivot,
-         write_pivot, frame);
+         write_pivot, frame, after);
    else
       adjust_values_kernel<false><<<value_grid, ADJ_THREADS, 0, stream>>>(
          gids, src_index, slots, data, kept, items, counters, mesh, dv3, part_sums, done, loss, mom_record, pivot,
-         write_pivot, frame);
+         write_pivot, frame, after);
    return cudaGetLastError();
 }
 

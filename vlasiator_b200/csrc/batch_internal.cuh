@@ -41,7 +41,7 @@ cudaError_t launch_remap(int dim, const ColumnSet* sets, SweepCounters* counters
                          const float* src_data, float* dst_data, uint32_t* dst_gids, const SweepCell* sweep_cells,
                          uint32_t* status, const MeshDev& mesh, int wall_margin, uint32_t set_capacity,
                          uint8_t* content_out, double content_threshold, bool exact, int recon, int grid,
-                         cudaStream_t stream);
+                         const HandOver& after, cudaStream_t stream);
 int remap_blocks_per_sm();
 struct CellAccelInputs {
    double B[3];
@@ -70,7 +70,8 @@ cudaError_t launch_adjust(const uint32_t* gids, const uint32_t* src_index, const
                           uint32_t n_cells, uint32_t* scratch, int grid, const uint32_t* order, MaskRec* masks,
                           uint32_t* pool, uint32_t* pool_top, uint32_t pool_cap, uint8_t* kept, AdjustItem* items,
                           double* part_sums, uint32_t* done, int value_grid, uint32_t few_cells, double* mom_record,
-                          double* pivot, int write_pivot, const MomentFrame& frame, cudaStream_t stream);
+                          double* pivot, int write_pivot, const MomentFrame& frame, const HandOver& after,
+                          cudaStream_t stream);
 int adjust_blocks_per_sm();
 int adjust_values_blocks_per_sm();
 size_t adjust_scratch_words(const MeshDev& mesh);
@@ -174,7 +175,10 @@ struct vlgpu_batch {
    double* isect12 = nullptr;  // 12 per cell
    double* loss = nullptr;     // RHOLOSSADJUST per cell
    uint32_t* status = nullptr;
+   // two blocks of counters, used in turn by the sweeps and adjustments: the
+   // next operation's (`turn`) is zero, the other is the last one's
    SweepCounters* counters = nullptr;
+   int turn = 0;
    BatchStats* stats = nullptr;
    // spatial grid (uniform, periodic, cells x fastest) and translation work arrays
    bool has_grid = false;
@@ -220,6 +224,7 @@ struct vlgpu_batch {
       const vlgpu::CellSlot* st_slots = nullptr;
       int cur = 0;
       int adj_next = 0;
+      int turn = 0;
       bool pivot_valid = false;      // at the start of the captured steps
       bool pivot_valid_end = false;  // after them
       unsigned long long launches = 0;

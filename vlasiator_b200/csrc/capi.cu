@@ -89,17 +89,19 @@ int sweep_device(vlgpu_batch* b, const SweepCell* sweep_cells, uint32_t dim, boo
    const uint32_t cap = (uint32_t)b->capacity;
    const int wm = (int)b->params.wall_margin;
    const double thr = b->params.min_value;
-   VL_CHECK(cudaMemsetAsync(b->counters, 0, sizeof(SweepCounters), b->stream));
+   SweepCounters* const counters = b->counters + b->turn;
+   b->turn ^= 1;
+   const HandOver after{b->rows_used + dst, b->counters + b->turn};
    if (!per_cell) {
       VL_CHECK(launch_columnize_batch((int)dim, b->st_gids, b->st_src, b->st_slots, b->slots[dst], b->perm, b->sets,
-                                      cap, cap, sweep_cells, b->status, b->counters, b->stats, b->mdev, wm,
+                                      cap, cap, sweep_cells, b->status, counters, b->stats, b->mdev, wm,
                                       b->n_cells, first_of_step ? 1 : 0, b->wide_cells, b->cell_order,
                                       b->col_wide_grid, (uint32_t)b->sm_count, b->stream));
       const bool prof = b->profiling && b->prof_used + 2 <= b->prof_events.size();
       if (prof) VL_CHECK(cudaEventRecord(b->prof_events[b->prof_used], b->stream));
-      VL_CHECK(launch_remap((int)dim, b->sets, b->counters, b->perm, b->data[src], b->data[dst], b->gids[dst],
+      VL_CHECK(launch_remap((int)dim, b->sets, counters, b->perm, b->data[src], b->data[dst], b->gids[dst],
                             sweep_cells, b->status, b->mdev, wm, cap, b->content, thr, b->exact, b->recon, b->remap_grid,
-                            b->stream));
+                            after, b->stream));
       if (prof) {
          VL_CHECK(cudaEventRecord(b->prof_events[b->prof_used + 1], b->stream));
          b->prof_used += 2;
@@ -110,19 +112,17 @@ int sweep_device(vlgpu_batch* b, const SweepCell* sweep_cells, uint32_t dim, boo
       // one columnize + remap launch pair per cell; set and output counters
       // keep running so the cells land in disjoint ranges
       for (uint32_t c = 0; c < b->n_cells; ++c) {
-         VL_CHECK(launch_rebase_work(b->counters, b->stream));
+         VL_CHECK(launch_rebase_work(counters, b->stream));
          VL_CHECK(launch_columnize((int)dim, b->st_gids, b->st_src, b->st_slots, b->slots[dst], b->perm, b->sets,
-                                   cap, cap, sweep_cells, b->status, b->counters, b->stats, b->mdev, wm, c, c + 1,
+                                   cap, cap, sweep_cells, b->status, counters, b->stats, b->mdev, wm, c, c + 1,
                                    first_of_step ? 1 : 0, b->stream));
-         VL_CHECK(launch_remap((int)dim, b->sets, b->counters, b->perm, b->data[src], b->data[dst], b->gids[dst],
+         VL_CHECK(launch_remap((int)dim, b->sets, counters, b->perm, b->data[src], b->data[dst], b->gids[dst],
                                sweep_cells, b->status, b->mdev, wm, cap, b->content, thr, b->exact, b->recon, b->sm_count,
-                               b->stream));
+                               after, b->stream));
          b->launches += 3;
          b->remap_launches += 1;
       }
    }
-   VL_CHECK(cudaMemcpyAsync(b->rows_used + dst, &b->counters->dst_top, sizeof(uint32_t), cudaMemcpyDeviceToDevice,
-                            b->stream));
    set_direct_state(b, dst);
    b->content_valid = true;
    return VLGPU_OK;
@@ -166,7 +166,9 @@ int moments_both_device(vlgpu_batch* b, double* record) {
 int adjust_device(vlgpu_batch* b, double* record, bool write_pivot) {
    const int a = b->adj_next;
    b->adj_next = 1 - a;
-   VL_CHECK(cudaMemsetAsync(b->counters, 0, sizeof(SweepCounters), b->stream));
+   SweepCounters* const counters = b->counters + b->turn;
+   b->turn ^= 1;
+   const HandOver after{b->rows_used + 2 + a, b->counters + b->turn};
    const double dv3 = b->dv_d[0] * b->dv_d[1] * b->dv_d[2];
    MomentFrame frame{};
    for (int d = 0; d < 3; ++d) {
@@ -179,16 +181,14 @@ int adjust_device(vlgpu_batch* b, double* record, bool write_pivot) {
    VL_CHECK(launch_adjust(b->st_gids, b->st_src, b->st_slots, b->content, b->content_valid,
                           b->data[b->cur], b->neighbors, b->adj_gids[a], b->adj_src[a], b->adj_slots[a], b->loss,
                           b->status,
-                          b->counters, (uint32_t)b->capacity, b->mdev, b->params.min_value,
+                          counters, (uint32_t)b->capacity, b->mdev, b->params.min_value,
                           (int)b->params.add_width_v, dv3, b->n_cells, b->adj_scratch, b->adj_grid,
                           b->cell_order, b->mask_recs, b->mask_pool, b->mask_top, b->mask_cap,
                           reinterpret_cast<uint8_t*>(b->perm), b->adj_items,
                           b->mom_parts, b->mom_done, b->adj_value_grid, (uint32_t)b->sm_count, record, b->pivot,
-                          write_pivot ? 1 : 0, frame, b->stream));
+                          write_pivot ? 1 : 0, frame, after, b->stream));
    // content flags first unless a sweep left them, content masks on a grid
    b->launches += 2 + (b->content_valid ? 0 : 1) + (b->neighbors && b->mask_recs ? 1 : 0);
-   VL_CHECK(cudaMemcpyAsync(b->rows_used + 2 + a, &b->counters->dst_top, sizeof(uint32_t), cudaMemcpyDeviceToDevice,
-                            b->stream));
    b->st_gids = b->adj_gids[a];
    b->st_src = b->adj_src[a];
    b->st_slots = b->adj_slots[a];
@@ -413,9 +413,9 @@ int vlgpu_batch_create(const vlgpu_mesh* mesh, const vlgpu_params* params, uint3
    if ((e = cudaMemset(b->loss, 0, sizeof(double) * n_cells)) != cudaSuccess) return fail(e, "loss");
    if ((e = cudaMalloc(&b->status, sizeof(uint32_t) * n_cells)) != cudaSuccess) return fail(e, "status");
    if ((e = cudaMemset(b->status, 0, sizeof(uint32_t) * n_cells)) != cudaSuccess) return fail(e, "status");
-   if ((e = cudaMalloc(&b->counters, sizeof(SweepCounters))) != cudaSuccess) return fail(e, "counters");
+   if ((e = cudaMalloc(&b->counters, 2 * sizeof(SweepCounters))) != cudaSuccess) return fail(e, "counters");
    // no sweep has run: vlgpu_batch_sync reads the overflow flag from here
-   if ((e = cudaMemset(b->counters, 0, sizeof(SweepCounters))) != cudaSuccess) return fail(e, "counters");
+   if ((e = cudaMemset(b->counters, 0, 2 * sizeof(SweepCounters))) != cudaSuccess) return fail(e, "counters");
    if ((e = cudaMalloc(&b->stats, sizeof(BatchStats))) != cudaSuccess) return fail(e, "stats");
    if ((e = cudaMalloc(&b->rows_used, sizeof(uint32_t) * 4)) != cudaSuccess) return fail(e, "rows");
    if ((e = cudaMalloc(&b->adj_scratch, sizeof(uint32_t) * adjust_scratch_words(b->mdev) *
@@ -981,8 +981,8 @@ int vlgpu_batch_capture(vlgpu_batch* b, int slot, int kind, uint32_t n_steps, co
       VL_CHECK(cudaGraphExecDestroy(g.exec));
       g.exec = nullptr;
    }
-   const vlgpu_batch::GraphSlot start{nullptr,      b->st_gids,     b->st_src, b->st_slots, b->cur,
-                                      b->adj_next,  b->pivot_valid, false,     0,           0};
+   const vlgpu_batch::GraphSlot start{nullptr,     b->st_gids, b->st_src,      b->st_slots, b->cur,
+                                      b->adj_next, b->turn,    b->pivot_valid, false,       0, 0};
    const bool content_valid = b->content_valid;
    const unsigned long long l0 = b->launches, r0 = b->remap_launches;
    VL_CHECK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeRelaxed));
@@ -993,12 +993,14 @@ int vlgpu_batch_capture(vlgpu_batch* b, int slot, int kind, uint32_t n_steps, co
    const cudaError_t ec = cudaStreamEndCapture(b->stream, &graph);
    // nothing ran: the host's view of the buffers is the one before the capture
    const bool same_buffers = b->st_gids == start.st_gids && b->st_src == start.st_src &&
-                             b->st_slots == start.st_slots && b->cur == start.cur && b->adj_next == start.adj_next;
+                             b->st_slots == start.st_slots && b->cur == start.cur && b->adj_next == start.adj_next &&
+                             b->turn == start.turn;
    b->st_gids = start.st_gids;
    b->st_src = start.st_src;
    b->st_slots = start.st_slots;
    b->cur = start.cur;
    b->adj_next = start.adj_next;
+   b->turn = start.turn;
    b->content_valid = content_valid;
    const bool pivot_end = b->pivot_valid;
    b->pivot_valid = start.pivot_valid;
@@ -1033,6 +1035,10 @@ int vlgpu_batch_replay(vlgpu_batch* b, int slot) {
        b->adj_next != g.adj_next || (g.pivot_valid && !b->pivot_valid))
       return VLGPU_EINVAL;  // the batch is not in the state the graph was captured in
    VL_CHECK(cudaSetDevice(b->device));
+   if (b->turn != g.turn) {  // the captured steps start with the other block of counters
+      VL_CHECK(cudaMemsetAsync(b->counters + g.turn, 0, sizeof(SweepCounters), b->stream));
+      b->turn = g.turn;
+   }
    VL_CHECK(cudaGraphLaunch(g.exec, b->stream));
    b->launches += g.launches;
    b->remap_launches += g.remap_launches;
@@ -1059,7 +1065,7 @@ int vlgpu_batch_sync(vlgpu_batch* b) {
    VL_CHECK(cudaSetDevice(b->device));
    VL_CHECK(cudaStreamSynchronize(b->stream));
    SweepCounters c{};
-   VL_CHECK(cudaMemcpy(&c, b->counters, sizeof(c), cudaMemcpyDeviceToHost));
+   VL_CHECK(cudaMemcpy(&c, b->counters + (b->turn ^ 1), sizeof(c), cudaMemcpyDeviceToHost));
    if (c.overflow) return VLGPU_ENOMEM;
    if (b->tcounters) {
       TransCounters t{};

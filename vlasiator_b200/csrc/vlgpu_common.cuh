@@ -136,6 +136,19 @@ struct SweepCounters {
    uint32_t n_items;    // adjustment: parts of the pass over the values
 };
 
+// What the last kernel of a sweep or an adjustment leaves for the operations
+// after it: the rows it used, and the other block of counters zeroed for the
+// next operation (a batch uses two in turn).  Null: not wanted.
+struct HandOver {
+   uint32_t* rows_out;
+   SweepCounters* next;
+};
+__device__ __forceinline__ void hand_over(const HandOver& h, const SweepCounters* counters) {
+   if (blockIdx.x != 0 || threadIdx.x != 0) return;
+   if (h.rows_out) *h.rows_out = counters->dst_top;
+   if (h.next) *h.next = SweepCounters{};
+}
+
 // One part of the adjustment's pass over a cell's values.
 struct AdjustItem {
    uint32_t cell, part;
