@@ -453,8 +453,9 @@ __global__ void __launch_bounds__(THREADS) columnize_kernel(
    uint32_t set_capacity, uint32_t dst_capacity,
    const SweepCell* __restrict__ sweep_cells, uint32_t* __restrict__ status, SweepCounters* __restrict__ counters,
    BatchStats* __restrict__ stats, MeshDev mesh, int wall_margin, uint32_t cell_begin, uint32_t cell_end,
-   int first_of_step, const uint32_t* __restrict__ order, uint32_t plane_cap, uint32_t* __restrict__ wide_cells) {
-   if (cell_begin + blockIdx.x >= cell_end) return;
+   int first_of_step, const uint32_t* __restrict__ order, uint32_t plane_cap, uint32_t* __restrict__ wide_cells,
+   const uint32_t* __restrict__ stop) {
+   if (cell_begin + blockIdx.x >= cell_end || (stop && *stop)) return;
    const uint32_t cell = order ? order[blockIdx.x] : cell_begin + blockIdx.x;
    columnize_cell<DIM>(cell, gids, src_index, src_slots, dst_slots, perm, sets, set_capacity, dst_capacity,
                        sweep_cells, status, counters, stats, mesh, wall_margin, first_of_step, plane_cap,
@@ -1504,7 +1505,7 @@ cudaError_t launch_columnize(int dim, const uint32_t* gids, const uint32_t* src_
                              uint32_t* perm, ColumnSet* sets, uint32_t set_capacity, uint32_t dst_capacity,
                              const SweepCell* sweep_cells, uint32_t* status, SweepCounters* counters,
                              BatchStats* stats, const MeshDev& mesh, int wall_margin, uint32_t cell_begin,
-                             uint32_t cell_end, int first_of_step, cudaStream_t stream) {
+                             uint32_t cell_end, int first_of_step, const uint32_t* stop, cudaStream_t stream) {
    uint32_t li, lj;
    plane_lengths(mesh.len, dim, li, lj);
    const size_t smem = columnize_smem_bytes(li * lj);
@@ -1517,7 +1518,7 @@ cudaError_t launch_columnize(int dim, const uint32_t* gids, const uint32_t* src_
    if (e != cudaSuccess) return e;                                                                              \
    columnize_kernel<D, COL_FEW_THREADS><<<n, COL_FEW_THREADS, smem, stream>>>(                                  \
       gids, src_index, src_slots, dst_slots, perm, sets, set_capacity, dst_capacity, sweep_cells, status, counters, \
-      stats, mesh, wall_margin, cell_begin, cell_end, first_of_step, nullptr, 0xffffffffu, nullptr);
+      stats, mesh, wall_margin, cell_begin, cell_end, first_of_step, nullptr, 0xffffffffu, nullptr, stop);
    if (dim == 0) { VLGPU_COL(0) } else if (dim == 1) { VLGPU_COL(1) } else { VLGPU_COL(2) }
 #undef VLGPU_COL
    return cudaGetLastError();
@@ -1540,7 +1541,7 @@ cudaError_t launch_columnize_batch(int dim, const uint32_t* gids, const uint32_t
    if (n_cells <= few_cells)
       return launch_columnize(dim, gids, src_index, src_slots, dst_slots, perm, sets, set_capacity, dst_capacity,
                               sweep_cells, status, counters, stats, mesh, wall_margin, 0, n_cells, first_of_step,
-                              stream);
+                              nullptr, stream);
    const uint32_t cap = li * lj < COL_CAP_PLANE ? li * lj : COL_CAP_PLANE;
    const size_t smem_cap = columnize_smem_bytes(cap);
    const size_t smem = columnize_smem_bytes(li * lj);
@@ -1554,7 +1555,7 @@ cudaError_t launch_columnize_batch(int dim, const uint32_t* gids, const uint32_t
    if (e != cudaSuccess) return e;                                                                               \
    columnize_kernel<D, COL_THREADS><<<n_cells, COL_THREADS, smem_cap, stream>>>(                                              \
       gids, src_index, src_slots, dst_slots, perm, sets, set_capacity, dst_capacity, sweep_cells, status, counters, \
-      stats, mesh, wall_margin, 0, n_cells, first_of_step, order, cap, wide_cells);                              \
+      stats, mesh, wall_margin, 0, n_cells, first_of_step, order, cap, wide_cells, nullptr);                              \
    columnize_wide_kernel<D><<<g2, COL_FEW_THREADS, smem, stream>>>(gids, src_index, src_slots, dst_slots, perm, sets, \
                                                                set_capacity, dst_capacity, sweep_cells, status,   \
                                                                counters, stats, mesh, wall_margin, first_of_step, \

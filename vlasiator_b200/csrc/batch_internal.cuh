@@ -29,7 +29,8 @@ cudaError_t launch_columnize(int dim, const uint32_t* gids, const uint32_t* src_
                              CellSlot* dst_slots, uint32_t* perm, ColumnSet* sets, uint32_t set_capacity,
                              uint32_t dst_capacity, const SweepCell* sweep_cells, uint32_t* status,
                              SweepCounters* counters, BatchStats* stats, const MeshDev& mesh, int wall_margin,
-                             uint32_t cell_begin, uint32_t cell_end, int first_of_step, cudaStream_t stream);
+                             uint32_t cell_begin, uint32_t cell_end, int first_of_step, const uint32_t* stop,
+                             cudaStream_t stream);
 cudaError_t launch_columnize_batch(int dim, const uint32_t* gids, const uint32_t* src_index,
                                    const CellSlot* src_slots, CellSlot* dst_slots, uint32_t* perm, ColumnSet* sets,
                                    uint32_t set_capacity, uint32_t dst_capacity, const SweepCell* sweep_cells,

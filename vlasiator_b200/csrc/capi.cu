@@ -115,7 +115,7 @@ int sweep_device(vlgpu_batch* b, const SweepCell* sweep_cells, uint32_t dim, boo
          VL_CHECK(launch_rebase_work(counters, b->stream));
          VL_CHECK(launch_columnize((int)dim, b->st_gids, b->st_src, b->st_slots, b->slots[dst], b->perm, b->sets,
                                    cap, cap, sweep_cells, b->status, counters, b->stats, b->mdev, wm, c, c + 1,
-                                   first_of_step ? 1 : 0, b->stream));
+                                   first_of_step ? 1 : 0, nullptr, b->stream));
          VL_CHECK(launch_remap((int)dim, b->sets, counters, b->perm, b->data[src], b->data[dst], b->gids[dst],
                                sweep_cells, b->status, b->mdev, wm, cap, b->content, thr, b->exact, b->recon, b->sm_count,
                                after, b->stream));

@@ -25,7 +25,8 @@ cudaError_t launch_columnize(int dim, const uint32_t* gids, const uint32_t* src_
                              CellSlot* dst_slots, uint32_t* perm, ColumnSet* sets, uint32_t set_capacity,
                              uint32_t dst_capacity, const SweepCell* sweep_cells, uint32_t* status,
                              SweepCounters* counters, BatchStats* stats, const MeshDev& mesh, int wall_margin,
-                             uint32_t cell_begin, uint32_t cell_end, int first_of_step, cudaStream_t stream);
+                             uint32_t cell_begin, uint32_t cell_end, int first_of_step, const uint32_t* stop,
+                             cudaStream_t stream);
 cudaError_t launch_remap(int dim, const ColumnSet* sets, SweepCounters* counters, const uint32_t* perm,
                          const float* src_data, float* dst_data, uint32_t* dst_gids, const SweepCell* sweep_cells,
                          uint32_t* status, const MeshDev& mesh, int wall_margin, uint32_t set_capacity,
@@ -39,18 +40,23 @@ constexpr uint32_t NA_MAX_BLOCKS = VLGPU_NOALLOC_MAX_BLOCKS;
 constexpr uint32_t NA_MAX_CELLS = VLGPU_NOALLOC_MAX_CELLS;
 constexpr int NA_MAX_DEVICES = 64;
 
-// Layout of the scratch array.  Everything up to `zeroed_end` is cleared at
-// the start of every call; the rest is fully written before it is read.
-struct NoallocLayout {
+// What a call reads back, and the part of it that is cleared first.  The
+// per-cell arrays follow one another for the call's own number of cells, so
+// that they travel in one copy.
+struct NoallocHeader {
    SweepCounters counters;
    uint32_t bad_gid;
    uint32_t pad0[3];
    BatchStats stats;
-   uint32_t status[NA_MAX_CELLS];
-   unsigned char zeroed_end[16];
-   CellSlot src_slots[NA_MAX_CELLS];
-   CellSlot dst_slots[NA_MAX_CELLS];
-   SweepCell sweep[NA_MAX_CELLS];
+};
+
+// Layout of the scratch array: results (header, then per cell the output slot
+// and the status) and inputs (per cell the sweep parameters, then the slots);
+// the rest is fully written before it is read.
+struct NoallocLayout {
+   NoallocHeader header;
+   unsigned char results[NA_MAX_CELLS * (sizeof(CellSlot) + sizeof(uint32_t))];
+   alignas(16) unsigned char inputs[NA_MAX_CELLS * (sizeof(SweepCell) + sizeof(CellSlot))];
    uint32_t perm[NA_MAX_BLOCKS];
    ColumnSet sets[NA_MAX_BLOCKS];   // a column set holds at least one source block
    uint8_t content[NA_MAX_BLOCKS];  // written by the remap for every output block
@@ -160,25 +166,26 @@ extern "C" int vlgpu_map_1d_noalloc(const vlgpu_mesh* mesh, const vlgpu_params* 
    cudaStream_t s = static_cast<cudaStream_t>(stream);
 
    // device views of the scratch
-   SweepCounters* d_counters = reinterpret_cast<SweepCounters*>(base + offsetof(NoallocLayout, counters));
-   uint32_t* d_bad = reinterpret_cast<uint32_t*>(base + offsetof(NoallocLayout, bad_gid));
-   BatchStats* d_stats = reinterpret_cast<BatchStats*>(base + offsetof(NoallocLayout, stats));
-   uint32_t* d_status = reinterpret_cast<uint32_t*>(base + offsetof(NoallocLayout, status));
-   CellSlot* d_src_slots = reinterpret_cast<CellSlot*>(base + offsetof(NoallocLayout, src_slots));
-   CellSlot* d_dst_slots = reinterpret_cast<CellSlot*>(base + offsetof(NoallocLayout, dst_slots));
-   SweepCell* d_sweep = reinterpret_cast<SweepCell*>(base + offsetof(NoallocLayout, sweep));
+   NoallocHeader* d_header = reinterpret_cast<NoallocHeader*>(base);
+   SweepCounters* d_counters = &d_header->counters;
+   uint32_t* d_bad = &d_header->bad_gid;
+   BatchStats* d_stats = &d_header->stats;
+   CellSlot* d_dst_slots = reinterpret_cast<CellSlot*>(base + offsetof(NoallocLayout, results));
+   uint32_t* d_status = reinterpret_cast<uint32_t*>(d_dst_slots + n_cells);
+   SweepCell* d_sweep = reinterpret_cast<SweepCell*>(base + offsetof(NoallocLayout, inputs));
+   CellSlot* d_src_slots = reinterpret_cast<CellSlot*>(d_sweep + n_cells);
    uint32_t* d_perm = reinterpret_cast<uint32_t*>(base + offsetof(NoallocLayout, perm));
    ColumnSet* d_sets = reinterpret_cast<ColumnSet*>(base + offsetof(NoallocLayout, sets));
    uint8_t* d_content = reinterpret_cast<uint8_t*>(base + offsetof(NoallocLayout, content));
 
    // host staging on the stack (no heap use either)
-   SweepCell h_sweep[NA_MAX_CELLS];
-   CellSlot h_slots[NA_MAX_CELLS];
-   uint32_t h_status[NA_MAX_CELLS];
+   alignas(16) unsigned char h_inputs[sizeof(NoallocLayout::inputs)];
+   alignas(16) unsigned char h_results[sizeof(NoallocHeader) + sizeof(NoallocLayout::results)];
+   SweepCell* h_sweep = reinterpret_cast<SweepCell*>(h_inputs);
+   CellSlot* h_src_slots = reinterpret_cast<CellSlot*>(h_sweep + n_cells);
    for (uint32_t c = 0; c < n_cells; ++c) {
       h_sweep[c] = make_sweep_cell(intersections + 4 * (size_t)c, dimension, params->min_value);
-      h_slots[c].off = (uint32_t)offsets[c];
-      h_slots[c].count = (uint32_t)(offsets[c + 1] - offsets[c]);
+      h_src_slots[c] = CellSlot{(uint32_t)offsets[c], (uint32_t)(offsets[c + 1] - offsets[c])};
    }
    MeshDev mdev{};
    for (int d = 0; d < 3; ++d) {
@@ -190,43 +197,45 @@ extern "C" int vlgpu_map_1d_noalloc(const vlgpu_mesh* mesh, const vlgpu_params* 
    set_block_reciprocals(mdev);
 
    // the previous call's counters, flags and statuses must not leak into this one
-   NA_CHECK(cudaMemsetAsync(base, 0, offsetof(NoallocLayout, zeroed_end), s));
-   NA_CHECK(cudaMemcpyAsync(d_sweep, h_sweep, sizeof(SweepCell) * n_cells, cudaMemcpyHostToDevice, s));
-   NA_CHECK(cudaMemcpyAsync(d_src_slots, h_slots, sizeof(CellSlot) * n_cells, cudaMemcpyHostToDevice, s));
+   const size_t results_bytes = sizeof(NoallocHeader) + n_cells * (sizeof(CellSlot) + sizeof(uint32_t));
+   NA_CHECK(cudaMemsetAsync(base, 0, results_bytes, s));
+   NA_CHECK(cudaMemcpyAsync(d_sweep, h_inputs, n_cells * (sizeof(SweepCell) + sizeof(CellSlot)), cudaMemcpyHostToDevice,
+                            s));
+   const uint32_t max_gid = mesh->len[0] * mesh->len[1] * mesh->len[2];
    if (end > begin) {
-      uint32_t h_bad = 0;
-      const uint32_t max_gid = mesh->len[0] * mesh->len[1] * mesh->len[2];
+      // a bad block ID stops the sweep's first kernel, which then leaves no
+      // sets for the second: the host learns of it with the results, without
+      // a wait of its own
       const uint64_t n = end - begin;
       const unsigned grid = (unsigned)((n + 255) / 256 < 1024 ? (n + 255) / 256 : 1024);
       check_gids_kernel<<<grid, 256, 0, s>>>(gids_in, begin, end, max_gid, d_bad);
       NA_CHECK(cudaGetLastError());
-      NA_CHECK(cudaMemcpyAsync(&h_bad, d_bad, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-      NA_CHECK(cudaStreamSynchronize(s));
-      if (h_bad) {
-         std::fprintf(stderr, "vlgpu_map_1d_noalloc: a block ID lies outside the %u-block mesh\n", max_gid);
-         return VLGPU_EINVAL;
-      }
    }
 
    const uint32_t dst_cap = (uint32_t)(out_capacity < NA_MAX_BLOCKS ? out_capacity : NA_MAX_BLOCKS);
    const int wm = (int)params->wall_margin;
    NA_CHECK(launch_columnize((int)dimension, gids_in, nullptr, d_src_slots, d_dst_slots, d_perm, d_sets,
                              NA_MAX_BLOCKS, dst_cap, d_sweep, d_status, d_counters, d_stats, mdev, wm, 0, n_cells, 0,
-                             s));
+                             d_bad, s));
    NA_CHECK(launch_remap((int)dimension, d_sets, d_counters, d_perm, data_in, data_out, gids_out, d_sweep, d_status,
-                         mdev, wm, NA_MAX_BLOCKS, d_content, params->min_value, false, 2, remap_grid, HandOver{nullptr, nullptr}, s));
+                         mdev, wm, NA_MAX_BLOCKS, d_content, params->min_value, false, 2, remap_grid,
+                         HandOver{nullptr, nullptr}, s));
 
-   SweepCounters h_counters{};
-   NA_CHECK(cudaMemcpyAsync(h_slots, d_dst_slots, sizeof(CellSlot) * n_cells, cudaMemcpyDeviceToHost, s));
-   NA_CHECK(cudaMemcpyAsync(h_status, d_status, sizeof(uint32_t) * n_cells, cudaMemcpyDeviceToHost, s));
-   NA_CHECK(cudaMemcpyAsync(&h_counters, d_counters, sizeof(SweepCounters), cudaMemcpyDeviceToHost, s));
+   NA_CHECK(cudaMemcpyAsync(h_results, base, results_bytes, cudaMemcpyDeviceToHost, s));
    NA_CHECK(cudaStreamSynchronize(s));
+   const NoallocHeader& h_header = *reinterpret_cast<const NoallocHeader*>(h_results);
+   const CellSlot* h_slots = reinterpret_cast<const CellSlot*>(h_results + sizeof(NoallocHeader));
+   const uint32_t* h_status = reinterpret_cast<const uint32_t*>(h_slots + n_cells);
+   if (h_header.bad_gid) {
+      std::fprintf(stderr, "vlgpu_map_1d_noalloc: a block ID lies outside the %u-block mesh\n", max_gid);
+      return VLGPU_EINVAL;
+   }
    for (uint32_t c = 0; c < n_cells; ++c) {
       cell_off[c] = h_slots[c].off;
       cell_count[c] = h_slots[c].count;
       if (status) status[c] = h_status[c];
    }
-   if (h_counters.overflow) {
+   if (h_header.counters.overflow) {
       std::fprintf(stderr, "vlgpu_map_1d_noalloc: the output needs more than %u blocks (out_capacity %llu, limit %u)\n",
                    dst_cap, (unsigned long long)out_capacity, NA_MAX_BLOCKS);
       return VLGPU_ENOMEM;
