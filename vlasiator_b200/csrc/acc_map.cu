@@ -216,6 +216,7 @@ __device__ __forceinline__ void columnize_cell(
    __shared__ uint32_t warp_sums[32];
    __shared__ uint32_t s_bbox[4];
    __shared__ uint32_t s_set_base, s_dst_base, s_nsets, s_ntgt, s_flags;
+   __shared__ uint32_t s_bin[MAX_LEN + 1];  // sets by length, longest first: count, then first record
 
    const CellSlot src = src_slots[cell];
    const SweepCell P = sweep_cells[cell];
@@ -273,8 +274,10 @@ __device__ __forceinline__ void columnize_cell(
    uint32_t* mask = smem;                   // 3 * plane
    uint32_t* prefix = smem + 3 * plane;     // plane
    uint16_t* set_t = (uint16_t*)(prefix + plane);  // plane (set index -> t)
-   uint32_t* tcount = prefix + plane + (plane + 1) / 2;  // plane
+   uint16_t* rank = (uint16_t*)(prefix + plane + (plane + 1) / 2);  // plane (set index -> record)
+   uint32_t* tcount = prefix + plane + 2 * ((plane + 1) / 2);       // plane
    for (uint32_t q = threadIdx.x; q < 3 * plane; q += blockDim.x) mask[q] = 0;
+   for (uint32_t q = threadIdx.x; q <= MAX_LEN; q += blockDim.x) s_bin[q] = 0;
    __syncthreads();
    // pass 2: occupancy masks along the sweep dimension; where the list runs
    // along the sweep (the x sweep of a list in ID order) the lanes that set
@@ -331,13 +334,43 @@ __device__ __forceinline__ void columnize_cell(
       const uint32_t n = __popc(mask[3 * t]) + __popc(mask[3 * t + 1]) + __popc(mask[3 * t + 2]);
       prefix[t] = blk_base;
       blk_base += n;
-      if (n > 0) set_t[set_base++] = (uint16_t)t;
+      if (n > 0) {
+         set_t[set_base++] = (uint16_t)t;
+         atomicAdd(&s_bin[MAX_LEN - n], 1u);
+      }
    }
    if (threadIdx.x == 0) {
       const uint32_t base = atomicAdd(&counters->n_sets, tot_sets);
       s_set_base = base;
       s_nsets = tot_sets;
       if (base + tot_sets > set_capacity) s_flags |= VLGPU_CELL_NOMEM;
+   }
+   __syncthreads();
+   // the records go by length, so that the sets a warp of the remap walks in
+   // step are equally long (28 -> 30.5 of 32 lanes busy, 10% fewer instructions; six
+   // steps of 4096 cells 31.5 -> 29.3 ms); the output keeps the sets' order
+   if (warp == 0) {
+      constexpr int PER = (MAX_LEN + 1 + 31) / 32;
+      uint32_t n[PER], sum = 0;
+#pragma unroll
+      for (int q = 0; q < PER; ++q) {
+         const int k = (int)lane * PER + q;
+         n[q] = (k <= MAX_LEN) ? s_bin[k] : 0u;
+         sum += n[q];
+      }
+      uint32_t x = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+         const uint32_t y = __shfl_up_sync(FULL, x, o);
+         if ((int)lane >= o) x += y;
+      }
+      x -= sum;
+#pragma unroll
+      for (int q = 0; q < PER; ++q) {
+         const int k = (int)lane * PER + q;
+         if (k <= MAX_LEN) s_bin[k] = x;
+         x += n[q];
+      }
    }
    __syncthreads();
    const bool sets_ok = !(s_flags & VLGPU_CELL_NOMEM);
@@ -378,7 +411,9 @@ __device__ __forceinline__ void columnize_cell(
          cs.dst_pos = 0;
          cs.src_mask[0] = m[0]; cs.src_mask[1] = m[1]; cs.src_mask[2] = m[2];
          cs.tgt_mask[0] = tm[0]; cs.tgt_mask[1] = tm[1]; cs.tgt_mask[2] = tm[2];
-         sets[s_set_base + s] = cs;
+         const uint32_t r = atomicAdd(&s_bin[MAX_LEN - (__popc(m[0]) + __popc(m[1]) + __popc(m[2]))], 1u);
+         rank[s] = (uint16_t)r;
+         sets[s_set_base + r] = cs;
       }
    }
    if (wall) atomicOr(&s_flags, VLGPU_CELL_WALL);
@@ -401,7 +436,7 @@ __device__ __forceinline__ void columnize_cell(
    const bool ok = !(s_flags & VLGPU_CELL_NOMEM);
    if (ok) {
       for (uint32_t s = q0; s < q1; ++s) {
-         sets[s_set_base + s].dst_pos = s_dst_base + tbase;
+         sets[s_set_base + rank[s]].dst_pos = s_dst_base + tbase;
          tbase += tcount[s];
       }
       // source permutation in (set, k) order
@@ -483,7 +518,7 @@ __global__ void __launch_bounds__(COL_FEW_THREADS) columnize_wide_kernel(
 
 // Dynamic shared memory of columnize for a full transverse plane.
 size_t columnize_smem_bytes(uint32_t plane) {
-   return sizeof(uint32_t) * (3 * plane + plane + (plane + 1) / 2 + plane) + 16;
+   return sizeof(uint32_t) * (3 * plane + plane + 2 * ((plane + 1) / 2) + plane) + 16;
 }
 
 // ---------------------------------------------------------------------------
@@ -1078,27 +1113,27 @@ constexpr uint32_t PAIR_SLOT_MASK = (RING_CELLS - 1) * PAIR_SLOT_BYTES;
 constexpr int PAIR_CTAS = 3;  // per SM: 72 to 80 registers, 192 KB of rings
 constexpr size_t PAIR_SMEM = (size_t)RING_CELLS * PAIR_SLOT_BYTES;
 
+// The block that stands for one without data.
+__device__ __align__(16) const float zero_block[WID3] = {};
+
 // The lane's two columns of the block at `row`: cells g = 0..3 along the
-// sweep, .x and .y the two columns (zeros for a block without data).
+// sweep, .x and .y the two columns.  data and zeros point at the lane's first
+// cell; a block without data reads the block of zeros (one select of the
+// address instead of eight moves and four predicated loads).
 template <int DIM>
-__device__ __forceinline__ void load_pair(const float* __restrict__ lane_data, uint32_t row, float2 v[4]) {
-   const float* __restrict__ blk = lane_data + (size_t)row * WID3;
+__device__ __forceinline__ void load_pair(const float* __restrict__ data, const float* __restrict__ zeros, uint32_t row,
+                                          float2 v[4]) {
+   const float* __restrict__ blk = (row == NO_BLOCK) ? zeros : data + (size_t)row * WID3;
    if (DIM == 0) {
-      float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a;
-      if (row != NO_BLOCK) {
-         a = __ldg(reinterpret_cast<const float4*>(blk));
-         b = __ldg(reinterpret_cast<const float4*>(blk) + 1);
-      }
+      const float4 a = __ldg(reinterpret_cast<const float4*>(blk));
+      const float4 b = __ldg(reinterpret_cast<const float4*>(blk) + 1);
       v[0] = make_float2(a.x, b.x);
       v[1] = make_float2(a.y, b.y);
       v[2] = make_float2(a.z, b.z);
       v[3] = make_float2(a.w, b.w);
    } else {
 #pragma unroll
-      for (int g = 0; g < 4; ++g) {
-         v[g] = make_float2(0.0f, 0.0f);
-         if (row != NO_BLOCK) v[g] = __ldg(reinterpret_cast<const float2*>(blk + g * (DIM == 1 ? WID : WID2)));
-      }
+      for (int g = 0; g < 4; ++g) v[g] = __ldg(reinterpret_cast<const float2*>(blk + g * (DIM == 1 ? WID : WID2)));
    }
 }
 
@@ -1124,7 +1159,7 @@ __device__ __forceinline__ void pass_through_pair(const ColumnSet& cs, const uin
    uint32_t r = 0;
    for (int k = mask_next_set(cs.src_mask, 0); k < 96; k = mask_next_set(cs.src_mask, k + 1), ++r) {
       float2 v[4];
-      load_pair<DIM>(src_data + off, perm[cs.src_pos + r], v);
+      load_pair<DIM>(src_data + off, zero_block + off, perm[cs.src_pos + r], v);
       const uint32_t o = cs.dst_pos + r;
       store_pair<DIM>(dst_data + (size_t)o * WID3 + off, v);
       bool c = false;
@@ -1411,14 +1446,14 @@ __global__ void __launch_bounds__(PAIR_THREADS, PAIR_CTAS) remap_pair_kernel(
       float2 w[4], n[4];  // the values of block `it` and of the one after it
       {
          const uint32_t r0 = n_src > 0 ? __ldg(perm + pos) : NO_BLOCK;
-         load_pair<DIM>(src_data + off, r0, w);
+         load_pair<DIM>(src_data + off, zero_block + off, r0, w);
       }
       uint32_t row = n_src > 1 ? __ldg(perm + pos + 1) : NO_BLOCK;  // data row of block it + 1
       if (n_src > 0) start(w);
       // (one pass at least: a set without source blocks writes its targets)
       for (int it = 0; it == 0 || it < iters; ++it) {
          const bool active = it < n_src, last = left == 1;
-         load_pair<DIM>(src_data + off, row, n);
+         load_pair<DIM>(src_data + off, zero_block + off, row, n);
          row = (it + 2 < n_src) ? __ldg(perm + pos + it + 2) : NO_BLOCK;
          if (active) {
             // zero padding above the column
