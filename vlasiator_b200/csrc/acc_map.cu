@@ -165,6 +165,7 @@ __device__ __forceinline__ void set_corners(const SweepCell& P, uint32_t si, uin
 constexpr int COL_THREADS = 256;
 constexpr int COL_FEW_THREADS = 1024;
 constexpr int COL_UNROLL = 4;  // list entries a thread has in flight
+constexpr uint32_t NO_BLOCK = 0xffffffffu;  // a list entry without data: all zero
 
 // Swapped indices of a block ID, by the mesh's reciprocals.
 template <int DIM>
@@ -210,8 +211,8 @@ __device__ __forceinline__ void columnize_cell(
    const CellSlot* __restrict__ src_slots, CellSlot* __restrict__ dst_slots, uint32_t* __restrict__ perm,
    ColumnSet* __restrict__ sets, uint32_t set_capacity, uint32_t dst_capacity,
    const SweepCell* __restrict__ sweep_cells, uint32_t* __restrict__ status, SweepCounters* __restrict__ counters,
-   BatchStats* __restrict__ stats, const MeshDev& mesh, int wall_margin, int first_of_step, uint32_t plane_cap,
-   uint32_t* __restrict__ wide_cells) {
+   BatchStats* __restrict__ stats, const MeshDev& mesh, int wall_margin, int first_of_step, uint32_t zero_row,
+   uint32_t plane_cap, uint32_t* __restrict__ wide_cells) {
    extern __shared__ uint32_t smem[];
    __shared__ uint32_t warp_sums[32];
    __shared__ uint32_t s_bbox[4];
@@ -447,6 +448,7 @@ __device__ __forceinline__ void columnize_cell(
             const uint32_t b = e + blockDim.x * u, at = src.off + (b < src.count ? b : e);
             g[u] = gids[at];
             row[u] = src_index ? src_index[at] : at;
+            row[u] = (row[u] == NO_BLOCK) ? zero_row : row[u];
          }
 #pragma unroll
          for (int u = 0; u < COL_UNROLL; ++u) {
@@ -488,12 +490,12 @@ __global__ void __launch_bounds__(THREADS) columnize_kernel(
    uint32_t set_capacity, uint32_t dst_capacity,
    const SweepCell* __restrict__ sweep_cells, uint32_t* __restrict__ status, SweepCounters* __restrict__ counters,
    BatchStats* __restrict__ stats, MeshDev mesh, int wall_margin, uint32_t cell_begin, uint32_t cell_end,
-   int first_of_step, const uint32_t* __restrict__ order, uint32_t plane_cap, uint32_t* __restrict__ wide_cells,
-   const uint32_t* __restrict__ stop) {
+   int first_of_step, uint32_t zero_row, const uint32_t* __restrict__ order, uint32_t plane_cap,
+   uint32_t* __restrict__ wide_cells, const uint32_t* __restrict__ stop) {
    if (cell_begin + blockIdx.x >= cell_end || (stop && *stop)) return;
    const uint32_t cell = order ? order[blockIdx.x] : cell_begin + blockIdx.x;
    columnize_cell<DIM>(cell, gids, src_index, src_slots, dst_slots, perm, sets, set_capacity, dst_capacity,
-                       sweep_cells, status, counters, stats, mesh, wall_margin, first_of_step, plane_cap,
+                       sweep_cells, status, counters, stats, mesh, wall_margin, first_of_step, zero_row, plane_cap,
                        wide_cells);
 }
 
@@ -505,13 +507,13 @@ __global__ void __launch_bounds__(COL_FEW_THREADS) columnize_wide_kernel(
    CellSlot* __restrict__ dst_slots, uint32_t* __restrict__ perm, ColumnSet* __restrict__ sets,
    uint32_t set_capacity, uint32_t dst_capacity,
    const SweepCell* __restrict__ sweep_cells, uint32_t* __restrict__ status, SweepCounters* __restrict__ counters,
-   BatchStats* __restrict__ stats, MeshDev mesh, int wall_margin, int first_of_step,
+   BatchStats* __restrict__ stats, MeshDev mesh, int wall_margin, int first_of_step, uint32_t zero_row,
    const uint32_t* __restrict__ wide_cells) {
    const uint32_t n = counters->n_wide;
    for (uint32_t it = blockIdx.x; it < n; it += gridDim.x) {
       columnize_cell<DIM>(wide_cells[it], gids, src_index, src_slots, dst_slots, perm, sets, set_capacity,
                           dst_capacity, sweep_cells, status, counters, stats, mesh, wall_margin, first_of_step,
-                          0xffffffffu, nullptr);
+                          zero_row, 0xffffffffu, nullptr);
       __syncthreads();  // the next cell reuses the shared state
    }
 }
@@ -564,16 +566,11 @@ struct SetClaims {
    }
 };
 
-constexpr uint32_t NO_BLOCK = 0xffffffffu;  // a block that exists with all-zero data
 
 __device__ __forceinline__ int clampi(int x, int lo, int hi) { return x < lo ? lo : (x > hi ? hi : x); }
 
 template <int DIM>
 __device__ __forceinline__ void load_lane(const float* __restrict__ data, uint32_t idx, int i, int j, float v[4]) {
-   if (idx == NO_BLOCK) {
-      v[0] = v[1] = v[2] = v[3] = 0.0f;
-      return;
-   }
    const float* __restrict__ blk = data + (size_t)idx * WID3;
    if (DIM == 0) {
       const float4 q = __ldg(reinterpret_cast<const float4*>(blk + cell_offset<0>(i, j, 0)));
@@ -1113,17 +1110,11 @@ constexpr uint32_t PAIR_SLOT_MASK = (RING_CELLS - 1) * PAIR_SLOT_BYTES;
 constexpr int PAIR_CTAS = 3;  // per SM: 72 to 80 registers, 192 KB of rings
 constexpr size_t PAIR_SMEM = (size_t)RING_CELLS * PAIR_SLOT_BYTES;
 
-// The block that stands for one without data.
-__device__ __align__(16) const float zero_block[WID3] = {};
-
-// The lane's two columns of the block at `row`: cells g = 0..3 along the
-// sweep, .x and .y the two columns.  data and zeros point at the lane's first
-// cell; a block without data reads the block of zeros (one select of the
-// address instead of eight moves and four predicated loads).
+// The lane's two columns of the block at `row` (data: the lane's first cell of
+// row 0): cells g = 0..3 along the sweep, .x and .y the two columns.
 template <int DIM>
-__device__ __forceinline__ void load_pair(const float* __restrict__ data, const float* __restrict__ zeros, uint32_t row,
-                                          float2 v[4]) {
-   const float* __restrict__ blk = (row == NO_BLOCK) ? zeros : data + (size_t)row * WID3;
+__device__ __forceinline__ void load_pair(const float* __restrict__ data, uint32_t row, float2 v[4]) {
+   const float* __restrict__ blk = data + (size_t)row * WID3;
    if (DIM == 0) {
       const float4 a = __ldg(reinterpret_cast<const float4*>(blk));
       const float4 b = __ldg(reinterpret_cast<const float4*>(blk) + 1);
@@ -1159,7 +1150,7 @@ __device__ __forceinline__ void pass_through_pair(const ColumnSet& cs, const uin
    uint32_t r = 0;
    for (int k = mask_next_set(cs.src_mask, 0); k < 96; k = mask_next_set(cs.src_mask, k + 1), ++r) {
       float2 v[4];
-      load_pair<DIM>(src_data + off, zero_block + off, perm[cs.src_pos + r], v);
+      load_pair<DIM>(src_data + off, perm[cs.src_pos + r], v);
       const uint32_t o = cs.dst_pos + r;
       store_pair<DIM>(dst_data + (size_t)o * WID3 + off, v);
       bool c = false;
@@ -1443,18 +1434,17 @@ __global__ void __launch_bounds__(PAIR_THREADS, PAIR_CTAS) remap_pair_kernel(
          v_l = fa(v_l, mesh.dv);
       };
 
-      float2 w[4], n[4];  // the values of block `it` and of the one after it
-      {
-         const uint32_t r0 = n_src > 0 ? __ldg(perm + pos) : NO_BLOCK;
-         load_pair<DIM>(src_data + off, zero_block + off, r0, w);
-      }
-      uint32_t row = n_src > 1 ? __ldg(perm + pos + 1) : NO_BLOCK;  // data row of block it + 1
+      // the values of block `it` and of the one after it
+      float2 w[4] = {zero2, zero2, zero2, zero2}, n[4] = {zero2, zero2, zero2, zero2};
+      uint32_t row = 0;  // data row of block it + 1
+      if (n_src > 0) load_pair<DIM>(src_data + off, __ldg(perm + pos), w);
+      if (n_src > 1) row = __ldg(perm + pos + 1);
       if (n_src > 0) start(w);
       // (one pass at least: a set without source blocks writes its targets)
       for (int it = 0; it == 0 || it < iters; ++it) {
          const bool active = it < n_src, last = left == 1;
-         load_pair<DIM>(src_data + off, zero_block + off, row, n);
-         row = (it + 2 < n_src) ? __ldg(perm + pos + it + 2) : NO_BLOCK;
+         if (it + 1 < n_src) load_pair<DIM>(src_data + off, row, n);
+         if (it + 2 < n_src) row = __ldg(perm + pos + it + 2);
          if (active) {
             // zero padding above the column
             const float2 n0 = last ? zero2 : n[0], n1 = last ? zero2 : n[1];
@@ -1540,7 +1530,8 @@ cudaError_t launch_columnize(int dim, const uint32_t* gids, const uint32_t* src_
                              uint32_t* perm, ColumnSet* sets, uint32_t set_capacity, uint32_t dst_capacity,
                              const SweepCell* sweep_cells, uint32_t* status, SweepCounters* counters,
                              BatchStats* stats, const MeshDev& mesh, int wall_margin, uint32_t cell_begin,
-                             uint32_t cell_end, int first_of_step, const uint32_t* stop, cudaStream_t stream) {
+                             uint32_t cell_end, int first_of_step, uint32_t zero_row, const uint32_t* stop,
+                             cudaStream_t stream) {
    uint32_t li, lj;
    plane_lengths(mesh.len, dim, li, lj);
    const size_t smem = columnize_smem_bytes(li * lj);
@@ -1553,7 +1544,7 @@ cudaError_t launch_columnize(int dim, const uint32_t* gids, const uint32_t* src_
    if (e != cudaSuccess) return e;                                                                              \
    columnize_kernel<D, COL_FEW_THREADS><<<n, COL_FEW_THREADS, smem, stream>>>(                                  \
       gids, src_index, src_slots, dst_slots, perm, sets, set_capacity, dst_capacity, sweep_cells, status, counters, \
-      stats, mesh, wall_margin, cell_begin, cell_end, first_of_step, nullptr, 0xffffffffu, nullptr, stop);
+      stats, mesh, wall_margin, cell_begin, cell_end, first_of_step, zero_row, nullptr, 0xffffffffu, nullptr, stop);
    if (dim == 0) { VLGPU_COL(0) } else if (dim == 1) { VLGPU_COL(1) } else { VLGPU_COL(2) }
 #undef VLGPU_COL
    return cudaGetLastError();
@@ -1568,15 +1559,16 @@ cudaError_t launch_columnize_batch(int dim, const uint32_t* gids, const uint32_t
                                    const CellSlot* src_slots, CellSlot* dst_slots, uint32_t* perm, ColumnSet* sets,
                                    uint32_t set_capacity, uint32_t dst_capacity, const SweepCell* sweep_cells,
                                    uint32_t* status, SweepCounters* counters, BatchStats* stats, const MeshDev& mesh,
-                                   int wall_margin, uint32_t n_cells, int first_of_step, uint32_t* wide_cells,
-                                   const uint32_t* order, int wide_grid, uint32_t few_cells, cudaStream_t stream) {
+                                   int wall_margin, uint32_t n_cells, int first_of_step, uint32_t zero_row,
+                                   uint32_t* wide_cells, const uint32_t* order, int wide_grid, uint32_t few_cells,
+                                   cudaStream_t stream) {
    if (n_cells == 0) return cudaSuccess;
    uint32_t li, lj;
    plane_lengths(mesh.len, dim, li, lj);
    if (n_cells <= few_cells)
       return launch_columnize(dim, gids, src_index, src_slots, dst_slots, perm, sets, set_capacity, dst_capacity,
                               sweep_cells, status, counters, stats, mesh, wall_margin, 0, n_cells, first_of_step,
-                              nullptr, stream);
+                              zero_row, nullptr, stream);
    const uint32_t cap = li * lj < COL_CAP_PLANE ? li * lj : COL_CAP_PLANE;
    const size_t smem_cap = columnize_smem_bytes(cap);
    const size_t smem = columnize_smem_bytes(li * lj);
@@ -1590,11 +1582,11 @@ cudaError_t launch_columnize_batch(int dim, const uint32_t* gids, const uint32_t
    if (e != cudaSuccess) return e;                                                                               \
    columnize_kernel<D, COL_THREADS><<<n_cells, COL_THREADS, smem_cap, stream>>>(                                              \
       gids, src_index, src_slots, dst_slots, perm, sets, set_capacity, dst_capacity, sweep_cells, status, counters, \
-      stats, mesh, wall_margin, 0, n_cells, first_of_step, order, cap, wide_cells, nullptr);                              \
+      stats, mesh, wall_margin, 0, n_cells, first_of_step, zero_row, order, cap, wide_cells, nullptr);                              \
    columnize_wide_kernel<D><<<g2, COL_FEW_THREADS, smem, stream>>>(gids, src_index, src_slots, dst_slots, perm, sets, \
                                                                set_capacity, dst_capacity, sweep_cells, status,   \
                                                                counters, stats, mesh, wall_margin, first_of_step, \
-                                                               wide_cells);
+                                                               zero_row, wide_cells);
    if (dim == 0) { VLGPU_COLB(0) } else if (dim == 1) { VLGPU_COLB(1) } else { VLGPU_COLB(2) }
 #undef VLGPU_COLB
    return cudaGetLastError();

@@ -29,14 +29,15 @@ cudaError_t launch_columnize(int dim, const uint32_t* gids, const uint32_t* src_
                              CellSlot* dst_slots, uint32_t* perm, ColumnSet* sets, uint32_t set_capacity,
                              uint32_t dst_capacity, const SweepCell* sweep_cells, uint32_t* status,
                              SweepCounters* counters, BatchStats* stats, const MeshDev& mesh, int wall_margin,
-                             uint32_t cell_begin, uint32_t cell_end, int first_of_step, const uint32_t* stop,
+                             uint32_t cell_begin, uint32_t cell_end, int first_of_step, uint32_t zero_row, const uint32_t* stop,
                              cudaStream_t stream);
 cudaError_t launch_columnize_batch(int dim, const uint32_t* gids, const uint32_t* src_index,
                                    const CellSlot* src_slots, CellSlot* dst_slots, uint32_t* perm, ColumnSet* sets,
                                    uint32_t set_capacity, uint32_t dst_capacity, const SweepCell* sweep_cells,
                                    uint32_t* status, SweepCounters* counters, BatchStats* stats, const MeshDev& mesh,
-                                   int wall_margin, uint32_t n_cells, int first_of_step, uint32_t* wide_cells,
-                                   const uint32_t* order, int wide_grid, uint32_t few_cells, cudaStream_t stream);
+                                   int wall_margin, uint32_t n_cells, int first_of_step, uint32_t zero_row,
+                                   uint32_t* wide_cells, const uint32_t* order, int wide_grid, uint32_t few_cells,
+                                   cudaStream_t stream);
 int columnize_wide_blocks_per_sm(const MeshDev& mesh);
 cudaError_t launch_remap(int dim, const ColumnSet* sets, SweepCounters* counters, const uint32_t* perm,
                          const float* src_data, float* dst_data, uint32_t* dst_gids, const SweepCell* sweep_cells,
@@ -106,8 +107,8 @@ struct TransCounters {
 constexpr uint32_t TR_MAX_N = 128;
 cudaError_t launch_pencil_union(const uint32_t* gids, const CellSlot* slots, int dim, uint32_t nx, uint32_t ny,
                                 uint32_t nz, const MeshDev& mesh, uint32_t* item_gid, uint32_t* item_pencil,
-                                uint32_t* rows, uint32_t* srcs, const uint32_t* src_index, uint32_t item_cap,
-                                uint64_t row_cap, TransCounters* tc, uint32_t* status, cudaStream_t stream);
+                                uint32_t* rows, uint32_t* srcs, const uint32_t* src_index, uint32_t zero_row,
+                                uint32_t item_cap, uint64_t row_cap, TransCounters* tc, uint32_t* status, cudaStream_t stream);
 cudaError_t launch_trans_remap(int dim, uint32_t N, const uint32_t* item_gid, const uint32_t* item_pencil,
                                const uint32_t* rows, const uint32_t* srcs, TransCounters* tc, uint32_t item_cap,
                                uint64_t row_cap, const uint32_t* src_index, const float* src, float* dst,
@@ -142,7 +143,7 @@ struct vlgpu_batch {
    double vmin_d[3], bs_d[3], dv_d[3];
    // data pools and the lists written by sweeps into them
    uint32_t* gids[2] = {nullptr, nullptr};
-   float* data[2] = {nullptr, nullptr};
+   float* data[2] = {nullptr, nullptr};  // capacity rows and one of zeros, which stands for blocks without data
    CellSlot* slots[2] = {nullptr, nullptr};
    uint8_t* content = nullptr;  // content flag per output row of the last sweep
    // lists written by block adjustment (two, used alternately)

@@ -95,7 +95,7 @@ int sweep_device(vlgpu_batch* b, const SweepCell* sweep_cells, uint32_t dim, boo
    if (!per_cell) {
       VL_CHECK(launch_columnize_batch((int)dim, b->st_gids, b->st_src, b->st_slots, b->slots[dst], b->perm, b->sets,
                                       cap, cap, sweep_cells, b->status, counters, b->stats, b->mdev, wm,
-                                      b->n_cells, first_of_step ? 1 : 0, b->wide_cells, b->cell_order,
+                                      b->n_cells, first_of_step ? 1 : 0, cap, b->wide_cells, b->cell_order,
                                       b->col_wide_grid, (uint32_t)b->sm_count, b->stream));
       const bool prof = b->profiling && b->prof_used + 2 <= b->prof_events.size();
       if (prof) VL_CHECK(cudaEventRecord(b->prof_events[b->prof_used], b->stream));
@@ -115,7 +115,7 @@ int sweep_device(vlgpu_batch* b, const SweepCell* sweep_cells, uint32_t dim, boo
          VL_CHECK(launch_rebase_work(counters, b->stream));
          VL_CHECK(launch_columnize((int)dim, b->st_gids, b->st_src, b->st_slots, b->slots[dst], b->perm, b->sets,
                                    cap, cap, sweep_cells, b->status, counters, b->stats, b->mdev, wm, c, c + 1,
-                                   first_of_step ? 1 : 0, nullptr, b->stream));
+                                   first_of_step ? 1 : 0, cap, nullptr, b->stream));
          VL_CHECK(launch_remap((int)dim, b->sets, counters, b->perm, b->data[src], b->data[dst], b->gids[dst],
                                sweep_cells, b->status, b->mdev, wm, cap, b->content, thr, b->exact, b->recon, b->sm_count,
                                after, b->stream));
@@ -272,7 +272,7 @@ int translate_device(vlgpu_batch* b, uint32_t dim, double dt) {
    VL_CHECK(cudaMemsetAsync(b->tcounters, 0, sizeof(TransCounters), b->stream));
    VL_CHECK(launch_pencil_union(b->st_gids, b->st_slots, (int)dim, b->grid_dims[0], b->grid_dims[1],
                                 b->grid_dims[2], b->mdev, b->item_gid, b->item_pencil, b->trans_rows,
-                                b->trans_src, b->st_src, (uint32_t)b->capacity, b->row_cap, b->tcounters, b->status,
+                                b->trans_src, b->st_src, (uint32_t)b->capacity, (uint32_t)b->capacity, b->row_cap, b->tcounters, b->status,
                                 b->stream));
    int per_sm = trans_blocks_per_sm(N, b->exact);
    if (b->cps[3] > 0 && (int)b->cps[3] < per_sm) per_sm = (int)b->cps[3];
@@ -383,7 +383,8 @@ int vlgpu_batch_create(const vlgpu_mesh* mesh, const vlgpu_params* params, uint3
    const uint64_t cap = block_capacity;
    for (int p = 0; p < 2; ++p) {
       if ((e = cudaMalloc(&b->gids[p], sizeof(uint32_t) * cap)) != cudaSuccess) return fail(e, "gids");
-      if ((e = cudaMalloc(&b->data[p], sizeof(float) * WID3 * cap)) != cudaSuccess) return fail(e, "data");
+      if ((e = cudaMalloc(&b->data[p], sizeof(float) * WID3 * (cap + 1))) != cudaSuccess) return fail(e, "data");
+      if ((e = cudaMemset(b->data[p] + WID3 * cap, 0, sizeof(float) * WID3)) != cudaSuccess) return fail(e, "data");
       if ((e = cudaMalloc(&b->slots[p], sizeof(CellSlot) * n_cells)) != cudaSuccess) return fail(e, "slots");
       if ((e = cudaMemset(b->slots[p], 0, sizeof(CellSlot) * n_cells)) != cudaSuccess) return fail(e, "slots");
       if ((e = cudaMalloc(&b->adj_gids[p], sizeof(uint32_t) * cap)) != cudaSuccess) return fail(e, "adj");

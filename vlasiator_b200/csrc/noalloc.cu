@@ -25,7 +25,7 @@ cudaError_t launch_columnize(int dim, const uint32_t* gids, const uint32_t* src_
                              CellSlot* dst_slots, uint32_t* perm, ColumnSet* sets, uint32_t set_capacity,
                              uint32_t dst_capacity, const SweepCell* sweep_cells, uint32_t* status,
                              SweepCounters* counters, BatchStats* stats, const MeshDev& mesh, int wall_margin,
-                             uint32_t cell_begin, uint32_t cell_end, int first_of_step, const uint32_t* stop,
+                             uint32_t cell_begin, uint32_t cell_end, int first_of_step, uint32_t zero_row, const uint32_t* stop,
                              cudaStream_t stream);
 cudaError_t launch_remap(int dim, const ColumnSet* sets, SweepCounters* counters, const uint32_t* perm,
                          const float* src_data, float* dst_data, uint32_t* dst_gids, const SweepCell* sweep_cells,
@@ -216,7 +216,7 @@ extern "C" int vlgpu_map_1d_noalloc(const vlgpu_mesh* mesh, const vlgpu_params* 
    const int wm = (int)params->wall_margin;
    NA_CHECK(launch_columnize((int)dimension, gids_in, nullptr, d_src_slots, d_dst_slots, d_perm, d_sets,
                              NA_MAX_BLOCKS, dst_cap, d_sweep, d_status, d_counters, d_stats, mdev, wm, 0, n_cells, 0,
-                             d_bad, s));
+                             0, d_bad, s));
    NA_CHECK(launch_remap((int)dimension, d_sets, d_counters, d_perm, data_in, data_out, gids_out, d_sweep, d_status,
                          mdev, wm, NA_MAX_BLOCKS, d_content, params->min_value, false, 2, remap_grid,
                          HandOver{nullptr, nullptr}, s));

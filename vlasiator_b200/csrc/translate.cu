@@ -184,7 +184,8 @@ __global__ void __launch_bounds__(UNION_THREADS) pencil_union_kernel(
    const uint32_t* __restrict__ gids, const CellSlot* __restrict__ slots, int dim, uint32_t nx, uint32_t ny,
    uint32_t N, uint32_t n_words, uint32_t* __restrict__ item_gid, uint32_t* __restrict__ item_pencil,
    uint32_t* __restrict__ rows, uint32_t* __restrict__ srcs, const uint32_t* __restrict__ src_index,
-   uint32_t item_cap, uint64_t row_cap, TransCounters* __restrict__ tc, uint32_t* __restrict__ status) {
+   uint32_t zero_row, uint32_t item_cap, uint64_t row_cap, TransCounters* __restrict__ tc,
+   uint32_t* __restrict__ status) {
    extern __shared__ uint32_t usm[];
    uint32_t* bm = usm;             // n_words: union bitmap
    uint32_t* pre = usm + n_words;  // n_words: union entries before each word
@@ -259,14 +260,15 @@ __global__ void __launch_bounds__(UNION_THREADS) pencil_union_kernel(
    const uint64_t row0 = (uint64_t)base * N;
    for (uint64_t e = threadIdx.x; e < (uint64_t)total * N; e += blockDim.x) {
       rows[row0 + e] = NO_ROW;
-      srcs[row0 + e] = NO_DATA;
+      srcs[row0 + e] = zero_row;
    }
    __syncthreads();
    for_blocks([&](uint32_t x, uint32_t at, uint32_t g) {
       const uint32_t w = g >> 5;
       const uint32_t r = pre[w] + __popc(bm[w] & ((1u << (g & 31)) - 1u));
       rows[row0 + (uint64_t)r * N + x] = at;
-      srcs[row0 + (uint64_t)r * N + x] = src_index ? src_index[at] : at;
+      const uint32_t row = src_index ? src_index[at] : at;
+      srcs[row0 + (uint64_t)r * N + x] = (row == NO_DATA) ? zero_row : row;
    });
 }
 
@@ -430,11 +432,10 @@ __device__ __forceinline__ void plane_shift(uint32_t sw2, int k, float dvz, floa
    wm = up ? -zt : -zt - 1.0f;
 }
 
-// This lane's two columns of the block at data index idx (zeros where the
-// cell lacks the block).
-__device__ __forceinline__ float2 load_column_pair(const float* __restrict__ src, uint32_t idx, int lane) {
-   return (idx != NO_DATA) ? reinterpret_cast<const float2*>(src + (size_t)idx * WID3)[lane]
-                           : make_float2(0.0f, 0.0f);
+// This lane's two columns of the block at data row idx (src2: the lane's place
+// in row 0).
+__device__ __forceinline__ float2 load_column_pair(const float2* __restrict__ src2, uint32_t idx) {
+   return __ldg(src2 + (size_t)idx * (WID3 / 2));
 }
 
 // px (py) = 1 when the plane of this lane's first (second) column holds a
@@ -509,6 +510,8 @@ __global__ void __launch_bounds__(TF_THREADS, TF_CTAS) trans_fused_kernel(
    const uint32_t pmask = plane_lanes<DIM>(lane);
    const int kx = lane_plane<DIM>(lane), ky = (DIM == 0) ? kx + 1 : kx;
    const float dvz = mesh.dv[DIM], vz_min = mesh.vmin[DIM];
+   const float2* __restrict__ src2 = reinterpret_cast<const float2*>(src) + lane;
+   float2* __restrict__ dst2 = reinterpret_cast<float2*>(dst) + lane;
 
    // copy item q's header and tables into slice sl (entries past row_cap, of
    // an item whose pencil did not fit, read as none)
@@ -525,7 +528,7 @@ __global__ void __launch_bounds__(TF_THREADS, TF_CTAS) trans_fused_kernel(
       for (uint32_t m = lane; m < N + 6; m += 32) {
          const uint32_t cell = (m + 3u * N - 3u) % N;
          if (base + cell < row_cap) cp_async4(sl + 2 + m, srcs + base + cell);
-         else sl[2 + m] = NO_DATA;
+         else sl[2 + m] = 0u;
       }
       for (uint32_t m = lane; m < N; m += 32) {
          if (base + m < row_cap) cp_async4(sl + N + 8 + m, rows + base + m);
@@ -556,12 +559,13 @@ __global__ void __launch_bounds__(TF_THREADS, TF_CTAS) trans_fused_kernel(
       const float2 share = make_float2(upx ? 1.0f : 0.0f, upy ? 1.0f : 0.0f);
       const float2 turn = make_float2(upx ? -1.0f : 1.0f, upy ? -1.0f : 1.0f);
 
-      // window cells -3 .. L+2 of the first batch (past N+2: not needed, any
-      // positive value)
+      for (uint32_t m = lane; m < N; m += 32)
+         if (trow[m] != NO_ROW) dst_gids[trow[m]] = gid;
+
+      // window cells -3 .. L+2 of the first batch (past N+2, not needed: the
+      // last one again)
       float2 w[W];
-      auto window_cell = [&](uint32_t m) {
-         return (m < N + 6) ? load_column_pair(src, tsrc[m], lane) : make_float2(1.0f, 1.0f);
-      };
+      auto window_cell = [&](uint32_t m) { return load_column_pair(src2, tsrc[min(m, N + 5)]); };
 #pragma unroll
       for (int j = 0; j < W; ++j) w[j] = window_cell((uint32_t)j);
       // every value of the window's first six cells positive / of the others
@@ -619,36 +623,35 @@ __global__ void __launch_bounds__(TF_THREADS, TF_CTAS) trans_fused_kernel(
          auto batch = [&](auto test, uint32_t ax, uint32_t ay) {
 #pragma unroll
             for (int i = 0; i < L; ++i) {
-               if (s0 + (uint32_t)i >= N) break;  // the last batch of a pencil may be short
+               if (s0 + (uint32_t)i >= N) return false;  // the pencil ends inside this batch
                float2 nb = outgoing(w[i + 3], w[i + 4], w[i + 5], w[(i + 6 < W) ? i + 6 : W - 1]);
                if constexpr (decltype(test)::value) {
                   if (!((ax >> (i + 4)) & 1u)) nb.x = 0.0f;
                   if (!((ay >> (i + 4)) & 1u)) nb.y = 0.0f;
                }
                const uint32_t r = trow[s0 + i];
-               if (r != NO_ROW) {
-                  float2 own = p_minus(w[i + 3], nb_0);
-                  if constexpr (decltype(test)::value) {
-                     if (!((ax >> (i + 3)) & 1u)) own.x = 0.0f;
-                     if (!((ay >> (i + 3)) & 1u)) own.y = 0.0f;
-                  }
-                  const float2 out = __fadd2_rn(own, make_float2(upx ? nb_m1.x : nb.x, upy ? nb_m1.y : nb.y));
-                  reinterpret_cast<float2*>(dst + (size_t)r * WID3)[lane] = out;
-                  if (lane == 0) dst_gids[r] = gid;
+               float2 own = p_minus(w[i + 3], nb_0);
+               if constexpr (decltype(test)::value) {
+                  if (!((ax >> (i + 3)) & 1u)) own.x = 0.0f;
+                  if (!((ay >> (i + 3)) & 1u)) own.y = 0.0f;
                }
+               const float2 out = __fadd2_rn(own, make_float2(upx ? nb_m1.x : nb.x, upy ? nb_m1.y : nb.y));
+               if (r != NO_ROW) dst2[(size_t)r * (WID3 / 2)] = out;
                nb_m1 = nb_0;
                nb_0 = nb;
             }
+            return true;
          };
          const bool tail = positive(6, W);
          if (head && tail) {
-            batch(std::false_type{}, 0u, 0u);
+            if (!batch(std::false_type{}, 0u, 0u)) break;
          } else {
             // bit j: some positive value in window cells j-2 .. j+2
             uint32_t posx, posy;
             plane_bits(posx, posy);
-            batch(std::true_type{}, posx | (posx << 1) | (posx << 2) | (posx >> 1) | (posx >> 2),
-                  posy | (posy << 1) | (posy << 2) | (posy >> 1) | (posy >> 2));
+            if (!batch(std::true_type{}, posx | (posx << 1) | (posx << 2) | (posx >> 1) | (posx >> 2),
+                       posy | (posy << 1) | (posy << 2) | (posy >> 1) | (posy >> 2)))
+               break;
          }
          head = tail;
          s0 += L;
@@ -684,8 +687,8 @@ uint32_t union_words(const MeshDev& mesh) { return (mesh.len[0] * mesh.len[1] * 
 
 cudaError_t launch_pencil_union(const uint32_t* gids, const CellSlot* slots, int dim, uint32_t nx, uint32_t ny,
                                 uint32_t nz, const MeshDev& mesh, uint32_t* item_gid, uint32_t* item_pencil,
-                                uint32_t* rows, uint32_t* srcs, const uint32_t* src_index, uint32_t item_cap,
-                                uint64_t row_cap, TransCounters* tc, uint32_t* status, cudaStream_t stream) {
+                                uint32_t* rows, uint32_t* srcs, const uint32_t* src_index, uint32_t zero_row,
+                                uint32_t item_cap, uint64_t row_cap, TransCounters* tc, uint32_t* status, cudaStream_t stream) {
    const uint32_t dims[3] = {nx, ny, nz};
    const uint32_t N = dims[dim];
    const uint32_t n_pencils = nx * ny * nz / N;
@@ -694,7 +697,8 @@ cudaError_t launch_pencil_union(const uint32_t* gids, const CellSlot* slots, int
    cudaError_t e = cudaFuncSetAttribute(pencil_union_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
    if (e != cudaSuccess) return e;
    pencil_union_kernel<<<n_pencils, UNION_THREADS, smem, stream>>>(gids, slots, dim, nx, ny, N, n_words, item_gid,
-                                                                     item_pencil, rows, srcs, src_index, item_cap,
+                                                                     item_pencil, rows, srcs, src_index, zero_row,
+                                                                     item_cap,
                                                                      row_cap, tc, status);
    return cudaGetLastError();
 }
