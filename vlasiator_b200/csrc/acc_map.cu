@@ -159,10 +159,15 @@ __device__ __forceinline__ void set_corners(const SweepCell& P, uint32_t si, uin
 // ---------------------------------------------------------------------------
 // columnize: one CTA per cell
 // ---------------------------------------------------------------------------
-// Threads per CTA: COL_THREADS where the cells outnumber the SMs, so that six
-// CTAs share an SM and hide one another's barriers; COL_FEW_THREADS where a
-// CTA has an SM to itself anyway (launch_columnize_batch).
+// Threads per CTA (launch_columnize_batch).  Where every cell has an SM to
+// itself the largest cell is the launch's time, so its CTA is as large as can
+// be; up to eight cells per SM the largest ones still decide; with more cells
+// six small CTAs share an SM and hide one another's barriers.  A step of 13
+// cells of 12000 blocks, with 1024 threads: 1215 -> 872 us; of 1024 drifting
+// cells (512 against 256 threads, the adjustment's lists likewise): 1451 ->
+// 1375 us; of 4096: 512 threads take 2% longer than 256.
 constexpr int COL_THREADS = 256;
+constexpr int COL_MID_THREADS = 512;
 constexpr int COL_FEW_THREADS = 1024;
 constexpr int COL_UNROLL = 4;  // list entries a thread has in flight
 constexpr uint32_t NO_BLOCK = 0xffffffffu;  // a list entry without data: all zero
@@ -1574,20 +1579,26 @@ cudaError_t launch_columnize_batch(int dim, const uint32_t* gids, const uint32_t
    const size_t smem = columnize_smem_bytes(li * lj);
    const uint32_t g2 = (uint32_t)wide_grid < n_cells ? (uint32_t)wide_grid : n_cells;
    cudaError_t e = cudaSuccess;
-#define VLGPU_COLB(D)                                                                                           \
-   e = cudaFuncSetAttribute(columnize_kernel<D, COL_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,      \
+#define VLGPU_COLB(D, THREADS)                                                                                           \
+   e = cudaFuncSetAttribute(columnize_kernel<D, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,      \
                             (int)smem);                                                                          \
    if (e != cudaSuccess) return e;                                                                               \
    e = cudaFuncSetAttribute(columnize_wide_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
    if (e != cudaSuccess) return e;                                                                               \
-   columnize_kernel<D, COL_THREADS><<<n_cells, COL_THREADS, smem_cap, stream>>>(                                              \
+   columnize_kernel<D, THREADS><<<n_cells, THREADS, smem_cap, stream>>>(                                              \
       gids, src_index, src_slots, dst_slots, perm, sets, set_capacity, dst_capacity, sweep_cells, status, counters, \
       stats, mesh, wall_margin, 0, n_cells, first_of_step, zero_row, order, cap, wide_cells, nullptr);                              \
    columnize_wide_kernel<D><<<g2, COL_FEW_THREADS, smem, stream>>>(gids, src_index, src_slots, dst_slots, perm, sets, \
                                                                set_capacity, dst_capacity, sweep_cells, status,   \
                                                                counters, stats, mesh, wall_margin, first_of_step, \
                                                                zero_row, wide_cells);
-   if (dim == 0) { VLGPU_COLB(0) } else if (dim == 1) { VLGPU_COLB(1) } else { VLGPU_COLB(2) }
+   if (n_cells <= 8 * few_cells) {
+      if (dim == 0) { VLGPU_COLB(0, COL_MID_THREADS) } else if (dim == 1) { VLGPU_COLB(1, COL_MID_THREADS) }
+      else { VLGPU_COLB(2, COL_MID_THREADS) }
+   } else {
+      if (dim == 0) { VLGPU_COLB(0, COL_THREADS) } else if (dim == 1) { VLGPU_COLB(1, COL_THREADS) }
+      else { VLGPU_COLB(2, COL_THREADS) }
+   }
 #undef VLGPU_COLB
    return cudaGetLastError();
 }

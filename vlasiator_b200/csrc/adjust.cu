@@ -35,7 +35,10 @@
 namespace vlgpu {
 
 constexpr int ADJ_THREADS = 256;
-constexpr int ADJ_FEW_THREADS = 1024;  // list CTAs where the cells do not outnumber the SMs
+// list CTAs where the cells do not outnumber the SMs, and up to eight cells
+// per SM (the rule and the figures are columnize's, acc_map.cu)
+constexpr int ADJ_FEW_THREADS = 1024;
+constexpr int ADJ_MID_THREADS = 512;
 constexpr int ADJ_ROWS = 2;           // rows a lane has in flight, and as many on their way
 constexpr int ADJ_VALUE_CTAS = 3;         // CTAs per SM of the pass over the values
 constexpr int ADJ_UNROLL = 4;          // list entries per thread in flight
@@ -753,12 +756,7 @@ cudaError_t launch_adjust(const uint32_t* gids, const uint32_t* src_index, const
                           cudaStream_t stream) {
    if (n_cells == 0) return cudaSuccess;
    const size_t smem = adjust_smem_bytes();
-   const bool few = n_cells <= few_cells;
-   cudaError_t e = few ? cudaFuncSetAttribute(adjust_kernel<ADJ_FEW_THREADS>,
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                       : cudaFuncSetAttribute(adjust_kernel<ADJ_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)smem);
-   if (e != cudaSuccess) return e;
+   cudaError_t e = cudaSuccess;
    if (!content_valid) {
       float threshold = (float)min_value;  // the smallest float >= min_value
       if ((double)threshold < min_value) threshold = std::nextafterf(threshold, FLT_MAX);
@@ -776,12 +774,19 @@ cudaError_t launch_adjust(const uint32_t* gids, const uint32_t* src_index, const
    // the counters are zero here
    const uint32_t g = (uint32_t)grid < n_cells ? (uint32_t)grid : n_cells;
 #define VLGPU_ADJ(T)                                                                                               \
+   e = cudaFuncSetAttribute(adjust_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);            \
+   if (e != cudaSuccess) return e;                                                                                 \
    adjust_kernel<T><<<g, T, smem, stream>>>(gids, src_index, slots, content, neighbors, out_gids, out_src,        \
                                             out_slots, status, counters, out_capacity, mesh, add_width,            \
                                             n_cells, ADJ_SMEM_ROWS, scratch, use_masks ? masks : nullptr, pool,    \
                                             order, kept, items, mom_record, pivot, write_pivot)
-   if (few) VLGPU_ADJ(ADJ_FEW_THREADS);
-   else VLGPU_ADJ(ADJ_THREADS);
+   if (n_cells <= few_cells) {
+      VLGPU_ADJ(ADJ_FEW_THREADS);
+   } else if (n_cells <= 8 * few_cells) {
+      VLGPU_ADJ(ADJ_MID_THREADS);
+   } else {
+      VLGPU_ADJ(ADJ_THREADS);
+   }
 #undef VLGPU_ADJ
    if ((e = cudaGetLastError()) != cudaSuccess) return e;
    if (mom_record)

@@ -419,14 +419,15 @@ __device__ __forceinline__ int lane_plane(int lane) {
    return lane >> 3;
 }
 
-// Shift of plane k of the block at swapped index sw2 along the sweep
-// dimension, as a fraction of the cell (cpu_trans_map_amr.cpp:60-80).  The
-// part that leaves a cell is the one above the edge w = 1 - z where the plane
-// moves up, the one below w = -z where it moves down; wm = w - 1.
-__device__ __forceinline__ void plane_shift(uint32_t sw2, int k, float dvz, float vz_min, float dt, float h, float& w,
-                                            float& wm, bool& up) {
-   const float cell_vz = __double2float_rn(((double)(sw2 * WID + k) + 0.5) * (double)dvz + (double)vz_min);
-   const float zt = __fdiv_rn(__fmul_rn(cell_vz, dt), h);
+// Shift of the velocity plane `plane` (cells along the sweep dimension), as a
+// fraction of the cell (cpu_trans_map_amr.cpp:60-80).
+__device__ __forceinline__ float plane_shift(uint32_t plane, float dvz, float vz_min, float dt, float h) {
+   const float cell_vz = __double2float_rn(((double)plane + 0.5) * (double)dvz + (double)vz_min);
+   return __fdiv_rn(__fmul_rn(cell_vz, dt), h);
+}
+// The part that leaves a cell is the one above the edge w = 1 - zt where the
+// plane moves up, the one below w = -zt where it moves down; wm = w - 1.
+__device__ __forceinline__ void plane_edge(float zt, float& w, float& wm, bool& up) {
    up = zt > 0.0f;
    w = up ? 1.0f - zt : -zt;
    wm = up ? -zt : -zt - 1.0f;
@@ -510,6 +511,11 @@ __global__ void __launch_bounds__(TF_THREADS, TF_CTAS) trans_fused_kernel(
    const uint32_t pmask = plane_lanes<DIM>(lane);
    const int kx = lane_plane<DIM>(lane), ky = (DIM == 0) ? kx + 1 : kx;
    const float dvz = mesh.dv[DIM], vz_min = mesh.vmin[DIM];
+   // the shifts of all planes, once per CTA
+   __shared__ float s_shift[WID * MAX_LEN];
+   for (uint32_t k = threadIdx.x; k < WID * mesh.len[DIM]; k += TF_THREADS)
+      s_shift[k] = plane_shift(k, dvz, vz_min, dt, h);
+   __syncthreads();
    const float2* __restrict__ src2 = reinterpret_cast<const float2*>(src) + lane;
    float2* __restrict__ dst2 = reinterpret_cast<float2*>(dst) + lane;
 
@@ -526,7 +532,9 @@ __global__ void __launch_bounds__(TF_THREADS, TF_CTAS) trans_fused_kernel(
       }
       const uint64_t base = (uint64_t)q * N;
       for (uint32_t m = lane; m < N + 6; m += 32) {
-         const uint32_t cell = (m + 3u * N - 3u) % N;
+         // (m - 3) mod N: at most one step, or a few where N < 6
+         uint32_t cell = (m < 3u) ? m + 3u * N - 3u : m - 3u;
+         while (cell >= N) cell -= N;
          if (base + cell < row_cap) cp_async4(sl + 2 + m, srcs + base + cell);
          else sl[2 + m] = 0u;
       }
@@ -549,12 +557,13 @@ __global__ void __launch_bounds__(TF_THREADS, TF_CTAS) trans_fused_kernel(
       prefetch(q + n_warps, slices + (parity ^ 1u) * tf_slice_words(N));
       if (pencil == BAD_ITEM) continue;
 
-      uint32_t sw[3];
-      swapped_indices(gid, mesh.len, DIM, sw);
+      uint32_t bx, by, bz;
+      block_xyz(mesh, gid, bx, by, bz);
+      const float* const zt = s_shift + WID * (DIM == 0 ? bx : (DIM == 1 ? by : bz));
       float2 we, wm;
       bool upx, upy;
-      plane_shift(sw[2], kx, dvz, vz_min, dt, h, we.x, wm.x, upx);
-      plane_shift(sw[2], ky, dvz, vz_min, dt, h, we.y, wm.y, upy);
+      plane_edge(zt[kx], we.x, wm.x, upx);
+      plane_edge(zt[ky], we.y, wm.y, upy);
       // outgoing = share v0 + turn I(we)
       const float2 share = make_float2(upx ? 1.0f : 0.0f, upy ? 1.0f : 0.0f);
       const float2 turn = make_float2(upx ? -1.0f : 1.0f, upy ? -1.0f : 1.0f);
