@@ -108,12 +108,13 @@ constexpr uint32_t TR_MAX_N = 128;
 cudaError_t launch_pencil_union(const uint32_t* gids, const CellSlot* slots, int dim, uint32_t nx, uint32_t ny,
                                 uint32_t nz, const MeshDev& mesh, uint32_t* item_gid, uint32_t* item_pencil,
                                 uint32_t* rows, uint32_t* srcs, const uint32_t* src_index, uint32_t zero_row,
-                                uint32_t item_cap, uint64_t row_cap, TransCounters* tc, uint32_t* status, cudaStream_t stream);
+                                uint32_t item_cap, uint64_t row_cap, TransCounters* tc, uint32_t* status, CellSlot* dst_slots,
+                                const uint32_t* rows_in, uint32_t* rows_out, cudaStream_t stream);
 cudaError_t launch_trans_remap(int dim, uint32_t N, const uint32_t* item_gid, const uint32_t* item_pencil,
                                const uint32_t* rows, const uint32_t* srcs, TransCounters* tc, uint32_t item_cap,
                                uint64_t row_cap, const uint32_t* src_index, const float* src, float* dst,
                                uint32_t* dst_gids, const MeshDev& mesh, float dt, float dz, float threshold, bool exact,
-                               int grid, cudaStream_t stream);
+                               int grid, TransCounters* next, cudaStream_t stream);
 int trans_blocks_per_sm(uint32_t N, bool exact);
 uint32_t union_words(const MeshDev& mesh);
 constexpr int MOM_COUNT = 16;
@@ -191,7 +192,8 @@ struct vlgpu_batch {
    uint32_t* trans_rows = nullptr;  // per item and pencil cell: list row of the block (or none)
    uint32_t* trans_src = nullptr;   // the same entries: data index in the source pool (or none)
    uint64_t row_cap = 0;
-   TransCounters* tcounters = nullptr;
+   TransCounters* tcounters = nullptr;  // two, in turn: the next sweep's (`trans_turn`) is zero
+   int trans_turn = 0;
    int32_t* neighbors = nullptr;  // 26 per cell (-1: none), the spatial neighbours block adjustment consults
    double* dt_buf = nullptr;      // 2 per cell: r-space and v-space time-step limits
    uint32_t* adj_scratch = nullptr;  // per adjustment CTA: masks of a cell too wide for shared memory
@@ -227,6 +229,7 @@ struct vlgpu_batch {
       int cur = 0;
       int adj_next = 0;
       int turn = 0;
+      int trans_turn = 0;
       bool pivot_valid = false;      // at the start of the captured steps
       bool pivot_valid_end = false;  // after them
       unsigned long long launches = 0;

@@ -269,22 +269,19 @@ int accelerate_device(vlgpu_batch* b, uint32_t map_order, bool per_cell, bool ne
 int translate_device(vlgpu_batch* b, uint32_t dim, double dt) {
    const int d = 1 - b->cur;
    const uint32_t N = b->grid_dims[dim];
-   VL_CHECK(cudaMemsetAsync(b->tcounters, 0, sizeof(TransCounters), b->stream));
+   TransCounters* const tc = b->tcounters + b->trans_turn;
+   b->trans_turn ^= 1;
    VL_CHECK(launch_pencil_union(b->st_gids, b->st_slots, (int)dim, b->grid_dims[0], b->grid_dims[1],
                                 b->grid_dims[2], b->mdev, b->item_gid, b->item_pencil, b->trans_rows,
-                                b->trans_src, b->st_src, (uint32_t)b->capacity, (uint32_t)b->capacity, b->row_cap, b->tcounters, b->status,
-                                b->stream));
+                                b->trans_src, b->st_src, (uint32_t)b->capacity, (uint32_t)b->capacity, b->row_cap, tc, b->status, b->slots[d],
+                                b->rows_used + b->st_list, b->rows_used + d, b->stream));
    int per_sm = trans_blocks_per_sm(N, b->exact);
    if (b->cps[3] > 0 && (int)b->cps[3] < per_sm) per_sm = (int)b->cps[3];
    const int grid = b->sm_count * per_sm;
-   VL_CHECK(launch_trans_remap((int)dim, N, b->item_gid, b->item_pencil, b->trans_rows, b->trans_src, b->tcounters,
+   VL_CHECK(launch_trans_remap((int)dim, N, b->item_gid, b->item_pencil, b->trans_rows, b->trans_src, tc,
                                (uint32_t)b->capacity, b->row_cap, b->st_src, b->data[b->cur], b->data[d], b->gids[d],
                                b->mdev, (float)dt, (float)b->grid_dx[dim], (float)b->params.min_value, b->exact, grid,
-                               b->stream));
-   VL_CHECK(cudaMemcpyAsync(b->slots[d], b->st_slots, sizeof(CellSlot) * b->n_cells, cudaMemcpyDeviceToDevice,
-                            b->stream));
-   VL_CHECK(cudaMemcpyAsync(b->rows_used + d, b->rows_used + b->st_list, sizeof(uint32_t), cudaMemcpyDeviceToDevice,
-                            b->stream));
+                               b->tcounters + b->trans_turn, b->stream));
    b->launches += 2;
    set_direct_state(b, d);
    b->content_valid = false;
@@ -814,8 +811,8 @@ int vlgpu_batch_set_grid(vlgpu_batch* b, const uint32_t dims[3], const double dx
       VL_CHECK(cudaMalloc(&b->mask_recs, sizeof(MaskRec) * b->n_cells));
       VL_CHECK(cudaMalloc(&b->mask_pool, sizeof(uint32_t) * words));
       VL_CHECK(cudaMalloc(&b->mask_top, sizeof(uint32_t)));
-      VL_CHECK(cudaMalloc(&b->tcounters, sizeof(TransCounters)));
-      VL_CHECK(cudaMemset(b->tcounters, 0, sizeof(TransCounters)));
+      VL_CHECK(cudaMalloc(&b->tcounters, 2 * sizeof(TransCounters)));
+      VL_CHECK(cudaMemset(b->tcounters, 0, 2 * sizeof(TransCounters)));
    }
    // the 26 nearest neighbours of every cell, periodic, the cell itself excluded
    std::vector<int32_t> nb((size_t)b->n_cells * 26);
@@ -983,7 +980,7 @@ int vlgpu_batch_capture(vlgpu_batch* b, int slot, int kind, uint32_t n_steps, co
       g.exec = nullptr;
    }
    const vlgpu_batch::GraphSlot start{nullptr,     b->st_gids, b->st_src,      b->st_slots, b->cur,
-                                      b->adj_next, b->turn,    b->pivot_valid, false,       0, 0};
+                                      b->adj_next, b->turn,    b->trans_turn,  b->pivot_valid, false, 0, 0};
    const bool content_valid = b->content_valid;
    const unsigned long long l0 = b->launches, r0 = b->remap_launches;
    VL_CHECK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeRelaxed));
@@ -995,13 +992,14 @@ int vlgpu_batch_capture(vlgpu_batch* b, int slot, int kind, uint32_t n_steps, co
    // nothing ran: the host's view of the buffers is the one before the capture
    const bool same_buffers = b->st_gids == start.st_gids && b->st_src == start.st_src &&
                              b->st_slots == start.st_slots && b->cur == start.cur && b->adj_next == start.adj_next &&
-                             b->turn == start.turn;
+                             b->turn == start.turn && b->trans_turn == start.trans_turn;
    b->st_gids = start.st_gids;
    b->st_src = start.st_src;
    b->st_slots = start.st_slots;
    b->cur = start.cur;
    b->adj_next = start.adj_next;
    b->turn = start.turn;
+   b->trans_turn = start.trans_turn;
    b->content_valid = content_valid;
    const bool pivot_end = b->pivot_valid;
    b->pivot_valid = start.pivot_valid;
@@ -1040,6 +1038,10 @@ int vlgpu_batch_replay(vlgpu_batch* b, int slot) {
       VL_CHECK(cudaMemsetAsync(b->counters + g.turn, 0, sizeof(SweepCounters), b->stream));
       b->turn = g.turn;
    }
+   if (b->trans_turn != g.trans_turn) {
+      VL_CHECK(cudaMemsetAsync(b->tcounters + g.trans_turn, 0, sizeof(TransCounters), b->stream));
+      b->trans_turn = g.trans_turn;
+   }
    VL_CHECK(cudaGraphLaunch(g.exec, b->stream));
    b->launches += g.launches;
    b->remap_launches += g.remap_launches;
@@ -1070,7 +1072,7 @@ int vlgpu_batch_sync(vlgpu_batch* b) {
    if (c.overflow) return VLGPU_ENOMEM;
    if (b->tcounters) {
       TransCounters t{};
-      VL_CHECK(cudaMemcpy(&t, b->tcounters, sizeof(t), cudaMemcpyDeviceToHost));
+      VL_CHECK(cudaMemcpy(&t, b->tcounters + (b->trans_turn ^ 1), sizeof(t), cudaMemcpyDeviceToHost));
       if (t.overflow) return VLGPU_ENOMEM;
    }
    return VLGPU_OK;

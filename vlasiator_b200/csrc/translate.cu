@@ -63,7 +63,8 @@ constexpr uint32_t UNION_UNROLL = 4;         // pencil cells whose lists a threa
 constexpr int TR_THREADS = 256;
 constexpr uint32_t TR_MAX_N = 128;           // cells per pencil
 
-// Counters of one translation sweep, zeroed before the union kernel.
+// Counters of one translation sweep.  A batch uses two in turn: the remap
+// kernel, the sweep's last, zeroes the next sweep's.
 struct TransCounters {
    uint32_t n_items;
    uint32_t work;
@@ -185,7 +186,8 @@ __global__ void __launch_bounds__(UNION_THREADS) pencil_union_kernel(
    uint32_t N, uint32_t n_words, uint32_t* __restrict__ item_gid, uint32_t* __restrict__ item_pencil,
    uint32_t* __restrict__ rows, uint32_t* __restrict__ srcs, const uint32_t* __restrict__ src_index,
    uint32_t zero_row, uint32_t item_cap, uint64_t row_cap, TransCounters* __restrict__ tc,
-   uint32_t* __restrict__ status) {
+   uint32_t* __restrict__ status, CellSlot* __restrict__ dst_slots, const uint32_t* __restrict__ rows_in,
+   uint32_t* __restrict__ rows_out) {
    extern __shared__ uint32_t usm[];
    uint32_t* bm = usm;             // n_words: union bitmap
    uint32_t* pre = usm + n_words;  // n_words: union entries before each word
@@ -194,6 +196,12 @@ __global__ void __launch_bounds__(UNION_THREADS) pencil_union_kernel(
    __shared__ int s_ok;
    const uint32_t p = blockIdx.x;
    for (uint32_t w = threadIdx.x; w < n_words; w += blockDim.x) bm[w] = 0u;
+   // the sweep keeps the lists: slots and row count go to the output as they are
+   for (uint32_t x = threadIdx.x; x < N; x += blockDim.x) {
+      const uint32_t c = pencil_cell(p, x, dim, nx, ny);
+      dst_slots[c] = slots[c];
+   }
+   if (p == 0 && threadIdx.x == 0) *rows_out = *rows_in;
    __syncthreads();
    // the pencil's lists, UNION_UNROLL cells at a time so that their slots and
    // IDs are on their way together: visit(x, list position, block ID)
@@ -280,8 +288,9 @@ __global__ void __launch_bounds__(TR_THREADS) trans_remap_kernel(
    const uint32_t* __restrict__ item_gid, const uint32_t* __restrict__ item_pencil, const uint32_t* __restrict__ rows,
    TransCounters* __restrict__ tc, uint32_t item_cap, const uint32_t* __restrict__ src_index,
    const float* __restrict__ src, float* __restrict__ dst, uint32_t* __restrict__ dst_gids, MeshDev mesh,
-   uint32_t N, FaceConsts fc, float dt, float threshold, float scale) {
+   uint32_t N, FaceConsts fc, float dt, float threshold, float scale, TransCounters* __restrict__ next) {
    extern __shared__ float tsm[];
+   if (blockIdx.x == 0 && threadIdx.x == 0) *next = TransCounters{};
    const uint32_t NE = N * WID3;
    float* V = tsm;                          // values of the item's blocks, [x][c]
    float* NB = tsm + NE;                    // outgoing integral (ngbr) of every cell
@@ -499,15 +508,13 @@ __global__ void __launch_bounds__(TF_THREADS, TF_CTAS) trans_fused_kernel(
    const uint32_t* __restrict__ item_gid, const uint32_t* __restrict__ item_pencil, const uint32_t* __restrict__ rows,
    const uint32_t* __restrict__ srcs, const TransCounters* __restrict__ tc, uint32_t item_cap, uint64_t row_cap,
    const float* __restrict__ src, float* __restrict__ dst, uint32_t* __restrict__ dst_gids, MeshDev mesh,
-   uint32_t N, float dt, float h) {
+   uint32_t N, float dt, float h, TransCounters* __restrict__ next) {
    constexpr int W = L + 6;
    extern __shared__ uint32_t tf_smem[];
    const int lane = threadIdx.x & 31;
    uint32_t* const slices = tf_smem + (threadIdx.x >> 5) * 2 * tf_slice_words(N);
    const uint32_t warp0 = (blockIdx.x * TF_THREADS + threadIdx.x) >> 5;
    const uint32_t n_warps = (gridDim.x * TF_THREADS) >> 5;
-   uint32_t n_items = *((const volatile uint32_t*)&tc->n_items);
-   n_items = (n_items < item_cap) ? n_items : item_cap;
    const uint32_t pmask = plane_lanes<DIM>(lane);
    const int kx = lane_plane<DIM>(lane), ky = (DIM == 0) ? kx + 1 : kx;
    const float dvz = mesh.dv[DIM], vz_min = mesh.vmin[DIM];
@@ -516,6 +523,9 @@ __global__ void __launch_bounds__(TF_THREADS, TF_CTAS) trans_fused_kernel(
    for (uint32_t k = threadIdx.x; k < WID * mesh.len[DIM]; k += TF_THREADS)
       s_shift[k] = plane_shift(k, dvz, vz_min, dt, h);
    __syncthreads();
+   if (blockIdx.x == 0 && threadIdx.x == 0) *next = TransCounters{};
+   uint32_t n_items = tc->n_items;
+   n_items = (n_items < item_cap) ? n_items : item_cap;
    const float2* __restrict__ src2 = reinterpret_cast<const float2*>(src) + lane;
    float2* __restrict__ dst2 = reinterpret_cast<float2*>(dst) + lane;
 
@@ -697,7 +707,8 @@ uint32_t union_words(const MeshDev& mesh) { return (mesh.len[0] * mesh.len[1] * 
 cudaError_t launch_pencil_union(const uint32_t* gids, const CellSlot* slots, int dim, uint32_t nx, uint32_t ny,
                                 uint32_t nz, const MeshDev& mesh, uint32_t* item_gid, uint32_t* item_pencil,
                                 uint32_t* rows, uint32_t* srcs, const uint32_t* src_index, uint32_t zero_row,
-                                uint32_t item_cap, uint64_t row_cap, TransCounters* tc, uint32_t* status, cudaStream_t stream) {
+                                uint32_t item_cap, uint64_t row_cap, TransCounters* tc, uint32_t* status, CellSlot* dst_slots,
+                                const uint32_t* rows_in, uint32_t* rows_out, cudaStream_t stream) {
    const uint32_t dims[3] = {nx, ny, nz};
    const uint32_t N = dims[dim];
    const uint32_t n_pencils = nx * ny * nz / N;
@@ -708,7 +719,7 @@ cudaError_t launch_pencil_union(const uint32_t* gids, const CellSlot* slots, int
    pencil_union_kernel<<<n_pencils, UNION_THREADS, smem, stream>>>(gids, slots, dim, nx, ny, N, n_words, item_gid,
                                                                      item_pencil, rows, srcs, src_index, zero_row,
                                                                      item_cap,
-                                                                     row_cap, tc, status);
+                                                                     row_cap, tc, status, dst_slots, rows_in, rows_out);
    return cudaGetLastError();
 }
 
@@ -733,12 +744,12 @@ cudaError_t launch_trans_remap(int dim, uint32_t N, const uint32_t* item_gid, co
                                const uint32_t* rows, const uint32_t* srcs, TransCounters* tc, uint32_t item_cap,
                                uint64_t row_cap, const uint32_t* src_index, const float* src, float* dst,
                                uint32_t* dst_gids, const MeshDev& mesh, float dt, float dz, float threshold, bool exact,
-                               int grid, cudaStream_t stream) {
+                               int grid, TransCounters* next, cudaStream_t stream) {
    if (!exact) {
       const size_t smem = trans_fused_smem_bytes(N);
 #define VLGPU_TF(D, L)                                                                                    \
    trans_fused_kernel<D, L><<<grid, TF_THREADS, smem, stream>>>(item_gid, item_pencil, rows, srcs, tc, item_cap, \
-                                                                row_cap, src, dst, dst_gids, mesh, N, dt, dz);
+                                                                row_cap, src, dst, dst_gids, mesh, N, dt, dz, next);
       if (dim == 0) { VLGPU_TF(0, TF_BATCH) } else if (dim == 1) { VLGPU_TF(1, TF_BATCH) } else { VLGPU_TF(2, TF_BATCH) }
 #undef VLGPU_TF
       return cudaGetLastError();
@@ -751,7 +762,7 @@ cudaError_t launch_trans_remap(int dim, uint32_t N, const uint32_t* item_gid, co
    e = cudaFuncSetAttribute(trans_remap_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);      \
    if (e != cudaSuccess) return e;                                                                               \
    trans_remap_kernel<D><<<grid, TR_THREADS, smem, stream>>>(item_gid, item_pencil, rows, tc, item_cap, src_index, \
-                                                             src, dst, dst_gids, mesh, N, fc, dt, threshold, scale);
+                                                             src, dst, dst_gids, mesh, N, fc, dt, threshold, scale, next);
    if (dim == 0) { VLGPU_TR(0) } else if (dim == 1) { VLGPU_TR(1) } else { VLGPU_TR(2) }
 #undef VLGPU_TR
    return cudaGetLastError();
