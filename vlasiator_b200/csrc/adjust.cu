@@ -82,35 +82,37 @@ __device__ __forceinline__ uint32_t adj_exclusive_scan(uint32_t v, uint32_t* war
 
 // Content flags of a list whose values no sweep has just written
 // (compute_block_has_content: any of a block's 64 values >= the threshold; an
-// added block has none), one byte per row.  Half a warp per block, four blocks
-// in flight, the blocks of a cell over the gridDim.y CTAs of its column: one
-// coalesced read of the VDF, where the list CTAs read it twice with a thread
-// per block.
-// Adjustment, moments and packing of 1024 cells (1.45 M blocks): 1446 -> 1279 us.
+// added block has none), one byte per row of the list in use.  Half a warp per
+// block, four blocks in flight: one coalesced read of the VDF, where the list
+// CTAs read it twice with a thread per block.  Over rows and not cells, so
+// that no CTA is left with a large cell: 262 us for 1024 cells of 30 to 9000
+// blocks with a CTA each, 61 us with the rows spread evenly.  (Rows of the
+// list that no cell owns any more may name any data row: only rows of the pool
+// are read.)
 constexpr int FLAG_THREADS = 256;
 constexpr uint32_t FLAG_BLOCKS = 4 * FLAG_THREADS / 16;  // blocks a CTA reads per pass
 __global__ void __launch_bounds__(FLAG_THREADS) content_flags_kernel(const uint32_t* __restrict__ src_index,
-                                                                     const CellSlot* __restrict__ slots,
-                                                                     const float* __restrict__ data, float threshold,
-                                                                     uint8_t* __restrict__ content) {
-   const CellSlot s = slots[blockIdx.x];
+                                                                     const uint32_t* __restrict__ rows_used,
+                                                                     uint32_t capacity, const float* __restrict__ data,
+                                                                     float threshold, uint8_t* __restrict__ content) {
+   const uint32_t n = min(*rows_used, capacity);
    const uint32_t sub = threadIdx.x & 15, hw = threadIdx.x >> 4, half = (threadIdx.x >> 4) & 1;
-   for (uint32_t b0 = blockIdx.y * FLAG_BLOCKS; b0 < s.count; b0 += gridDim.y * FLAG_BLOCKS) {
+   for (uint64_t b0 = (uint64_t)blockIdx.x * FLAG_BLOCKS; b0 < n; b0 += (uint64_t)gridDim.x * FLAG_BLOCKS) {
       float4 v[4];
 #pragma unroll
       for (uint32_t u = 0; u < 4; ++u) {
-         const uint32_t b = b0 + hw + u * (FLAG_THREADS / 16);
+         const uint64_t b = b0 + hw + u * (FLAG_THREADS / 16);
          v[u] = make_float4(-1.f, -1.f, -1.f, -1.f);  // the threshold is positive
-         if (b < s.count) {
-            const uint32_t row = src_index ? src_index[s.off + b] : s.off + b;
-            if (row != NO_BLOCK) v[u] = __ldg(reinterpret_cast<const float4*>(data + (size_t)row * WID3) + sub);
+         if (b < n) {
+            const uint32_t row = src_index ? src_index[b] : (uint32_t)b;
+            if (row < capacity) v[u] = __ldg(reinterpret_cast<const float4*>(data + (size_t)row * WID3) + sub);
          }
       }
 #pragma unroll
       for (uint32_t u = 0; u < 4; ++u) {
-         const uint32_t b = b0 + hw + u * (FLAG_THREADS / 16);
+         const uint64_t b = b0 + hw + u * (FLAG_THREADS / 16);
          const unsigned any = __ballot_sync(0xffffffffu, fmaxf(fmaxf(v[u].x, v[u].y), fmaxf(v[u].z, v[u].w)) >= threshold);
-         if (sub == 0 && b < s.count) content[s.off + b] = ((any >> (16 * half)) & 0xffffu) ? 1 : 0;
+         if (sub == 0 && b < n) content[b] = ((any >> (16 * half)) & 0xffffu) ? 1 : 0;
       }
    }
 }
@@ -746,7 +748,8 @@ int adjust_blocks_per_sm() {
 // `kept`: a byte per row of the old list; `items`: at most one per ADJ_TILE
 // old blocks and one per cell.  The caller lends the sweeps' work arrays.
 cudaError_t launch_adjust(const uint32_t* gids, const uint32_t* src_index, const CellSlot* slots,
-                          uint8_t* content, bool content_valid, const float* data, const int32_t* neighbors,
+                          uint8_t* content, bool content_valid, const uint32_t* rows_used, const float* data,
+                          const int32_t* neighbors,
                           uint32_t* out_gids, uint32_t* out_src, CellSlot* out_slots, double* loss, uint32_t* status, SweepCounters* counters,
                           uint32_t out_capacity, const MeshDev& mesh, double min_value, int add_width, double dv3,
                           uint32_t n_cells, uint32_t* scratch, int grid, const uint32_t* order, MaskRec* masks,
@@ -760,9 +763,8 @@ cudaError_t launch_adjust(const uint32_t* gids, const uint32_t* src_index, const
    if (!content_valid) {
       float threshold = (float)min_value;  // the smallest float >= min_value
       if ((double)threshold < min_value) threshold = std::nextafterf(threshold, FLT_MAX);
-      const uint32_t spread = 8u * few_cells / n_cells;
-      content_flags_kernel<<<dim3(n_cells, spread > 1 ? (spread < 64 ? spread : 64) : 1), FLAG_THREADS, 0, stream>>>(
-         src_index, slots, data, threshold, content);
+      content_flags_kernel<<<8 * few_cells, FLAG_THREADS, 0, stream>>>(src_index, rows_used, out_capacity, data,
+                                                                      threshold, content);
    }
    const bool use_masks = neighbors && masks && pool && pool_top;
    if (use_masks) {

@@ -66,7 +66,8 @@ cudaError_t launch_geometry(const CellAccelInputs* in, const double* moments, do
                             const double vmin[3], const double dv[3], uint32_t map_order, float threshold,
                             cudaStream_t stream);
 cudaError_t launch_adjust(const uint32_t* gids, const uint32_t* src_index, const CellSlot* slots,
-                          uint8_t* content, bool content_valid, const float* data, const int32_t* neighbors,
+                          uint8_t* content, bool content_valid, const uint32_t* rows_used, const float* data,
+                          const int32_t* neighbors,
                           uint32_t* out_gids, uint32_t* out_src, CellSlot* out_slots, double* loss, uint32_t* status, SweepCounters* counters,
                           uint32_t out_capacity, const MeshDev& mesh, double min_value, int add_width, double dv3,
                           uint32_t n_cells, uint32_t* scratch, int grid, const uint32_t* order, MaskRec* masks,

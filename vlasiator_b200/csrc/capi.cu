@@ -179,7 +179,7 @@ int adjust_device(vlgpu_batch* b, double* record, bool write_pivot) {
    frame.mass = b->params.mass;
    frame.charge = b->params.charge;
    VL_CHECK(launch_adjust(b->st_gids, b->st_src, b->st_slots, b->content, b->content_valid,
-                          b->data[b->cur], b->neighbors, b->adj_gids[a], b->adj_src[a], b->adj_slots[a], b->loss,
+                          b->rows_used + b->st_list, b->data[b->cur], b->neighbors, b->adj_gids[a], b->adj_src[a], b->adj_slots[a], b->loss,
                           b->status,
                           counters, (uint32_t)b->capacity, b->mdev, b->params.min_value,
                           (int)b->params.add_width_v, dv3, b->n_cells, b->adj_scratch, b->adj_grid,
