@@ -34,7 +34,12 @@ namespace vlgpu {
 // order with compensated sums and writes the record, so the result does not
 // depend on which warp ran which part.  Half a warp reads one velocity block,
 // each lane one x-row of four cells as a float4 (i = 0..3 at j = sub & 3,
-// k = sub >> 2), two blocks per half-warp in flight.
+// k = sub >> 2), two blocks per half-warp in flight and two on their way.
+//
+// Bound by the latency of a part's first loads and of its sums: with four rows
+// in flight, positions taken apart per lane and two CTAs per SM 270 us for
+// 1024 cells (1.45 M blocks), with corners from a table, two rows and three
+// CTAs 201 us.
 //
 // The sums are those of blockVelocityFirstMoments / blockVelocitySecondMoments
 // (vlasovsolver/arch_moments.h:83-155) and the record that of
@@ -50,7 +55,9 @@ constexpr int MOM_THREADS = 256;
 // Parts of a cell with `count` blocks: enough that a part has at least
 // MOM_MIN_PART blocks, at most MOM_PARTS_PER_CELL.
 constexpr uint32_t MOM_MIN_PART = 64;
-constexpr uint32_t MOM_TILE = 256;  // blocks of a part staged at a time
+constexpr uint32_t MOM_TILE = 128;  // blocks of a part staged at a time
+constexpr int MOM_ROWS = 2;         // rows a lane has in flight, and as many on their way
+constexpr int MOM_CTAS = 3;         // per SM
 __device__ __forceinline__ uint32_t moment_parts(uint32_t count) {
    const uint32_t p = (count + MOM_MIN_PART - 1) / MOM_MIN_PART;
    return p < (uint32_t)MOM_PARTS_PER_CELL ? p : (uint32_t)MOM_PARTS_PER_CELL;
@@ -58,7 +65,7 @@ __device__ __forceinline__ uint32_t moment_parts(uint32_t count) {
 
 
 template <int MODE>
-__global__ void __launch_bounds__(MOM_THREADS, 2) moments_parts_kernel(
+__global__ void __launch_bounds__(MOM_THREADS, MOM_CTAS) moments_parts_kernel(
    const uint32_t* __restrict__ gids, const uint32_t* __restrict__ src_index, const float* __restrict__ data,
    const CellSlot* __restrict__ slots, double* moments, double* pivot, const double* shift,
    double* __restrict__ part_sums, uint32_t* __restrict__ done, MeshDev mesh, double vmin0, double vmin1,
@@ -67,7 +74,15 @@ __global__ void __launch_bounds__(MOM_THREADS, 2) moments_parts_kernel(
    constexpr bool SECOND = MODE != MOM_FIRST;
    constexpr int NS = SECOND ? 10 : 4;
    __shared__ double sh[MOM_THREADS / 32][NS][33];  // a warp's lane sums, one row per sum (padded)
-   __shared__ uint32_t sg[MOM_THREADS / 32][MOM_TILE], si[MOM_THREADS / 32][MOM_TILE];  // a tile's block IDs, rows
+   // a tile's blocks: position x + (y << 8) + (z << 16) and data row
+   __shared__ uint32_t sg[MOM_THREADS / 32][MOM_TILE], si[MOM_THREADS / 32][MOM_TILE];
+   __shared__ double s_corner[3][MAX_LEN];  // the blocks' lower corners along each axis
+   for (int i = threadIdx.x; i < MAX_LEN; i += MOM_THREADS) {
+      s_corner[0][i] = vmin0 + i * bs0;
+      s_corner[1][i] = vmin1 + i * bs1;
+      s_corner[2][i] = vmin2 + i * bs2;
+   }
+   __syncthreads();
    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
    const int half = lane >> 4, sub = lane & 15;
    const int j = sub & 3, k = sub >> 2;
@@ -109,20 +124,22 @@ __global__ void __launch_bounds__(MOM_THREADS, 2) moments_parts_kernel(
 #pragma unroll
       for (int q = 0; q < NS; ++q) t[q] = 0.0;
       // tiles of the part: the block IDs and data rows are staged in shared
-      // memory (coalesced), then half-warp h reads blocks h, h + 2, h + 4,
-      // h + 6 of every eight, all four loads in flight at once
+      // memory (coalesced), then half-warp h reads blocks h, h + 2, .. of every
+      // 2 MOM_ROWS
       for (uint32_t t0 = b0; t0 < b1; t0 += MOM_TILE) {
          const uint32_t n = (b1 - t0 < MOM_TILE) ? b1 - t0 : MOM_TILE;
          for (uint32_t q = lane; q < n; q += 32) {
-            sg[wl][q] = __ldg(gids + s.off + t0 + q);
+            uint32_t x, y, z;
+            block_xyz(mesh, __ldg(gids + s.off + t0 + q), x, y, z);
+            sg[wl][q] = x | (y << 8) | (z << 16);
             si[wl][q] = src_index ? __ldg(src_index + s.off + t0 + q) : s.off + t0 + q;
          }
          __syncwarp();
-         // rows of blocks q0 + 2u (u = 0..3) of this half-warp, the next four
+         // rows of blocks q0 + 2u (u < MOM_ROWS) of this half-warp, as many
          // prefetched while these are summed
          auto load4 = [&](uint32_t q0, float4* f) {
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
+            for (int u = 0; u < MOM_ROWS; ++u) {
                const uint32_t q = q0 + 2 * u;
                f[u] = make_float4(0.f, 0.f, 0.f, 0.f);
                if (q < n) {
@@ -132,22 +149,21 @@ __global__ void __launch_bounds__(MOM_THREADS, 2) moments_parts_kernel(
                }
             }
          };
-         float4 cur[4], nxt[4];
+         float4 cur[MOM_ROWS], nxt[MOM_ROWS];
          load4(half, cur);
-         for (uint32_t q0 = half; q0 < n; q0 += 8) {
-            load4(q0 + 8, nxt);
+         for (uint32_t q0 = half; q0 < n; q0 += 2 * MOM_ROWS) {
+            load4(q0 + 2 * MOM_ROWS, nxt);
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-               uint32_t bi, bj, bk;
-               block_xyz(mesh, sg[wl][(q0 + 2 * u < n) ? q0 + 2 * u : 0], bi, bj, bk);
+            for (int u = 0; u < MOM_ROWS; ++u) {
+               const uint32_t at = sg[wl][(q0 + 2 * u < n) ? q0 + 2 * u : 0];
                // the row's sums of f, i f and i^2 f (i = 0..3 along x)
                const double d0 = cur[u].x, d1 = cur[u].y, d2 = cur[u].z, d3 = cur[u].w;
                const double s0 = (d0 + d1) + (d2 + d3);
                const double s1 = fma(3.0, d3, fma(2.0, d2, d1));
                const double s2 = fma(9.0, d3, fma(4.0, d2, d1));
-               const double x0 = (vmin0 + bi * bs0) + ox;
-               const double uy = (vmin1 + bj * bs1) + oy;
-               const double uz = (vmin2 + bk * bs2) + oz;
+               const double x0 = s_corner[0][at & 0xffu] + ox;
+               const double uy = s_corner[1][(at >> 8) & 0xffu] + oy;
+               const double uz = s_corner[2][at >> 16] + oz;
                const double ds1 = dv0 * s1;
                const double sfx = fma(x0, s0, ds1);  // sum f x over the row
                t[0] += s0;
@@ -178,7 +194,7 @@ __global__ void __launch_bounds__(MOM_THREADS, 2) moments_parts_kernel(
                }
             }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) cur[u] = nxt[u];
+            for (int u = 0; u < MOM_ROWS; ++u) cur[u] = nxt[u];
          }
          __syncwarp();
       }
@@ -189,6 +205,7 @@ __global__ void __launch_bounds__(MOM_THREADS, 2) moments_parts_kernel(
       double* ps = part_sums + ((size_t)cell * MOM_PARTS_PER_CELL + part) * MOM_SUMS_PER_PART;
       if (lane < NS) {
          double v = 0.0;
+#pragma unroll 8
          for (int l = 0; l < 32; ++l) v += sh[wl][lane][l];
          ps[lane] = v;
       }
