@@ -18,7 +18,7 @@
 // data in the current pool (or none for an added block): no VDF value is
 // copied, the next sweep reads the kept blocks where they are.
 // adjust_values_kernel then reads the old blocks' values once, in parts of
-// about 128 blocks over all SMs: RHOLOSSADJUST and the "_V" moments.
+// 64 or 128 blocks over all SMs: RHOLOSSADJUST and the "_V" moments.
 //
 // On a grid, content_mask_kernel first writes every cell's content mask once
 // (its content bounding box and the x-mask rows over it, in a pool), so that
@@ -42,15 +42,22 @@ constexpr int ADJ_MID_THREADS = 512;
 constexpr int ADJ_ROWS = 2;           // rows a lane has in flight, and as many on their way
 constexpr int ADJ_VALUE_CTAS = 3;         // CTAs per SM of the pass over the values
 constexpr int ADJ_UNROLL = 4;          // list entries per thread in flight
-constexpr uint32_t ADJ_TILE = 128;     // old blocks of a part staged at a time
+constexpr uint32_t ADJ_TILE = 128;     // old blocks of a part, at most
 constexpr uint32_t ADJ_KEPT = 0x80000000u;  // staged positions: the block stays
 constexpr uint32_t NO_BLOCK = 0xffffffffu;
 
-// Parts of the pass over the values of a cell with `count` old blocks: about
-// ADJ_TILE blocks each, at most MOM_PARTS_PER_CELL.
-__host__ __device__ __forceinline__ uint32_t value_parts(uint32_t count) {
-   const uint32_t p = (count + ADJ_TILE - 1) / ADJ_TILE;
-   return p < (uint32_t)MOM_PARTS_PER_CELL ? p : (uint32_t)MOM_PARTS_PER_CELL;
+// Parts of the pass over the values of a cell with `count` old blocks: of 64
+// blocks up to 1024 blocks, of 128 above (by the cell alone, so that its sums
+// do not depend on the batch).  A part is a chain of about 0.8 us per four
+// blocks, so small parts make small cells fast: six steps of
+// a cell of 412 blocks 739 -> 686 us, of 13 cells of 12000 blocks (64 parts
+// each before) 2828 -> 2724 us.
+// Parts of 64 blocks for every cell make 4096 cells of 1423 blocks 5% slower
+// (29.2 -> 30.7 ms: a part's own loads and sums), parts of 32 blocks make a
+// cell of 412 blocks no faster (680 against 686 us).
+__device__ __forceinline__ uint32_t value_parts(uint32_t count) {
+   const uint32_t size = count <= 1024 ? ADJ_ITEM_BLOCKS : ADJ_TILE;
+   return (count + size - 1) / size;
 }
 
 __device__ __forceinline__ uint32_t adj_exclusive_scan(uint32_t v, uint32_t* warp_sums, uint32_t& total) {
@@ -538,7 +545,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) adjust_kernel(
       if (!ok) atomicOr(&counters->overflow, 1u);
    }
    __syncthreads();
-   for (uint32_t p = threadIdx.x; p < parts; p += THREADS) items[s_part + p] = AdjustItem{cell, p};
+   for (uint32_t p = threadIdx.x; p < parts; p += THREADS) items[s_part + p] = AdjustItem{cell, p, s_part};
    if (parts == 0 && mom_record && threadIdx.x < MOM_COUNT) {
       mom_record[(size_t)cell * MOM_COUNT + threadIdx.x] = 0.0;
       if (write_pivot) pivot[(size_t)cell * MOM_COUNT + threadIdx.x] = 0.0;
@@ -689,11 +696,16 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_VALUE_CTAS) adjust_values_ker
 #pragma unroll
       for (int q = 0; q < NS; ++q) s_sum[warp][q][lane] = t[q];
       __syncwarp();
-      double* ps = part_sums + ((size_t)cell * MOM_PARTS_PER_CELL + item.part) * MOM_SUMS_PER_PART;
-      if (lane < NS) {
+      double* ps = part_sums + ((size_t)item.first + item.part) * ADJ_SUMS;
+      {
+         // (sub < NS: half-warp h adds lanes 16 h .. 16 h + 15)
          double v = 0.0;
-         for (int l = 0; l < 32; ++l) v += s_sum[warp][lane][l];
-         ps[lane] = v;
+         if (sub < NS) {
+#pragma unroll
+            for (int l = 0; l < 16; ++l) v += s_sum[warp][sub][16 * half + l];
+         }
+         v += __shfl_xor_sync(FULL, v, 16);
+         if (lane < NS) ps[lane] = v;
       }
       __syncwarp();
       __threadfence();
@@ -706,9 +718,10 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_VALUE_CTAS) adjust_values_ker
       double S = 0.0;
       if (lane < NS) {
          double sum = 0.0, comp = 0.0;
-         const double* base = part_sums + (size_t)cell * MOM_PARTS_PER_CELL * MOM_SUMS_PER_PART + lane;
+         const double* base = part_sums + (size_t)item.first * ADJ_SUMS + lane;
+#pragma unroll 8
          for (uint32_t p = 0; p < parts; ++p) {
-            const double y = __ldcg(base + (size_t)p * MOM_SUMS_PER_PART) - comp;
+            const double y = __ldcg(base + (size_t)p * ADJ_SUMS) - comp;
             const double tt = sum + y;
             comp = (tt - sum) - y;
             sum = tt;
@@ -745,8 +758,8 @@ int adjust_blocks_per_sm() {
    return n > 0 ? n : 1;
 }
 
-// `kept`: a byte per row of the old list; `items`: at most one per ADJ_TILE
-// old blocks and one per cell.  The caller lends the sweeps' work arrays.
+// `kept`: a byte per row of the old list (lent from the sweeps' work arrays);
+// `items` and `part_sums`: an entry per ADJ_ITEM_BLOCKS old blocks and per cell.
 cudaError_t launch_adjust(const uint32_t* gids, const uint32_t* src_index, const CellSlot* slots,
                           uint8_t* content, bool content_valid, const uint32_t* rows_used, const float* data,
                           const int32_t* neighbors,

@@ -209,6 +209,7 @@ struct vlgpu_batch {
    uint32_t mask_cap = 0;
    int adj_grid = 0;
    AdjustItem* adj_items = nullptr;  // the parts of the adjustment's pass over the values
+   double* adj_sums = nullptr;       // and their sums
    int adj_value_grid = 0;  // CTAs of the adjustment's pass over the values
    int col_wide_grid = 0;  // CTAs of the wide-plane columnize
    double* moments_r = nullptr;   // MOM_COUNT per cell: the moments after translation (the "_R" set)

@@ -50,6 +50,7 @@ void free_batch(vlgpu_batch* b) {
    cudaFree(b->dt_buf);
    cudaFree(b->adj_scratch);
    cudaFree(b->adj_items);
+   cudaFree(b->adj_sums);
    cudaFree(b->wide_cells);
    cudaFree(b->halo_scratch);
    cudaFree(b->cell_order);
@@ -185,7 +186,7 @@ int adjust_device(vlgpu_batch* b, double* record, bool write_pivot) {
                           (int)b->params.add_width_v, dv3, b->n_cells, b->adj_scratch, b->adj_grid,
                           b->cell_order, b->mask_recs, b->mask_pool, b->mask_top, b->mask_cap,
                           reinterpret_cast<uint8_t*>(b->perm), b->adj_items,
-                          b->mom_parts, b->mom_done, b->adj_value_grid, (uint32_t)b->sm_count, record, b->pivot,
+                          b->adj_sums, b->mom_done, b->adj_value_grid, (uint32_t)b->sm_count, record, b->pivot,
                           write_pivot ? 1 : 0, frame, after, b->stream));
    // content flags first unless a sweep left them, content masks on a grid
    b->launches += 2 + (b->content_valid ? 0 : 1) + (b->neighbors && b->mask_recs ? 1 : 0);
@@ -420,9 +421,10 @@ int vlgpu_batch_create(const vlgpu_mesh* mesh, const vlgpu_params* params, uint3
                                             (size_t)std::min<uint32_t>((uint32_t)b->adj_grid, n_cells))) !=
        cudaSuccess)
       return fail(e, "adjust scratch");
-   // a part per 128 old blocks and one per cell, at most
-   if ((e = cudaMalloc(&b->adj_items, sizeof(AdjustItem) * (cap / 128 + n_cells))) != cudaSuccess)
-      return fail(e, "adjust items");
+   // a part per ADJ_ITEM_BLOCKS old blocks and one per cell, at most
+   const uint64_t items = cap / ADJ_ITEM_BLOCKS + n_cells;
+   if ((e = cudaMalloc(&b->adj_items, sizeof(AdjustItem) * items)) != cudaSuccess) return fail(e, "adjust items");
+   if ((e = cudaMalloc(&b->adj_sums, sizeof(double) * ADJ_SUMS * items)) != cudaSuccess) return fail(e, "adjust sums");
    if ((e = cudaMalloc(&b->wide_cells, sizeof(uint32_t) * n_cells)) != cudaSuccess) return fail(e, "wide");
    if ((e = cudaMalloc(&b->cell_order, sizeof(uint32_t) * n_cells)) != cudaSuccess) return fail(e, "order");
    if ((e = cudaMallocHost(&b->h_order, sizeof(uint32_t) * n_cells)) != cudaSuccess) return fail(e, "order");

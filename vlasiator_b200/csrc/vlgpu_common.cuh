@@ -16,7 +16,7 @@ constexpr int MAX_PLANE = 96 * 96;  // transverse plane entries
 // The moments split a cell's blocks into at most this many parts, each
 // summed by one warp into MOM_SUMS_PER_PART doubles of a work array.
 constexpr int MOM_PARTS_PER_CELL = 64;
-constexpr int MOM_SUMS_PER_PART = 11;  // the adjustment's parts add the removed mass
+constexpr int MOM_SUMS_PER_PART = 10;
 
 // Per-cell state of one batch, indexed by cell.
 struct CellSlot {
@@ -152,7 +152,10 @@ __device__ __forceinline__ void hand_over(const HandOver& h, const SweepCounters
 // One part of the adjustment's pass over a cell's values.
 struct AdjustItem {
    uint32_t cell, part;
+   uint32_t first;  // the item of the cell's part 0
 };
+constexpr uint32_t ADJ_ITEM_BLOCKS = 64;  // old blocks of a part, at least (but for the last of a cell)
+constexpr int ADJ_SUMS = 11;              // a part's sums: the removed mass and the moments'
 
 // Running totals kept on the device across sweeps (never reset by a sweep).
 struct BatchStats {
