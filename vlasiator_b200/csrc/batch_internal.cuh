@@ -119,6 +119,7 @@ cudaError_t launch_trans_remap(int dim, uint32_t N, const uint32_t* item_gid, co
 int trans_blocks_per_sm(uint32_t N, bool exact);
 uint32_t union_words(const MeshDev& mesh);
 constexpr int MOM_COUNT = 16;
+size_t pack_scratch_words(uint64_t capacity, uint32_t n_cells, int sm_count);
 constexpr double MU_0 = 1.25663706e-6;  // physicalconstants::MU_0 (common.h:561)
 }  // namespace vlgpu
 
@@ -201,7 +202,7 @@ struct vlgpu_batch {
    uint32_t* wide_cells = nullptr;  // the cells whose columnize plane is too wide for the capped kernel
    uint32_t* cell_order = nullptr;  // the cells by decreasing block count at the last upload (persistent kernels)
    uint32_t* h_order = nullptr;     // pinned staging of cell_order
-   uint32_t* halo_scratch = nullptr;  // cell descriptors of a pack / unpack of some cells (grown on demand)
+   uint32_t* halo_scratch = nullptr;  // chunk list of a pack, ID check of an unpack
    size_t halo_words = 0;
    vlgpu::MaskRec* mask_recs = nullptr;  // grid: per cell, its content mask record
    uint32_t* mask_pool = nullptr;        // grid: the content mask rows

@@ -425,6 +425,8 @@ int vlgpu_batch_create(const vlgpu_mesh* mesh, const vlgpu_params* params, uint3
    const uint64_t items = cap / ADJ_ITEM_BLOCKS + n_cells;
    if ((e = cudaMalloc(&b->adj_items, sizeof(AdjustItem) * items)) != cudaSuccess) return fail(e, "adjust items");
    if ((e = cudaMalloc(&b->adj_sums, sizeof(double) * ADJ_SUMS * items)) != cudaSuccess) return fail(e, "adjust sums");
+   b->halo_words = pack_scratch_words(cap, n_cells, b->sm_count);
+   if ((e = cudaMalloc(&b->halo_scratch, sizeof(uint32_t) * b->halo_words)) != cudaSuccess) return fail(e, "pack scratch");
    if ((e = cudaMalloc(&b->wide_cells, sizeof(uint32_t) * n_cells)) != cudaSuccess) return fail(e, "wide");
    if ((e = cudaMalloc(&b->cell_order, sizeof(uint32_t) * n_cells)) != cudaSuccess) return fail(e, "order");
    if ((e = cudaMallocHost(&b->h_order, sizeof(uint32_t) * n_cells)) != cudaSuccess) return fail(e, "order");

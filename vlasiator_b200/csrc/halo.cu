@@ -58,6 +58,12 @@ __global__ void check_gids_range_kernel(const uint32_t* __restrict__ gids, uint6
       if (gids[i] >= max_gid) *bad = 1u;
 }
 
+// Words of the chunk list of any selection that names a cell once: at most a
+// partial chunk per cell, and 16 full ones per SM or one per PACK_CHUNK blocks.
+size_t pack_scratch_words(uint64_t capacity, uint32_t n_cells, int sm_count) {
+   return 3 * ((size_t)n_cells + 16 * (size_t)sm_count + capacity / PACK_CHUNK);
+}
+
 }  // namespace vlgpu
 
 using namespace vlgpu;
@@ -78,13 +84,14 @@ int direct_state_slots(vlgpu_batch* b, std::vector<CellSlot>& slots, uint32_t ro
    return VLGPU_OK;
 }
 
-// Room for n uint32 words of the per-batch exchange scratch.
+// Room for n uint32 words of the per-batch exchange scratch (more than the
+// batch was made with only where cells are named several times).
 int halo_scratch(vlgpu_batch* b, size_t n) {
    if (n <= b->halo_words) return VLGPU_OK;
+   uint32_t* more = nullptr;
+   VL_CHECK(cudaMalloc(&more, sizeof(uint32_t) * n));
    cudaFree(b->halo_scratch);
-   b->halo_scratch = nullptr;
-   b->halo_words = 0;
-   VL_CHECK(cudaMalloc(&b->halo_scratch, sizeof(uint32_t) * n));
+   b->halo_scratch = more;
    b->halo_words = n;
    return VLGPU_OK;
 }
@@ -110,8 +117,6 @@ int unpack_all(vlgpu_batch* b, uint32_t n_sel, const uint32_t* cells, const uint
                const float* data, uint64_t total) {
    if (total > b->capacity) return VLGPU_ENOMEM;
    const int pool = 1 - b->cur;
-   const int st = halo_scratch(b, 1);
-   if (st != VLGPU_OK) return st;
    uint32_t bad = 0, used = 0;
    std::vector<CellSlot> slots(b->n_cells);
    uint32_t o = 0;
@@ -212,8 +217,6 @@ int vlgpu_batch_unpack_cells(vlgpu_batch* b, uint32_t n_sel, const uint32_t* cel
    if (L + total > b->capacity) return VLGPU_ENOMEM;
    if (total > 0) {
       // the blocks' IDs must lie on the batch's mesh
-      st = halo_scratch(b, 1);
-      if (st != VLGPU_OK) return st;
       VL_CHECK(cudaMemsetAsync(b->halo_scratch, 0, sizeof(uint32_t), b->stream));
       const uint32_t max_gid = b->mesh.len[0] * b->mesh.len[1] * b->mesh.len[2];
       check_gids_range_kernel<<<b->sm_count * 2, 256, 0, b->stream>>>(gids, total, max_gid, b->halo_scratch);
