@@ -107,7 +107,7 @@ int sweep_device(vlgpu_batch* b, const SweepCell* sweep_cells, uint32_t dim, boo
          VL_CHECK(cudaEventRecord(b->prof_events[b->prof_used + 1], b->stream));
          b->prof_used += 2;
       }
-      b->launches += 3;
+      b->launches += b->n_cells <= (uint32_t)b->sm_count ? 2 : 3;  // (no wide launch for few cells)
       b->remap_launches += 1;
    } else {
       // one columnize + remap launch pair per cell; set and output counters
