@@ -446,7 +446,7 @@ def run_ours(args):
                        "what": "device time of one batched acceleration step of all cells"},
         "plain_per_cell": plain,
         "status_cells_flagged": int((status != 0).sum()),
-        "roofline": {"bound": "hbm", "kernel": "remap_kernel" if args.exact else "remap_walk_kernel", "achieved": achieved, "peak": peak,
+        "roofline": {"bound": "hbm", "kernel": "remap_kernel" if args.exact else "remap_pair_kernel", "achieved": achieved, "peak": peak,
                      "peak_kind": peak_kind, "unit": "GB/s",
                      "frac": (achieved / peak) if achieved else None,
                      "traffic": (REMAP_DRAM_BYTES_PER_BLOCK * src_blocks / remap_n) if remap_n else None,

@@ -562,9 +562,12 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) adjust_kernel(
 // staged list in flight.  The last part of a cell to finish adds the parts in
 // part order, so the result does not depend on which warp took which part.
 //
-// Bound by the FP64 and conversion pipes and the latency of a part's first
-// rows: 166 us for 1024 drifting cells (1.45 M blocks) in the first form, two
-// CTAs per SM with eight rows of a lane in flight.
+// Bound by latency: of a part of 128 blocks' 48 us in a full launch, about 16
+// go into its chain of loads (item, slot, lists, first rows) and its hand-in
+// (sums, fence, counter); the FP64 pipe is 33% busy, HBM at 32%.  102 us for 512
+// drifting cells after three sweeps, where one CTA per cell for lists and
+// values took 301.  Corners staged per block, no branches and the loop
+// unrolled (half the instructions) made a step of 4096 cells 1.5% slower.
 template <bool FUSE>
 __global__ void __launch_bounds__(ADJ_THREADS, ADJ_VALUE_CTAS) adjust_values_kernel(
    const uint32_t* __restrict__ gids, const uint32_t* __restrict__ src_index, const CellSlot* __restrict__ slots,

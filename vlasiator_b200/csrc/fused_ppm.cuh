@@ -36,7 +36,11 @@ __device__ __forceinline__ float h7_derivative(float w0, float w1, float w2, flo
 // the Bernstein coefficients fd_l, fd_l + b0/3, fd_l + 2 b0/3 + b1/6, fd_r on
 // the cell; where none opposes the cell's slope, neither does the slope at an
 // inflexion point, and the roots (a square root and two quotients) are not
-// needed.
+// needed.  Where they are, approximate ones do: only the slope's sign there is
+// read.  The error against 64-bit sweeps is the same with rounded ones (9.4e-6 of
+// the peak here and 9.5e-6 with all divisions rounded), which take 792 us
+// instead of 749 for three sweeps of 256 cells with packing (1675 in the
+// form with v0 in every product and all roots).
 __device__ __forceinline__ float sqrt_approx(float x) {
    float r;
    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
