@@ -29,6 +29,7 @@
 #include <cfloat>
 #include <cmath>
 #include <cstdint>
+#include <type_traits>
 
 #include "fused_ppm.cuh"
 #include "vlgpu_common.cuh"
@@ -1104,6 +1105,11 @@ __global__ void __launch_bounds__(REMAP_THREADS, 3) remap_walk_kernel(
 //  - The ring of target cells lies slot by slot in shared memory (a slot of
 //    all the CTA's lanes is contiguous): a lane's slot is always in its own
 //    banks, whatever slots the other lanes are at.
+//  - The pending target's slot is written for every cell, complete or not,
+//    which saves the test.  That needs the slot to be the target's own: the
+//    pending target may not be a whole ring ahead of the oldest one that is
+//    still to be flushed.  Where the columns of a block face start far apart
+//    it can be, and those sets (PAIR_LEAN) write a target when it is complete.
 //
 // Bound by issue and the ALU pipe (72% and 60% busy with 24 warps per SM, the
 // most the ring's 64 KB per CTA leave room for).  Measured on 4096 drifting
@@ -1118,6 +1124,19 @@ constexpr uint32_t PAIR_SLOT_BYTES = PAIR_THREADS * sizeof(float2);  // one ring
 constexpr uint32_t PAIR_SLOT_MASK = (RING_CELLS - 1) * PAIR_SLOT_BYTES;
 constexpr int PAIR_CTAS = 3;  // per SM: 72 to 80 registers, 192 KB of rings
 constexpr size_t PAIR_SMEM = (size_t)RING_CELLS * PAIR_SLOT_BYTES;
+// The columns of a set start within S = 3 (|di| + |dj|) / dk target cells of
+// one another.  At the end of a block every target cell below the lowest
+// pending one's block is flushed, so during the next the highest pending
+// target is less than 3 + (S + 1) + (4 dv / dk + 1) cells above the oldest one
+// in the ring; where flushing waits for the set's next column, whose lowest
+// target block may lie below the highest one of this, less than 3 + 3 + 3 + S.
+// With S + 4 dv / dk <= 20 both are less than the ring's 32, with room for the
+// rounding of the edges.  (A step that turns by 22 degrees has 6.)
+constexpr float PAIR_LEAN = 20.0f;
+// Target cells of a column's start beyond which nothing can be right any more
+// (the mesh has 384): a start above is reported, one below counts as the
+// column's lowest target, and the slot's offset stays far from its 32 bits.
+constexpr float PAIR_FAR = 1e6f;
 
 // The lane's two columns of the block at `row` (data: the lane's first cell of
 // row 0): cells g = 0..3 along the sweep, .x and .y the two columns.
@@ -1245,6 +1264,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, PAIR_CTAS) remap_pair_kernel(
       constexpr int NO_COLUMN = 1 << 20;
       int left = 0, hi = 0, ncf = NO_COLUMN;
       int kb = 0, lo = 0;  // first block and lowest target cell of the column about to start
+      bool lean = false;   // see PAIR_LEAN
       if (sidx < n_sets) {
          const ColumnSet cs = sets[sidx];
          const SweepCell P = sweep_cells[cs.cell];
@@ -1266,6 +1286,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, PAIR_CTAS) remap_pair_kernel(
             // a cell whose Lagrangian cells do not advance (flagged by
             // columnize) gets its target blocks with zero values
             if (dk > 0.0f) n_src = __popc(cs.src_mask[0]) + __popc(cs.src_mask[1]) + __popc(cs.src_mask[2]);
+            lean = !(fmaf(3.0f, fabsf(P.di) + fabsf(P.dj), 4.0f * mesh.dv) <= PAIR_LEAN * dk);
             if (n_src > 0) {
                kb = mask_first(cs.src_mask);
                const int e = mask_run_end(cs.src_mask, kb);
@@ -1290,6 +1311,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, PAIR_CTAS) remap_pair_kernel(
       }
       __syncwarp();
       const int iters = __reduce_max_sync(FULL, n_src);
+      const bool any_lean = __any_sync(FULL, lean);  // the warp's sets walk in step
       bool range_err = false;
 
       // writes out the target blocks below `limit` that all the lanes of the
@@ -1341,10 +1363,11 @@ __global__ void __launch_bounds__(PAIR_THREADS, PAIR_CTAS) remap_pair_kernel(
       // the state at the start of the column whose first block is c
       auto start = [&](const float2 c[4]) {
          v_l = fa(fm((float)(WID * kb), mesh.dv), mesh.v_min);
-         // each lane's first target: the lowest g with (g+1) dk + im > v_l,
-         // from an approximate quotient
+         // each lane's first target: the lowest g with (g+1) dk + im > v_l
          auto first_target = [&](float imc, float& gf, float& uc, uint32_t& so) {
-            int g = __float2int_rz(__fdividef(fs(v_l, imc), dk));
+            const float q0 = fd(fs(v_l, imc), dk);
+            range_err |= q0 > PAIR_FAR;
+            int g = __float2int_rz(fminf(fmaxf(q0, -PAIR_FAR), PAIR_FAR));
             float e = fa(fm((float)(g + 1), dk), imc);
 #pragma unroll 1
             for (int q = 0; q < 3 && e <= v_l; ++q) {
@@ -1368,17 +1391,19 @@ __global__ void __launch_bounds__(PAIR_THREADS, PAIR_CTAS) remap_pair_kernel(
          };
          first_target(im.x, g2f.x, u.x, sox);
          first_target(im.y, g2f.y, u.y, soy);
-         // what another column left in the slots
-         nacc.x = -slot_x(sox);
-         nacc.y = -slot_y(soy);
+         // what another column left in the slots; a target above the ring's
+         // window has none yet, its slot is an older target's
+         const uint32_t end = (uint32_t)(next_flush + RING_BLOCKS) * (WID * PAIR_SLOT_BYTES);
+         nacc.x = sox < end ? -slot_x(sox) : 0.0f;
+         nacc.y = soy < end ? -slot_y(soy) : 0.0f;
          // zero padding below the column
          vm1 = zero2;
          if constexpr (RECON == RECON_PPM) ppm.start(zero2, zero2, c[0], c[1]);
          else ppm.b = c[0];
       };
 
-      // one cell: v0 with its upper neighbours
-      auto cell_step = [&](const float2 v0, const float2 vp1, const float2 vp2) {
+      // one cell: v0 with its upper neighbours; `complete_only`: see PAIR_LEAN
+      auto cell_step = [&](auto complete_only, const float2 v0, const float2 vp1, const float2 vp2) {
          // ---- reconstruction ----
          float2 s, l, r;
          if constexpr (RECON == RECON_PPM) {
@@ -1399,8 +1424,8 @@ __global__ void __launch_bounds__(PAIR_THREADS, PAIR_CTAS) remap_pair_kernel(
          const float2 D = __fmul2_rn(u, __ffma2_rn(__fmul2_rn(s, um), T, v0));
          // without an edge the slot is written again when its target is complete
          const float2 val = p_minus(D, nacc);
-         slot_x(sox) = val.x;
-         slot_y(soy) = val.y;
+         if (!decltype(complete_only)::value || hx) slot_x(sox) = val.x;
+         if (!decltype(complete_only)::value || hy) slot_y(soy) = val.y;
          nacc = p_minus(make_float2(hx ? D.x : nacc.x, hy ? D.y : nacc.y), v0);
          // the next edge, with the reference's roundings (the packed multiply
          // and add get contracted, so these are scalar)
@@ -1457,10 +1482,21 @@ __global__ void __launch_bounds__(PAIR_THREADS, PAIR_CTAS) remap_pair_kernel(
          if (active) {
             // zero padding above the column
             const float2 n0 = last ? zero2 : n[0], n1 = last ? zero2 : n[1];
-            cell_step(w[0], w[1], w[2]);
-            cell_step(w[1], w[2], w[3]);
-            cell_step(w[2], w[3], n0);
-            cell_step(w[3], n0, n1);
+            if (__builtin_expect(any_lean, 0)) {
+               // (a loop: a second unrolled copy would only lengthen the kernel)
+               float2 v[6] = {w[0], w[1], w[2], w[3], n0, n1};
+#pragma unroll 1
+               for (int q = 0; q < 4; ++q) {
+                  cell_step(std::true_type{}, v[0], v[1], v[2]);
+#pragma unroll
+                  for (int k = 0; k < 5; ++k) v[k] = v[k + 1];
+               }
+            } else {
+               cell_step(std::false_type{}, w[0], w[1], w[2]);
+               cell_step(std::false_type{}, w[1], w[2], w[3]);
+               cell_step(std::false_type{}, w[2], w[3], n0);
+               cell_step(std::false_type{}, w[3], n0, n1);
+            }
          }
          int limit = NO_COLUMN;  // target blocks below it are complete in this lane's columns
          if (active) {
@@ -1478,7 +1514,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, PAIR_CTAS) remap_pair_kernel(
                         slot((uint32_t)t * PAIR_SLOT_BYTES) = 0.0f;
                      }
                      range_err |= g > hi + RING_CELLS / 2;
-                     slot(so) = 0.0f;  // what was written there while it was pending
+                     if (!any_lean) slot(so) = 0.0f;  // what was written there while it was pending
                      slot((uint32_t)hi * PAIR_SLOT_BYTES) += rest;
                      return hi;
                   }
@@ -1486,7 +1522,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, PAIR_CTAS) remap_pair_kernel(
                   return g;
                };
                const int tx = close(gx, sox, -nacc.x, slot_x), ty = close(gy, soy, -nacc.y, slot_y);
-               top = max(tx, ty);
+               top = max(top, max(tx, ty));
                limit = ncf;
             }
             // everything this block wrote must lie inside the ring's window
