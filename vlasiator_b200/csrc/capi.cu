@@ -363,6 +363,8 @@ int vlgpu_batch_create(const vlgpu_mesh* mesh, const vlgpu_params* params, uint3
       free_batch(b);
       return s;
    };
+   // (on the batch's stream, which does not wait for the default one)
+   auto zeroed = [&](void* p, size_t bytes) { return cudaMemsetAsync(p, 0, bytes, b->stream); };
    cudaError_t e = cudaSetDevice(device);
    if (e != cudaSuccess) return fail(e, "cudaSetDevice");
    if ((e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking)) != cudaSuccess) return fail(e, "stream");
@@ -382,9 +384,9 @@ int vlgpu_batch_create(const vlgpu_mesh* mesh, const vlgpu_params* params, uint3
    for (int p = 0; p < 2; ++p) {
       if ((e = cudaMalloc(&b->gids[p], sizeof(uint32_t) * cap)) != cudaSuccess) return fail(e, "gids");
       if ((e = cudaMalloc(&b->data[p], sizeof(float) * WID3 * (cap + 1))) != cudaSuccess) return fail(e, "data");
-      if ((e = cudaMemset(b->data[p] + WID3 * cap, 0, sizeof(float) * WID3)) != cudaSuccess) return fail(e, "data");
+      if ((e = zeroed(b->data[p] + WID3 * cap, sizeof(float) * WID3)) != cudaSuccess) return fail(e, "data");
       if ((e = cudaMalloc(&b->slots[p], sizeof(CellSlot) * n_cells)) != cudaSuccess) return fail(e, "slots");
-      if ((e = cudaMemset(b->slots[p], 0, sizeof(CellSlot) * n_cells)) != cudaSuccess) return fail(e, "slots");
+      if ((e = zeroed(b->slots[p], sizeof(CellSlot) * n_cells)) != cudaSuccess) return fail(e, "slots");
       if ((e = cudaMalloc(&b->adj_gids[p], sizeof(uint32_t) * cap)) != cudaSuccess) return fail(e, "adj");
       if ((e = cudaMalloc(&b->adj_src[p], sizeof(uint32_t) * cap)) != cudaSuccess) return fail(e, "adj");
       if ((e = cudaMalloc(&b->adj_slots[p], sizeof(CellSlot) * n_cells)) != cudaSuccess) return fail(e, "adj");
@@ -395,26 +397,26 @@ int vlgpu_batch_create(const vlgpu_mesh* mesh, const vlgpu_params* params, uint3
    if ((e = cudaMalloc(&b->sweep_cells, sizeof(SweepCell) * n_cells)) != cudaSuccess) return fail(e, "sweep");
    if ((e = cudaMalloc(&b->sweep3, sizeof(SweepCell) * 3 * n_cells)) != cudaSuccess) return fail(e, "sweep3");
    if ((e = cudaMalloc(&b->accel_in, sizeof(CellAccelInputs) * n_cells)) != cudaSuccess) return fail(e, "accel");
-   if ((e = cudaMemset(b->accel_in, 0, sizeof(CellAccelInputs) * n_cells)) != cudaSuccess) return fail(e, "accel");
+   if ((e = zeroed(b->accel_in, sizeof(CellAccelInputs) * n_cells)) != cudaSuccess) return fail(e, "accel");
    if ((e = cudaMalloc(&b->moments, sizeof(double) * MOM_COUNT * n_cells)) != cudaSuccess) return fail(e, "mom");
-   if ((e = cudaMemset(b->moments, 0, sizeof(double) * MOM_COUNT * n_cells)) != cudaSuccess) return fail(e, "mom");
+   if ((e = zeroed(b->moments, sizeof(double) * MOM_COUNT * n_cells)) != cudaSuccess) return fail(e, "mom");
    if ((e = cudaMalloc(&b->pivot, sizeof(double) * MOM_COUNT * n_cells)) != cudaSuccess) return fail(e, "mom");
    if ((e = cudaMalloc(&b->mom_scratch, sizeof(double) * MOM_COUNT * n_cells)) != cudaSuccess) return fail(e, "mom");
-   if ((e = cudaMemset(b->pivot, 0, sizeof(double) * MOM_COUNT * n_cells)) != cudaSuccess) return fail(e, "mom");
+   if ((e = zeroed(b->pivot, sizeof(double) * MOM_COUNT * n_cells)) != cudaSuccess) return fail(e, "mom");
    if ((e = cudaMalloc(&b->mom_parts, sizeof(double) * MOM_SUMS_PER_PART * MOM_PARTS_PER_CELL * n_cells)) !=
        cudaSuccess)
       return fail(e, "mom");
    if ((e = cudaMalloc(&b->mom_done, sizeof(uint32_t) * n_cells)) != cudaSuccess) return fail(e, "mom");
-   if ((e = cudaMemset(b->mom_done, 0, sizeof(uint32_t) * n_cells)) != cudaSuccess) return fail(e, "mom");
+   if ((e = zeroed(b->mom_done, sizeof(uint32_t) * n_cells)) != cudaSuccess) return fail(e, "mom");
    if ((e = cudaMalloc(&b->isect12, sizeof(double) * 12 * n_cells)) != cudaSuccess) return fail(e, "isect");
-   if ((e = cudaMemset(b->isect12, 0, sizeof(double) * 12 * n_cells)) != cudaSuccess) return fail(e, "isect");
+   if ((e = zeroed(b->isect12, sizeof(double) * 12 * n_cells)) != cudaSuccess) return fail(e, "isect");
    if ((e = cudaMalloc(&b->loss, sizeof(double) * n_cells)) != cudaSuccess) return fail(e, "loss");
-   if ((e = cudaMemset(b->loss, 0, sizeof(double) * n_cells)) != cudaSuccess) return fail(e, "loss");
+   if ((e = zeroed(b->loss, sizeof(double) * n_cells)) != cudaSuccess) return fail(e, "loss");
    if ((e = cudaMalloc(&b->status, sizeof(uint32_t) * n_cells)) != cudaSuccess) return fail(e, "status");
-   if ((e = cudaMemset(b->status, 0, sizeof(uint32_t) * n_cells)) != cudaSuccess) return fail(e, "status");
+   if ((e = zeroed(b->status, sizeof(uint32_t) * n_cells)) != cudaSuccess) return fail(e, "status");
    if ((e = cudaMalloc(&b->counters, 2 * sizeof(SweepCounters))) != cudaSuccess) return fail(e, "counters");
    // no sweep has run: vlgpu_batch_sync reads the overflow flag from here
-   if ((e = cudaMemset(b->counters, 0, 2 * sizeof(SweepCounters))) != cudaSuccess) return fail(e, "counters");
+   if ((e = zeroed(b->counters, 2 * sizeof(SweepCounters))) != cudaSuccess) return fail(e, "counters");
    if ((e = cudaMalloc(&b->stats, sizeof(BatchStats))) != cudaSuccess) return fail(e, "stats");
    if ((e = cudaMalloc(&b->rows_used, sizeof(uint32_t) * 4)) != cudaSuccess) return fail(e, "rows");
    if ((e = cudaMalloc(&b->adj_scratch, sizeof(uint32_t) * adjust_scratch_words(b->mdev) *
@@ -431,11 +433,11 @@ int vlgpu_batch_create(const vlgpu_mesh* mesh, const vlgpu_params* params, uint3
    if ((e = cudaMalloc(&b->cell_order, sizeof(uint32_t) * n_cells)) != cudaSuccess) return fail(e, "order");
    if ((e = cudaMallocHost(&b->h_order, sizeof(uint32_t) * n_cells)) != cudaSuccess) return fail(e, "order");
    for (uint32_t c = 0; c < n_cells; ++c) b->h_order[c] = c;
-   if ((e = cudaMemcpy(b->cell_order, b->h_order, sizeof(uint32_t) * n_cells, cudaMemcpyHostToDevice)) !=
-       cudaSuccess)
+   if ((e = cudaMemcpyAsync(b->cell_order, b->h_order, sizeof(uint32_t) * n_cells, cudaMemcpyHostToDevice,
+                            b->stream)) != cudaSuccess)
       return fail(e, "order");
-   if ((e = cudaMemset(b->rows_used, 0, sizeof(uint32_t) * 4)) != cudaSuccess) return fail(e, "rows");
-   if ((e = cudaMemset(b->stats, 0, sizeof(BatchStats))) != cudaSuccess) return fail(e, "stats");
+   if ((e = zeroed(b->rows_used, sizeof(uint32_t) * 4)) != cudaSuccess) return fail(e, "rows");
+   if ((e = zeroed(b->stats, sizeof(BatchStats))) != cudaSuccess) return fail(e, "stats");
    if ((e = cudaMallocHost(&b->h_sweep, sizeof(SweepCell) * n_cells)) != cudaSuccess) return fail(e, "pinned");
    if ((e = cudaMallocHost(&b->h_accel, sizeof(CellAccelInputs) * n_cells)) != cudaSuccess) return fail(e, "pinned");
    if ((e = cudaEventCreateWithFlags(&b->ev_sweep, cudaEventDisableTiming)) != cudaSuccess) return fail(e, "event");
@@ -447,6 +449,7 @@ int vlgpu_batch_create(const vlgpu_mesh* mesh, const vlgpu_params* params, uint3
    if ((e = cudaEventCreateWithFlags(&b->ev_upload, cudaEventDisableTiming)) != cudaSuccess) return fail(e, "event");
    if ((e = cudaEventCreateWithFlags(&b->ev_order, cudaEventDisableTiming)) != cudaSuccess) return fail(e, "event");
    if ((e = cudaEventCreateWithFlags(&b->ev_slots, cudaEventDisableTiming)) != cudaSuccess) return fail(e, "event");
+   if ((e = cudaStreamSynchronize(b->stream)) != cudaSuccess) return fail(e, "create");  // h_order has been read
    set_direct_state(b, 0);
    *out = b;
    return VLGPU_OK;
@@ -500,11 +503,9 @@ int vlgpu_batch_upload(vlgpu_batch* b, const uint64_t* offsets, const uint32_t* 
    VL_CHECK(upload_cell_order(b, offsets));
    VL_CHECK(cudaMemsetAsync(b->status, 0, sizeof(uint32_t) * b->n_cells, b->stream));
    VL_CHECK(cudaMemsetAsync(b->loss, 0, sizeof(double) * b->n_cells, b->stream));
+   const uint32_t used = (uint32_t)total;
+   VL_CHECK(cudaMemcpyAsync(b->rows_used, &used, sizeof(uint32_t), cudaMemcpyHostToDevice, b->stream));
    VL_CHECK(cudaStreamSynchronize(b->stream));
-   {
-      const uint32_t used = (uint32_t)total;
-      VL_CHECK(cudaMemcpy(b->rows_used, &used, sizeof(uint32_t), cudaMemcpyHostToDevice));
-   }
    set_direct_state(b, 0);
    b->content_valid = false;
    consult_launch_table(b, (double)total / b->n_cells);
@@ -816,7 +817,7 @@ int vlgpu_batch_set_grid(vlgpu_batch* b, const uint32_t dims[3], const double dx
       VL_CHECK(cudaMalloc(&b->mask_pool, sizeof(uint32_t) * words));
       VL_CHECK(cudaMalloc(&b->mask_top, sizeof(uint32_t)));
       VL_CHECK(cudaMalloc(&b->tcounters, 2 * sizeof(TransCounters)));
-      VL_CHECK(cudaMemset(b->tcounters, 0, 2 * sizeof(TransCounters)));
+      VL_CHECK(cudaMemsetAsync(b->tcounters, 0, 2 * sizeof(TransCounters), b->stream));
    }
    // the 26 nearest neighbours of every cell, periodic, the cell itself excluded
    std::vector<int32_t> nb((size_t)b->n_cells * 26);
@@ -838,9 +839,10 @@ int vlgpu_batch_set_grid(vlgpu_batch* b, const uint32_t dims[3], const double dx
    if (!b->dt_buf) VL_CHECK(cudaMalloc(&b->dt_buf, sizeof(double) * 2 * b->n_cells));
    if (!b->moments_r) {
       VL_CHECK(cudaMalloc(&b->moments_r, sizeof(double) * MOM_COUNT * b->n_cells));
-      VL_CHECK(cudaMemset(b->moments_r, 0, sizeof(double) * MOM_COUNT * b->n_cells));
+      VL_CHECK(cudaMemsetAsync(b->moments_r, 0, sizeof(double) * MOM_COUNT * b->n_cells, b->stream));
    }
-   VL_CHECK(cudaMemcpy(b->neighbors, nb.data(), sizeof(int32_t) * nb.size(), cudaMemcpyHostToDevice));
+   VL_CHECK(cudaMemcpyAsync(b->neighbors, nb.data(), sizeof(int32_t) * nb.size(), cudaMemcpyHostToDevice, b->stream));
+   VL_CHECK(cudaStreamSynchronize(b->stream));
    for (int d = 0; d < 3; ++d) {
       b->grid_dims[d] = dims[d];
       b->grid_dx[d] = dx[d];
@@ -923,17 +925,18 @@ int vlgpu_batch_fill_maxwellian(vlgpu_batch* b, const vlgpu_maxwellian* cells) {
    FillCell* d_cells = nullptr;
    VL_CHECK(cudaStreamSynchronize(b->stream));
    VL_CHECK(cudaMalloc(&d_cells, sizeof(FillCell) * b->n_cells));
-   cudaError_t e = cudaMemcpy(d_cells, fc.data(), sizeof(FillCell) * b->n_cells, cudaMemcpyHostToDevice);
+   const uint32_t used = (uint32_t)total;
+   cudaError_t e = cudaMemcpyAsync(d_cells, fc.data(), sizeof(FillCell) * b->n_cells, cudaMemcpyHostToDevice, b->stream);
    if (e == cudaSuccess)
       e = launch_fill(d_cells, b->n_cells, b->mdev, b->vmin_d, b->bs_d, b->dv_d, m, b->gids[0], b->data[0],
                       b->slots[0], b->stream);
+   if (e == cudaSuccess)
+      e = cudaMemcpyAsync(b->rows_used, &used, sizeof(uint32_t), cudaMemcpyHostToDevice, b->stream);
+   if (e == cudaSuccess) e = cudaMemsetAsync(b->status, 0, sizeof(uint32_t) * b->n_cells, b->stream);
    if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
    cudaFree(d_cells);
    VL_CHECK(e);
    b->launches += 1;
-   const uint32_t used = (uint32_t)total;
-   VL_CHECK(cudaMemcpy(b->rows_used, &used, sizeof(uint32_t), cudaMemcpyHostToDevice));
-   VL_CHECK(cudaMemset(b->status, 0, sizeof(uint32_t) * b->n_cells));
    set_direct_state(b, 0);
    b->content_valid = false;
    // the first block adjustment prunes the candidates (grid.cpp:289)
