@@ -850,13 +850,17 @@ cudaError_t launch_materialize(const uint32_t* src_index, const float* src, floa
 }
 
 // The same for a row count known only on the device (*n_rows), grid-stride.
+// The count of a list that overflowed is what it would have needed, beyond the
+// pools' `capacity` rows (behind them lies the zero row), and rows that no
+// cell got hold any index: only rows of the pools are read and written.
 __global__ void materialize_rows_kernel(const uint32_t* __restrict__ src_index, const float4* __restrict__ src,
-                                        float4* __restrict__ dst, const uint32_t* __restrict__ n_rows) {
-   const uint64_t n = (uint64_t)(*n_rows) * 16;
+                                        float4* __restrict__ dst, const uint32_t* __restrict__ n_rows,
+                                        uint32_t capacity) {
+   const uint64_t n = (uint64_t)min(*n_rows, capacity) * 16;
    for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (uint64_t)gridDim.x * blockDim.x) {
       const uint64_t p = t >> 4;
       const uint32_t idx = src_index[p];
-      dst[t] = (idx == NO_BLOCK) ? make_float4(0.f, 0.f, 0.f, 0.f) : src[(uint64_t)idx * 16 + (t & 15)];
+      dst[t] = (idx >= capacity) ? make_float4(0.f, 0.f, 0.f, 0.f) : src[(uint64_t)idx * 16 + (t & 15)];
    }
 }
 
@@ -875,9 +879,9 @@ cudaError_t launch_slots_to_host(const CellSlot* src, CellSlot* host_dst, uint32
 }
 
 cudaError_t launch_materialize_rows(const uint32_t* src_index, const float* src, float* dst, const uint32_t* n_rows,
-                                    int grid, cudaStream_t stream) {
+                                    uint32_t capacity, int grid, cudaStream_t stream) {
    materialize_rows_kernel<<<grid, 256, 0, stream>>>(src_index, reinterpret_cast<const float4*>(src),
-                                                     reinterpret_cast<float4*>(dst), n_rows);
+                                                     reinterpret_cast<float4*>(dst), n_rows, capacity);
    return cudaGetLastError();
 }
 

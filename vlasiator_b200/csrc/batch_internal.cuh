@@ -98,7 +98,7 @@ cudaError_t launch_materialize(const uint32_t* src_index, const float* src, floa
                                cudaStream_t stream);
 cudaError_t launch_slots_to_host(const CellSlot* src, CellSlot* host_dst, uint32_t n, cudaStream_t stream);
 cudaError_t launch_materialize_rows(const uint32_t* src_index, const float* src, float* dst, const uint32_t* n_rows,
-                                    int grid, cudaStream_t stream);
+                                    uint32_t capacity, int grid, cudaStream_t stream);
 struct TransCounters {
    uint32_t n_items;
    uint32_t work;

@@ -224,7 +224,7 @@ int materialize_async(vlgpu_batch* b) {
    if (!b->st_src) return VLGPU_OK;
    const int dst = 1 - b->cur;
    VL_CHECK(launch_materialize_rows(b->st_src, b->data[b->cur], b->data[dst], b->rows_used + b->st_list,
-                                    b->sm_count * 8, b->stream));
+                                    (uint32_t)b->capacity, b->sm_count * 8, b->stream));
    b->launches += 1;
    VL_CHECK(cudaMemcpyAsync(b->rows_used + dst, b->rows_used + b->st_list, sizeof(uint32_t),
                             cudaMemcpyDeviceToDevice, b->stream));
