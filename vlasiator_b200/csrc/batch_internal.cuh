@@ -233,6 +233,7 @@ struct vlgpu_batch {
       int adj_next = 0;
       int turn = 0;
       int trans_turn = 0;
+      bool translates = false;       // Vlasov steps, not accelerations
       bool pivot_valid = false;      // at the start of the captured steps
       bool pivot_valid_end = false;  // after them
       unsigned long long launches = 0;

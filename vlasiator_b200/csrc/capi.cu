@@ -987,7 +987,8 @@ int vlgpu_batch_capture(vlgpu_batch* b, int slot, int kind, uint32_t n_steps, co
       g.exec = nullptr;
    }
    const vlgpu_batch::GraphSlot start{nullptr,     b->st_gids, b->st_src,      b->st_slots, b->cur,
-                                      b->adj_next, b->turn,    b->trans_turn,  b->pivot_valid, false, 0, 0};
+                                      b->adj_next, b->turn,    b->trans_turn,  kind == 1,  b->pivot_valid,
+                                      false,       0,          0};
    const bool content_valid = b->content_valid;
    const unsigned long long l0 = b->launches, r0 = b->remap_launches;
    VL_CHECK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeRelaxed));
@@ -1045,7 +1046,8 @@ int vlgpu_batch_replay(vlgpu_batch* b, int slot) {
       VL_CHECK(cudaMemsetAsync(b->counters + g.turn, 0, sizeof(SweepCounters), b->stream));
       b->turn = g.turn;
    }
-   if (b->trans_turn != g.trans_turn) {
+   // (a graph without translations leaves the last one's counters, and what they report, alone)
+   if (g.translates && b->trans_turn != g.trans_turn) {
       VL_CHECK(cudaMemsetAsync(b->tcounters + g.trans_turn, 0, sizeof(TransCounters), b->stream));
       b->trans_turn = g.trans_turn;
    }
