@@ -36,16 +36,10 @@ __device__ __forceinline__ float h7_derivative(float w0, float w1, float w2, flo
 // the Bernstein coefficients fd_l, fd_l + b0/3, fd_l + 2 b0/3 + b1/6, fd_r on
 // the cell; where none opposes the cell's slope, neither does the slope at an
 // inflexion point, and the roots (a square root and two quotients) are not
-// needed.  Where they are, approximate ones do: only the slope's sign there is
-// read.  The error against 64-bit sweeps is the same with rounded ones (9.4e-6 of
-// the peak here and 9.5e-6 with all divisions rounded), which take 792 us
-// instead of 749 for three sweeps of 256 cells with packing (1675 in the
-// form with v0 in every product and all roots).
-__device__ __forceinline__ float sqrt_approx(float x) {
-   float r;
-   asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
-   return r;
-}
+// needed.  Where they are, they are rounded ones: three sweeps of 256 cells with
+// packing take 793 us, 750 with approximate ones (of which only the slope's sign
+// is read: the error against 64-bit sweeps is the same 9.4e-6 of the peak), 1675
+// with v0 in every product and the roots taken in every cell.
 __device__ __forceinline__ void pqm_coeff_fused(float vm1, float v0, float vp1, float fv_l, float fv_r, float fd_l,
                                                 float fd_r, float a[5]) {
    const float dr = vp1 - v0, dl = v0 - vm1;
@@ -73,13 +67,16 @@ __device__ __forceinline__ void pqm_coeff_fused(float vm1, float v0, float vp1, 
    if (fminf(sign * s1, sign * s2) < 0.0f) {
       const float b2 = fmaf(30.0f, e, -180.0f * d);
       const float disc = fmaf(b1, b1, -4.0f * b0 * b2);
-      const float sq = disc < 0.0f ? b1 + 200.0f * b2 : sqrt_approx(disc);
-      const float root1 = __fdividef(-b1 + sq, 2.0f * b2);
-      const float root2 = __fdividef(-b1 - sq, 2.0f * b2);
+      const float sq = disc < 0.0f ? b1 + 200.0f * b2 : sqrtf(disc);
       const float c2 = 0.5f * b1, c3 = b2 * third;
-      const float r1s = (root1 >= 0.0f && root1 <= 1.0f) ? fmaf(root1, fmaf(root1, fmaf(root1, c3, c2), b0), fd_l) : sign;
-      const float r2s = (root2 >= 0.0f && root2 <= 1.0f) ? fmaf(root2, fmaf(root2, fmaf(root2, c3, c2), b0), fd_l) : sign;
-      if (fminf(r1s * sign, r2s * sign) < 0.0f) {
+      float against = 0.0f;  // the lower of the slopes (times sign) at the roots on the cell
+#pragma unroll 1
+      for (int q = 0; q < 2; ++q) {
+         const float root = ((q ? -sq : sq) - b1) / (2.0f * b2);
+         const float at = sign * fmaf(root, fmaf(root, fmaf(root, c3, c2), b0), fd_l);
+         if (root >= 0.0f && root <= 1.0f) against = fminf(against, at);
+      }
+      if (against < 0.0f) {
          if (adl <= adr) {
             // collapse to the left edge (eq. 21), then the PLM-slope checks (eqs. 28, 29)
             fd_l = third * fmaf(8.0f, L, -2.0f * R);
