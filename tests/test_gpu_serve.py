@@ -78,3 +78,16 @@ def test_budget_admission_queues_requests(mesh=VelocityMesh()):
         free = run_all(s, reqs)
     for k in range(len(reqs)):
         same(queued[k], free[k], f"request {k}")
+
+
+def test_budget_covers_the_batch():
+    """What a server allocates on the device stays within its budget, up to the arrays of the cells and the
+    allocations' granularity (about 25 of 2 MiB)."""
+    import torch
+    from vlasiator_b200.serve import Server
+    budget = 24 << 30
+    torch.cuda.synchronize()
+    free, _ = torch.cuda.mem_get_info()
+    with Server(VelocityMesh(), 4, budget):
+        used = free - torch.cuda.mem_get_info()[0]
+    assert 0.99 * budget < used <= budget + (50 << 20)

@@ -29,6 +29,14 @@ namespace {
 // adjustment lists (IDs and data indices), the permutation, the column sets
 // and the content flags.
 constexpr uint64_t BYTES_PER_BLOCK = 2 * 256 + 2 * 4 + 2 * 8 + 4 + sizeof(vlgpu::ColumnSet) + 1;
+// The bytes of a batch that go with its capacity: those, the two rows of zeros
+// behind the pools, the adjustment's items with their sums, and the chunk list
+// of a packing (582.6 per block in all).
+uint64_t capacity_bytes(uint64_t capacity) {
+   return capacity * BYTES_PER_BLOCK + 2 * 256 +
+          capacity / vlgpu::ADJ_ITEM_BLOCKS * (sizeof(vlgpu::AdjustItem) + vlgpu::ADJ_SUMS * sizeof(double)) +
+          vlgpu::pack_scratch_words(capacity, 0, 0) * sizeof(uint32_t);
+}
 // Admission keeps the live blocks below this fraction of the capacity, which
 // leaves room for the blocks a step adds and for the rows of new requests.
 constexpr double ADMIT_FRACTION = 0.6;
@@ -105,6 +113,8 @@ int vlgpu_server_create(const vlgpu_mesh* mesh, const vlgpu_params* params, uint
                         uint64_t hbm_budget_bytes, int device, vlgpu_server** out) {
    if (!out || max_cells == 0 || hbm_budget_bytes < BYTES_PER_BLOCK * 4096) return VLGPU_EINVAL;
    uint64_t capacity = hbm_budget_bytes / BYTES_PER_BLOCK;
+   if (capacity_bytes(capacity) > hbm_budget_bytes)
+      capacity -= (capacity_bytes(capacity) - hbm_budget_bytes + BYTES_PER_BLOCK - 1) / BYTES_PER_BLOCK;
    if (capacity >= 0xffffffffull) capacity = 0xfffffffeull;
    vlgpu_batch* b = nullptr;
    const int st = vlgpu_batch_create(mesh, params, max_cells, capacity, device, &b);
