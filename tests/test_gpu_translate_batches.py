@@ -44,3 +44,29 @@ def test_pencil_lengths(mesh, orc_sp, dim, n):
     for c in range(k):
         np.testing.assert_array_equal(got[c][0], gids[c])
         assert np.abs(got[c][1] - want[offs[c]:offs[c + 1]]).max() <= 1e-5 * peak
+
+
+@pytest.mark.parametrize("dim", [0, 1, 2])
+def test_planes_of_nan(mesh, dim):
+    """A plane of NaN has no positive value, so the remap is left out there, also where every other value is positive;
+    as the exact mode does it."""
+    from vlasiator_b200 import vlgpu
+    grid = [1, 1, 1]
+    grid[dim] = n = 9
+    gids = maxwellian_cell(mesh, 1e6, 2e5, (1e5, -2e5, 5e4)).gids
+    rng = np.random.default_rng(dim)
+    data = (1e-13 * rng.uniform(0.5, 1.0, (n, len(gids), 4, 4, 4))).astype(np.float32)  # [z][y][x]
+    plane = [slice(None)] * 3
+    plane[2 - dim] = 2
+    data[(slice(None), slice(3, None, 5), *plane)] = np.nan
+    data = data.reshape(n, len(gids), 64)
+    got = {}
+    for exact in (False, True):
+        with vlgpu.Batch(mesh, n, 4 * n * len(gids) + 4096, exact=exact) as b:
+            b.upload([gids] * n, list(data))
+            b.set_grid(grid, 3e5)
+            b.translate(dim, 0.7 * 3e5 / 1.2e6)
+            got[exact] = np.stack([d for _, d in b.cells()])
+            b.sync()
+    assert np.isfinite(got[True]).all()
+    assert np.abs(got[False] - got[True]).max() <= 1e-5 * 1e-13

@@ -442,6 +442,13 @@ __device__ __forceinline__ void plane_edge(float zt, float& w, float& wm, bool& 
    wm = up ? -zt : -zt - 1.0f;
 }
 
+// The lower of two values, NaN if either is one.
+__device__ __forceinline__ float min_or_nan(float a, float b) {
+   float r;
+   asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+   return r;
+}
+
 // This lane's two columns of the block at data row idx (src2: the lane's place
 // in row 0).
 __device__ __forceinline__ float2 load_column_pair(const float2* __restrict__ src2, uint32_t idx) {
@@ -587,11 +594,12 @@ __global__ void __launch_bounds__(TF_THREADS, TF_CTAS) trans_fused_kernel(
       auto window_cell = [&](uint32_t m) { return load_column_pair(src2, tsrc[min(m, N + 5)]); };
 #pragma unroll
       for (int j = 0; j < W; ++j) w[j] = window_cell((uint32_t)j);
-      // every value of the window's first six cells positive / of the others
+      // every value of the window's first six cells positive / of the others (a
+      // NaN is not)
       auto positive = [&](int j0, int j1) {
          float m = 1.0f;
 #pragma unroll
-         for (int j = j0; j < j1; ++j) m = fminf(m, fminf(w[j].x, w[j].y));
+         for (int j = j0; j < j1; ++j) m = min_or_nan(m, min_or_nan(w[j].x, w[j].y));
          return (bool)__all_sync(0xffffffffu, m > 0.0f);
       };
       // (columns of a plane in other lanes: bit j, some positive value in window cell j)
