@@ -736,7 +736,7 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_VALUE_CTAS) adjust_values_ker
 #pragma unroll
          for (int q = 0; q < 10; ++q) Sv[q] = __shfl_sync(FULL, S, q + 1);
          if (lane == 0)
-            moments_record<MOM_BOTH>(Sv, 0.0, 0.0, 0.0, U0, U1, U2, fr.dv[0], fr.dv[1], fr.dv[2], fr.mass, fr.charge,
+            moments_record<MOM_BOTH>(Sv, U0, U1, U2, fr.dv[0], fr.dv[1], fr.dv[2], fr.mass, fr.charge,
                                      mom_record + (size_t)cell * MOM_COUNT,
                                      write_pivot ? pivot + (size_t)cell * MOM_COUNT : nullptr);
       }

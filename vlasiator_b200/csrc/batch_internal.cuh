@@ -52,9 +52,9 @@ struct CellAccelInputs {
    double dt;
 };
 cudaError_t launch_moments(const uint32_t* gids, const uint32_t* src_index, const float* data, const CellSlot* slots,
-                           double* moments, const double* shift, const MeshDev& mesh, const double vmin[3],
-                           const double bs[3], const double dv[3], double mass, double charge, bool second,
-                           uint32_t n_cells, double* part_sums, uint32_t* done, int grid, cudaStream_t stream);
+                           double* moments, const MeshDev& mesh, const double vmin[3], const double bs[3],
+                           const double dv[3], double mass, double charge, uint32_t n_cells, double* part_sums,
+                           uint32_t* done, int grid, cudaStream_t stream);
 cudaError_t launch_moments_both(const uint32_t* gids, const uint32_t* src_index, const float* data,
                                 const CellSlot* slots, double* pivot, double* moments, const MeshDev& mesh,
                                 const double vmin[3], const double bs[3], const double dv[3], double mass,
@@ -261,7 +261,7 @@ int cuda_status(cudaError_t e, const char* what);
 void free_batch(vlgpu_batch* b);
 void set_direct_state(vlgpu_batch* b, int pool);
 int sweep_device(vlgpu_batch* b, const vlgpu::SweepCell* sweep_cells, uint32_t dim, bool per_cell, bool first_of_step);
-int moments_device(vlgpu_batch* b, bool second, double* record = nullptr, const double* shift = nullptr);
+int moments_device(vlgpu_batch* b, double* record = nullptr);
 int moments_both_device(vlgpu_batch* b, double* record);
 int adjust_device(vlgpu_batch* b, double* record = nullptr, bool write_pivot = false);
 int materialize(vlgpu_batch* b);

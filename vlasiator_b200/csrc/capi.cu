@@ -140,11 +140,11 @@ int run_sweep(vlgpu_batch* b, const double* intersections, size_t stride, uint32
    return sweep_device(b, b->sweep_cells, dim, per_cell, false);
 }
 
-int moments_device(vlgpu_batch* b, bool second, double* record, const double* shift) {
+int moments_device(vlgpu_batch* b, double* record) {
    b->launches += 1;
-   VL_CHECK(launch_moments(b->st_gids, b->st_src, b->data[b->cur], b->st_slots, record ? record : b->moments, shift,
-                           b->mdev, b->vmin_d, b->bs_d, b->dv_d, b->params.mass, b->params.charge, second,
-                           b->n_cells, b->mom_parts, b->mom_done, b->mom_grid, b->stream));
+   VL_CHECK(launch_moments(b->st_gids, b->st_src, b->data[b->cur], b->st_slots, record ? record : b->moments, b->mdev,
+                           b->vmin_d, b->bs_d, b->dv_d, b->params.mass, b->params.charge, b->n_cells, b->mom_parts,
+                           b->mom_done, b->mom_grid, b->stream));
    return VLGPU_OK;
 }
 
@@ -239,7 +239,7 @@ int geometry_device(vlgpu_batch* b, uint32_t map_order) {
    // unless the moments that ended the previous step or the Vlasov step's "_R"
    // moments already wrote it for this VDF
    if (!b->pivot_valid) {
-      const int st = moments_device(b, false, b->pivot);
+      const int st = moments_device(b, b->pivot);
       if (st != VLGPU_OK) return st;
       b->pivot_valid = true;
    }
@@ -727,7 +727,7 @@ int vlgpu_batch_rho_loss(vlgpu_batch* b, double* out) {
 int vlgpu_batch_moments(vlgpu_batch* b, int compute_second, double* out16) {
    if (!b || !out16) return VLGPU_EINVAL;
    VL_CHECK(cudaSetDevice(b->device));
-   const int st = compute_second ? moments_both_device(b, b->moments) : moments_device(b, false);
+   const int st = compute_second ? moments_both_device(b, b->moments) : moments_device(b);
    if (st != VLGPU_OK) return st;
    VL_CHECK(cudaMemcpyAsync(out16, b->moments, sizeof(double) * MOM_COUNT * b->n_cells, cudaMemcpyDeviceToHost,
                             b->stream));

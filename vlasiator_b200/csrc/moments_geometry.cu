@@ -67,12 +67,11 @@ __device__ __forceinline__ uint32_t moment_parts(uint32_t count) {
 template <int MODE>
 __global__ void __launch_bounds__(MOM_THREADS, MOM_CTAS) moments_parts_kernel(
    const uint32_t* __restrict__ gids, const uint32_t* __restrict__ src_index, const float* __restrict__ data,
-   const CellSlot* __restrict__ slots, double* moments, double* pivot, const double* shift,
+   const CellSlot* __restrict__ slots, double* moments, double* pivot,
    double* __restrict__ part_sums, uint32_t* __restrict__ done, MeshDev mesh, double vmin0, double vmin1,
    double vmin2, double bs0, double bs1, double bs2, double dv0, double dv1, double dv2, double mass, double charge,
    uint32_t n_cells) {
-   constexpr bool SECOND = MODE != MOM_FIRST;
-   constexpr int NS = SECOND ? 10 : 4;
+   constexpr int NS = MODE == MOM_BOTH ? 10 : 4;
    __shared__ double sh[MOM_THREADS / 32][NS][33];  // a warp's lane sums, one row per sum (padded)
    // a tile's blocks: position x + (y << 8) + (z << 16) and data row
    __shared__ uint32_t sg[MOM_THREADS / 32][MOM_TILE], si[MOM_THREADS / 32][MOM_TILE];
@@ -105,21 +104,15 @@ __global__ void __launch_bounds__(MOM_THREADS, MOM_CTAS) moments_parts_kernel(
       if (part >= parts) continue;
       const uint32_t b0 = (uint32_t)(((uint64_t)s.count * part) / parts);
       const uint32_t b1 = (uint32_t)(((uint64_t)s.count * (part + 1)) / parts);
-      // the reference velocity: the pivot's (MOM_BOTH) or the shift record's (MOM_SECOND)
+      // the reference velocity: the pivot's
       double U0 = 0.0, U1 = 0.0, U2 = 0.0;
       if (MODE == MOM_BOTH) {
          const double* pv = pivot + (size_t)cell * MOM_COUNT;
          U0 = pv[MOM_VX]; U1 = pv[MOM_VY]; U2 = pv[MOM_VZ];
-      } else if (MODE == MOM_SECOND) {
-         const double* sh_rec = shift + (size_t)cell * MOM_COUNT;
-         U0 = sh_rec[MOM_VX]; U1 = sh_rec[MOM_VY]; U2 = sh_rec[MOM_VZ];
       }
-      // the first sums are about F (0, or U in MOM_SECOND); a lane's row of
-      // four cells starts at the cell centre x0 = corner + dv0/2 - F0, the
-      // others follow at dv0 steps
-      const double F0 = (MODE == MOM_SECOND) ? U0 : 0.0, F1 = (MODE == MOM_SECOND) ? U1 : 0.0;
-      const double F2 = (MODE == MOM_SECOND) ? U2 : 0.0;
-      const double ox = 0.5 * dv0 - F0, oy = (j + 0.5) * dv1 - F1, oz = (k + 0.5) * dv2 - F2;
+      // a lane's row of four cells starts at the cell centre x0 = corner +
+      // dv0/2, the others follow at dv0 steps
+      const double ox = 0.5 * dv0, oy = (j + 0.5) * dv1, oz = (k + 0.5) * dv2;
       double t[NS];
 #pragma unroll
       for (int q = 0; q < NS; ++q) t[q] = 0.0;
@@ -170,18 +163,9 @@ __global__ void __launch_bounds__(MOM_THREADS, MOM_CTAS) moments_parts_kernel(
                t[1] += sfx;
                t[2] = fma(s0, uy, t[2]);
                t[3] = fma(s0, uz, t[3]);
-               if constexpr (MODE == MOM_SECOND) {
-                  // sum f x^2 = x0^2 s0 + 2 x0 dv0 s1 + dv0^2 s2
-                  t[4] += fma(x0, fma(x0, s0, 2.0 * ds1), dv0s * s2);
-                  const double s0y = s0 * uy;
-                  t[5] = fma(s0y, uy, t[5]);
-                  t[6] = fma(s0 * uz, uz, t[6]);
-                  t[7] = fma(s0y, uz, t[7]);
-                  t[8] = fma(sfx, uz, t[8]);
-                  t[9] = fma(sfx, uy, t[9]);
-               }
                if constexpr (MODE == MOM_BOTH) {
-                  // the same row relative to U (the first sums were about 0)
+                  // the same row relative to U (the first sums were about 0):
+                  // sum f y^2 = y0^2 s0 + 2 y0 dv0 s1 + dv0^2 s2
                   const double y0 = x0 - U0, vy = uy - U1, vz = uz - U2;
                   const double sfy = fma(y0, s0, ds1);
                   t[4] += fma(y0, fma(y0, s0, 2.0 * ds1), dv0s * s2);
@@ -233,7 +217,7 @@ __global__ void __launch_bounds__(MOM_THREADS, MOM_CTAS) moments_parts_kernel(
 #pragma unroll
       for (int q = 0; q < NS; ++q) Sv[q] = __shfl_sync(0xffffffffu, S, q);
       if (lane == 0) {
-         moments_record<MODE>(Sv, F0, F1, F2, U0, U1, U2, dv0, dv1, dv2, mass, charge,
+         moments_record<MODE>(Sv, U0, U1, U2, dv0, dv1, dv2, mass, charge,
                               moments + (size_t)cell * MOM_COUNT,
                               MODE == MOM_BOTH ? pivot + (size_t)cell * MOM_COUNT : nullptr);
          done[cell] = 0;  // ready for the next pass
@@ -357,19 +341,13 @@ int moments_blocks_per_sm() {
 }
 
 cudaError_t launch_moments(const uint32_t* gids, const uint32_t* src_index, const float* data, const CellSlot* slots,
-                           double* moments, const double* shift, const MeshDev& mesh, const double vmin[3],
-                           const double bs[3], const double dv[3], double mass, double charge, bool second,
-                           uint32_t n_cells, double* part_sums, uint32_t* done, int grid, cudaStream_t stream) {
+                           double* moments, const MeshDev& mesh, const double vmin[3], const double bs[3],
+                           const double dv[3], double mass, double charge, uint32_t n_cells, double* part_sums,
+                           uint32_t* done, int grid, cudaStream_t stream) {
    if (n_cells == 0) return cudaSuccess;
-   if (!shift) shift = moments;
-   if (second)
-      moments_parts_kernel<MOM_SECOND><<<grid, MOM_THREADS, 0, stream>>>(
-         gids, src_index, data, slots, moments, nullptr, shift, part_sums, done, mesh, vmin[0], vmin[1], vmin[2],
-         bs[0], bs[1], bs[2], dv[0], dv[1], dv[2], mass, charge, n_cells);
-   else
-      moments_parts_kernel<MOM_FIRST><<<grid, MOM_THREADS, 0, stream>>>(
-         gids, src_index, data, slots, moments, nullptr, shift, part_sums, done, mesh, vmin[0], vmin[1], vmin[2],
-         bs[0], bs[1], bs[2], dv[0], dv[1], dv[2], mass, charge, n_cells);
+   moments_parts_kernel<MOM_FIRST><<<grid, MOM_THREADS, 0, stream>>>(
+      gids, src_index, data, slots, moments, nullptr, part_sums, done, mesh, vmin[0], vmin[1], vmin[2], bs[0], bs[1],
+      bs[2], dv[0], dv[1], dv[2], mass, charge, n_cells);
    return cudaGetLastError();
 }
 
@@ -380,7 +358,7 @@ cudaError_t launch_moments_both(const uint32_t* gids, const uint32_t* src_index,
                                 cudaStream_t stream) {
    if (n_cells == 0) return cudaSuccess;
    moments_parts_kernel<MOM_BOTH><<<grid, MOM_THREADS, 0, stream>>>(
-      gids, src_index, data, slots, moments, pivot, nullptr, part_sums, done, mesh, vmin[0], vmin[1], vmin[2], bs[0],
+      gids, src_index, data, slots, moments, pivot, part_sums, done, mesh, vmin[0], vmin[1], vmin[2], bs[0],
       bs[1], bs[2], dv[0], dv[1], dv[2], mass, charge, n_cells);
    return cudaGetLastError();
 }

@@ -27,27 +27,24 @@ enum MomentSlot {
    MOM_COUNT = 16
 };
 
-// Modes: MOM_FIRST sums the first moments about 0; MOM_SECOND sums everything
-// about the U of the `shift` record; MOM_BOTH does both passes' work in one
-// read: the first sums about 0 with exactly MOM_FIRST's arithmetic (so the
+// Modes: MOM_FIRST sums the first moments about 0; MOM_BOTH the first and the
+// second ones in one read: the first sums about 0 with exactly MOM_FIRST's arithmetic (so the
 // first moments, which the next acceleration takes as its pivot, are
 // bit-identical to a MOM_FIRST pass) and the second sums about the U of the
 // pivot record, whose first sums T_a = S_a - U_a S0 follow from the former;
 // the cancellation in T_a costs about eps (U / v_th)^2 of P relative and
 // vanishes as U approaches V.  MOM_BOTH writes the full record to `out` and
 // the first moments (pressure zero, as MOM_FIRST) to the pivot record.
-constexpr int MOM_FIRST = 0, MOM_SECOND = 1, MOM_BOTH = 2;
+constexpr int MOM_FIRST = 0, MOM_BOTH = 1;
 
-// The record of a cell from its sums S (about U for the second moments; the
-// first sums about F, which is 0 or U).
+// The record of a cell from its sums S (the first about 0, the second about U).
 template <int MODE>
-__device__ __forceinline__ void moments_record(const double* S, double F0, double F1, double F2, double U0, double U1,
-                                            double U2, double dv0, double dv1, double dv2, double mass, double charge,
-                                            double* out, double* out1) {
-   constexpr bool SECOND = MODE != MOM_FIRST;
+__device__ __forceinline__ void moments_record(const double* S, double U0, double U1, double U2, double dv0,
+                                               double dv1, double dv2, double mass, double charge, double* out,
+                                               double* out1) {
    const double DV3 = dv0 * dv1 * dv2;
    const double a0 = S[0] * DV3;
-   const double a1 = (S[1] + F0 * S[0]) * DV3, a2 = (S[2] + F1 * S[0]) * DV3, a3 = (S[3] + F2 * S[0]) * DV3;
+   const double a1 = S[1] * DV3, a2 = S[2] * DV3, a3 = S[3] * DV3;
    const double rhom = a0 * mass;
    const double first[MOM_P11] = {a0,
                                   a1,
@@ -70,12 +67,10 @@ __device__ __forceinline__ void moments_record(const double* S, double F0, doubl
       for (int q = 0; q < 6; ++q) out1[MOM_P11 + q] = 0.0;
    }
    double P[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-   if constexpr (SECOND) {
+   if constexpr (MODE == MOM_BOTH) {
       if (S[0] != 0.0) {
-         // first sums about U (those of MOM_BOTH were taken about 0)
-         const double T1 = (MODE == MOM_BOTH) ? S[1] - U0 * S[0] : S[1];
-         const double T2 = (MODE == MOM_BOTH) ? S[2] - U1 * S[0] : S[2];
-         const double T3 = (MODE == MOM_BOTH) ? S[3] - U2 * S[0] : S[3];
+         // first sums about U
+         const double T1 = S[1] - U0 * S[0], T2 = S[2] - U1 * S[0], T3 = S[3] - U2 * S[0];
          const double m1 = T1 / S[0], m2 = T2 / S[0], m3 = T3 / S[0];
          const double pre = mass * DV3;
          P[0] = pre * (S[4] - T1 * m1);

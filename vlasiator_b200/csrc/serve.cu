@@ -253,7 +253,7 @@ int vlgpu_server_tick(vlgpu_server* s, uint32_t* n_active, uint32_t* n_pending, 
          // the admitted cells' pivots from their VDFs; every other cell keeps
          // the pivot its last step wrote, so a request's steps do not depend
          // on the requests admitted beside it
-         const int st = moments_device(b, false, b->mom_scratch);
+         const int st = moments_device(b, b->mom_scratch);
          if (st != VLGPU_OK) return st;
          for (uint32_t c : admitted)
             VL_CHECK(cudaMemcpyAsync(b->pivot + (size_t)c * MOM_COUNT, b->mom_scratch + (size_t)c * MOM_COUNT,
