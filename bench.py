@@ -48,9 +48,9 @@ UNIT = "cell-updates/s"
 WORKLOAD = "batched acceleration, 4096 drifting Maxwellian cells, 1 SLICE-3D step (PPM), dt=0.01 gyroperiod"
 BYTES_PER_CELL_SWEEP = 8  # read + write one fp32 phase-space cell per 1D sweep
 # DRAM bytes (read + write) of one remap launch per source block (every block
-# is read and written once, however many columns a lane walks), from one ncu capture (dram__bytes_read.sum + dram__bytes_write.sum = 204.9 +
-# 176.0 MB) of the 512-cell case of this workload (705,499 blocks at the step's
-# start), fused arithmetic; scaled by the source blocks of a launch to give the
+# is read and written once, however many columns a lane walks), from one ncu
+# capture (dram__bytes_read.sum + dram__bytes_write.sum = 204.9 + 176.0 MB) of the
+# 512-cell case of this workload (705,499 blocks at the step's start), fused arithmetic; scaled by the source blocks of a launch to give the
 # full-size traffic per launch.
 REMAP_DRAM_BYTES_PER_BLOCK = 380.9e6 / 705499
 DEFAULT_SEED = 2026  # the workload's seed unless --seed says otherwise
@@ -440,8 +440,8 @@ def run_ours(args):
         "gpu_launches": launches,
         "cuda_graph": bool(args.graph),
         "arithmetic": "exact (bit-identical to the reference's map_1d)" if args.exact else
-                      "fused (the remap walk: PPM face values once per face, target edges with the "
-                      "reference's rounding; 1e-5 of peak per sweep)",
+                      "fused (two columns per lane: PPM face values once per face, limiter in magnitudes, target "
+                      "edges with the reference's rounding; 1e-5 of peak per sweep)",
         "latency_ms": {"p50": float(np.percentile(step_ms, 50)), "p99": float(np.percentile(step_ms, 99)),
                        "what": "device time of one batched acceleration step of all cells"},
         "plain_per_cell": plain,

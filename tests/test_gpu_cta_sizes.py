@@ -1,11 +1,12 @@
 """The kernels that take a cell per CTA (columnize, the adjustment's lists)
 run with larger CTAs where the cells are few, and the adjustment's values are
-summed in parts of about 128 blocks.  A cell's step must not depend on any of
+summed in parts of 64 blocks (cells of up to 1024 blocks) or 128.  A cell's step must not depend on any of
 that: the same cells alone, beside a few and beside many others come out
 bit-identical, and equal to the oracle's adjustment and moments.
 
-Sizes: no block, one block, the edges of a staged tile and of a part (127 to
-129, 255 to 257 blocks), more blocks than 64 parts of 128, and a cell whose
+Sizes: no block, one block, the edges of a part of 64 (63 to 65, 127 to 129,
+255 to 257 blocks), of the change to parts of 128 (1023 to 1025) and of a part
+after it (1151 to 1153), more blocks than 64 parts of 128, and a cell whose
 transverse plane exceeds the capped columnize launch (1024 entries)."""
 import numpy as np
 import pytest
@@ -15,12 +16,13 @@ from vlasiator_b200.projects import maxwellian_cell
 
 pytestmark = pytest.mark.gpu
 
-COUNTS = (0, 1, 2, 127, 128, 129, 255, 256, 257)
+COUNTS = (0, 1, 2, 63, 64, 65, 127, 128, 129, 255, 256, 257, 1023, 1024, 1025, 1151, 1152, 1153)
 
 
 def _cells(mesh):
-    base = maxwellian_cell(mesh, 1e6, 8e5, (1e5, -2e5, 5e4))
-    cells = [(base.gids[:n], base.data[:n]) for n in COUNTS]
+    base, more = (maxwellian_cell(mesh, 1e6, T, (1e5, -2e5, 5e4)) for T in (8e5, 2e6))
+    assert len(more.gids) >= max(COUNTS)
+    cells = [((base if n < 512 else more).gids[:n], (base if n < 512 else more).data[:n]) for n in COUNTS]
     hot = maxwellian_cell(mesh, 3e6, 1.2e7, (0.0, 3e5, 0.0))
     assert len(hot.gids) > 64 * 128
     cells.append((hot.gids, hot.data))
@@ -69,7 +71,7 @@ def test_adjustment_against_oracle(alone, mesh, orc_sp):
         np.testing.assert_allclose(mom[c][9:15], m[9:15], rtol=0, atol=1e-9 * np.abs(m[9:15]).max())
 
 
-@pytest.mark.parametrize("copies", [3, 20, 115])  # 33, 220 and 1265 cells: each CTA size
+@pytest.mark.parametrize("copies", [3, 20, 60])  # 60, 400 and 1200 cells: each CTA size
 def test_same_in_every_batch_size(alone, mesh, copies):
     from vlasiator_b200 import vlgpu
     many = _run(vlgpu, mesh, _cells(mesh), copies)

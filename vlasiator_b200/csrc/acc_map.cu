@@ -1113,9 +1113,10 @@ __global__ void __launch_bounds__(REMAP_THREADS, 3) remap_walk_kernel(
 //
 // Bound by issue and the ALU pipe (72% and 60% busy with 24 warps per SM, the
 // most the ring's 64 KB per CTA leave room for).  Measured on 4096 drifting
-// Maxwellian cells (5.8 M blocks): 1145 us per sweep, 2870 GB/s of 8 B per
-// cell, against 1415 us and 2321 GB/s with half a warp per set; 64 cells: 38
-// against 53 us; PLM on 1024 cells: 247 against 291 us.  Two CTAs per SM with
+// Maxwellian cells (5.8 M blocks): 2870 GB/s of 8 B per cell against 2321 GB/s
+// with half a warp per set (1145 against 1415 us), and with the sets by length
+// (columnize_cell) 3197 GB/s; before that, 64 cells: 38 against 53 us; PLM on
+// 1024 cells: 247 against 291 us.  Two CTAs per SM with
 // 100 registers take 17% longer, a loop over two blocks that loads a block
 // ahead 25% (instruction cache); prefetches to L2 change nothing.
 constexpr int PAIR_THREADS = 256;
@@ -1570,6 +1571,12 @@ __global__ void __launch_bounds__(PAIR_THREADS, PAIR_CTAS) remap_pair_kernel(
 // ---------------------------------------------------------------------------
 // host-side launch helpers (used by capi.cu)
 // ---------------------------------------------------------------------------
+// Columnize of the cells [cell_begin, cell_end) in launch order, each with room
+// for the whole plane (at 67 x 67 two CTAs' worth of an SM's shared memory) and
+// one CTA of 1024 threads per SM: for few cells, and for the per-cell calls,
+// which bring one cell or a few.  (A call of map_1d_noalloc with many cells takes this form too:
+// 592 cells of 30 blocks 96 us in all, 1024 of 14 blocks 110 us; 105 and 121 us
+// with 256 threads, before its copies and waits were merged.)
 cudaError_t launch_columnize(int dim, const uint32_t* gids, const uint32_t* src_index, const CellSlot* src_slots,
                              CellSlot* dst_slots,
                              uint32_t* perm, ColumnSet* sets, uint32_t set_capacity, uint32_t dst_capacity,
@@ -1597,7 +1604,7 @@ cudaError_t launch_columnize(int dim, const uint32_t* gids, const uint32_t* src_
 
 // Columnize of every cell of a batch: one CTA per cell, the largest cells
 // first (order), with shared memory for planes of up to COL_CAP_PLANE entries,
-// which lets four CTAs share an SM; the cells with wider planes follow in
+// which lets six CTAs share an SM; the cells with wider planes follow in
 // columnize_wide_kernel.  The counters are zero before every sweep.
 constexpr uint32_t COL_CAP_PLANE = 1024;
 cudaError_t launch_columnize_batch(int dim, const uint32_t* gids, const uint32_t* src_index,

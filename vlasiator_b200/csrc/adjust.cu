@@ -54,7 +54,10 @@ constexpr uint32_t NO_BLOCK = 0xffffffffu;
 // each before) 2828 -> 2724 us.
 // Parts of 64 blocks for every cell make 4096 cells of 1423 blocks 5% slower
 // (29.2 -> 30.7 ms: a part's own loads and sums), parts of 32 blocks make a
-// cell of 412 blocks no faster (680 against 686 us).
+// cell of 412 blocks no faster (680 against 686 us).  The rule goes by the cell,
+// so large batches of small cells pay a little: a step of 2048 cells of 653
+// blocks 1157 us, 1129 with parts of 128; of 8192 cells of 310 blocks 2372
+// and 2337.
 __device__ __forceinline__ uint32_t value_parts(uint32_t count) {
    const uint32_t size = count <= 1024 ? ADJ_ITEM_BLOCKS : ADJ_TILE;
    return (count + size - 1) / size;

@@ -462,7 +462,7 @@ int vlgpu_batch_destroy(vlgpu_batch* b) {
    return VLGPU_OK;
 }
 
-// The cells by decreasing block count, for the warp-per-cell kernels (the
+// The cells by decreasing block count, for the kernels of a CTA per cell (the
 // longest cells start first).  Waits for the previous copy of the staging
 // buffer, then copies it on the batch's stream.
 static cudaError_t upload_cell_order(vlgpu_batch* b, const uint64_t* offsets) {

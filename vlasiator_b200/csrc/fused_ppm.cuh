@@ -124,11 +124,9 @@ __device__ __forceinline__ float pqm_integral(float u, const float a[5]) {
 
 // The h4 face of uniform cells, (-v_{-2} + 7 v_{-1} + 7 v_0 - v_1) / 12
 // (cpu_face_estimates.hpp:160-167), and PPM for two columns at once, with the
-// packed single-precision operations of sm_100 (__fadd2_rn, __fmul2_rn, __ffma2_rn;
-// y - x as fma(x, -1, y), exact before rounding); the limiter's comparisons
-// and selections stay per component.
+// packed single-precision operations of sm_100 (__fadd2_rn, __fmul2_rn, __ffma2_rn);
+// the limiter's comparisons and selections stay per component.
 __device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
-__device__ __forceinline__ float2 p_sub(float2 y, float2 x) { return __ffma2_rn(x, f2(-1.0f), y); }
 
 __device__ __forceinline__ float2 h4_face_x2(float2 vm2, float2 vm1, float2 v0, float2 vp1) {
    return __ffma2_rn(__fadd2_rn(vm1, v0), f2((float)(7.0 / 12.0)),
@@ -138,8 +136,11 @@ __device__ __forceinline__ float2 h4_face_x2(float2 vm2, float2 vm1, float2 v0, 
 // y - x of two columns.
 __device__ __forceinline__ float2 p_minus(float2 y, float2 x) { return __fadd2_rn(y, make_float2(-x.x, -x.y)); }
 
-// a b > 0 of two value differences as a factor 0 or 1: their scaled product,
-// saturated.  2^75 squared times the smallest denormal product is 1.
+// a b > 0 of two value differences as a factor: their product times 2^150,
+// saturated.  Where a b > 0 holds in single precision the product is 2^-149 at
+// least, so the factor is 1; it is 0 at an extremum.  (A positive product that
+// single precision loses, of differences below 1e-22, gives 1 or a fraction,
+// where the comparison would flatten the cell.)
 constexpr float SAME_SCALE = 37778931862957161709568.0f;
 
 // Half the superbee slope of two columns, h = min(|a|, |b|, max(|a|, |b|) / 2)

@@ -107,10 +107,6 @@ __device__ __forceinline__ void block_xyz(const MeshDev& m, uint32_t g, uint32_t
    }
 }
 
-// Content mask of one cell for the block adjustment on a grid: the (y, z)
-// bounding box of its content blocks (y1 < 0: none) and the offset of its
-// x-mask rows (3 words per row) in the mask pool, or 0xffffffff when the rows
-// were not stored (the cell's block list is read instead).
 // The velocity mesh in FP64 for the moment sums: minimum, block size and
 // cell size per dimension, and the species' mass and charge.
 struct MomentFrame {
@@ -118,21 +114,25 @@ struct MomentFrame {
    double mass, charge;
 };
 
+// Content mask of one cell for the block adjustment on a grid: the (y, z)
+// bounding box of its content blocks (y1 < 0: none) and the offset of its
+// x-mask rows (3 words per row) in the mask pool, or 0xffffffff when the rows
+// were not stored (the cell's block list is read instead).
 struct MaskRec {
    int32_t y0, y1, z0, z1;
    uint32_t off;
    uint32_t pad[3];
 };
 
-// Counters of one sweep, zeroed before the columnize launch.
+// Counters of one sweep or adjustment, zero when it starts (see HandOver).
 struct SweepCounters {
    uint32_t n_sets;
    uint32_t dst_top;
    uint32_t work;       // remap: sets claimed beyond the warps' first ones
    uint32_t first_set;  // remap: the first set of this launch
    uint32_t overflow;
-   uint32_t cell_next;  // warp-per-cell kernels (columnize, adjustment): next cell a warp takes
-   uint32_t n_wide;     // cells those kernels left to their CTA-per-cell forms
+   uint32_t cell_next;  // adjustment's lists: the next cell a CTA takes
+   uint32_t n_wide;     // cells columnize left to its wide-plane form
    uint32_t n_items;    // adjustment: parts of the pass over the values
 };
 
