@@ -75,3 +75,36 @@ def test_more_sets_than_workers(orc_sp):
         for c in range(k, n, 3):
             np.testing.assert_array_equal(got[c][0], g2[o])
             assert np.abs(got[c][1] - d2[o]).max() <= 1e-5 * d.max()
+
+
+@pytest.mark.parametrize("recon", ["plm", "ppm"])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("dim", [0, 1, 2])
+def test_what_is_not_finite_stays_where_it_is(orc_sp, dim, bad, recon):
+    """Single values that are not finite reach the target cells that they overlap, and no others: their neighbours'
+    reconstructions do without the faces they spoil.  Which cells those are the oracle says: a one among zeros is flat
+    in its cell."""
+    from vlasiator_b200 import vlgpu
+    rng = np.random.default_rng(300 + dim)
+    dv = float(MESH.dv[dim])
+    cells, ones = [], []
+    for n, spread in ((27, 3), (60, 6), (150, 10)):
+        g, d = _cell(rng, n, spread)
+        at = np.zeros(d.shape, bool)
+        at[::3, rng.integers(0, 64)] = True  # in every third block: not two neighbours in a column
+        ones.append(at.astype(np.float32))
+        cells.append((g, np.where(at, np.float32(bad), d)))
+    shear = np.array([0.03, -0.05, 0.02]) * dv
+    shear[dim] = 1.02 * dv
+    isect = np.array([-80 * 1.02 * dv - 80 * (shear.sum() - shear[dim]) + 0.4 * dv, *shear])
+    with vlgpu.Batch(MESH, len(cells), 65536, recon=recon) as b:
+        b.upload([g for g, _ in cells], [d for _, d in cells])
+        b.map_1d(np.tile(isect, (len(cells), 1)), dim)
+        got = b.cells()
+        assert not b.status().any()
+    for (g, _), at, (g2, d2) in zip(cells, ones, got):
+        go, reached, _ = orc_sp.map_1d(MESH, g, at, isect, dim, 1e-15)
+        o = np.argsort(go)
+        np.testing.assert_array_equal(g2, go[o])
+        assert np.isfinite(d2[reached[o] == 0.0]).all()
+        assert not np.isfinite(d2[reached[o] > 1e-3]).any()

@@ -166,15 +166,16 @@ struct PpmWalk {
       left = p_minus(v0, face);
       b = p_minus(v0, vm1);
       const float2 t = __fmul2_rn(p_minus(face, vm1), left);
-      out_x = t.x < 0.0f;
-      out_y = t.y < 0.0f;
+      out_x = !(t.x >= 0.0f);
+      out_y = !(t.y >= 0.0f);
    }
 };
 
 // PPM of two columns in magnitudes (cpu_1d_ppm.hpp:35-54): l = |v0 - left
 // face|, r = |right face - v0| after the limiters; with the slope's sign s the
 // integral of the reconstruction from 0 to u is u (v0 + s (u-1) (l + u (r-l))).
-// A face outside its two cells' values gives half the superbee slope instead;
+// A face outside its two cells' values (or one that is not a number, next to a
+// value that is not) gives half the superbee slope instead;
 // the Colella-Woodward corrections are l = min(l, 2r), r = min(r, 2l), of
 // which at most one acts; at an extremum s = 0 flattens the cell.
 __device__ __forceinline__ void ppm_magnitudes_x2(PpmWalk& c, float2 vm1, float2 v0, float2 vp1, float2 vp2, float2& s,
@@ -185,7 +186,7 @@ __device__ __forceinline__ void ppm_magnitudes_x2(PpmWalk& c, float2 vm1, float2
    const float2 fr = h4_face_x2(vm1, v0, vp1, vp2);
    const float2 right = p_minus(fr, v0), next = p_minus(vp1, fr);
    const float2 t = __fmul2_rn(right, next);
-   const bool or_x = t.x < 0.0f, or_y = t.y < 0.0f;
+   const bool or_x = !(t.x >= 0.0f), or_y = !(t.y >= 0.0f);
    const float2 lf = make_float2(c.out_x ? h.x : c.left.x, c.out_y ? h.y : c.left.y);
    const float2 rf = make_float2(or_x ? h.x : right.x, or_y ? h.y : right.y);
    const float2 l2 = __fmul2_rn(lf, f2(2.0f)), r2 = __fmul2_rn(rf, f2(2.0f));
