@@ -75,3 +75,32 @@ def test_vlasov_graph_replays_match_and_state_is_checked(vl, mesh):
                     b.replay(3)
             b.sync()
     _same(outs[0], outs[1])
+
+
+def test_a_refused_capture_leaves_the_batch_as_it_was(vl, mesh):
+    """A capture that would not end in the buffers it starts from (here: from an uploaded state) is refused; what
+    follows goes on from the state before it, its rows in use among it."""
+    import torch
+    cells = random_drifting_cells(6, seed=31)
+    gids, data = [c.gids for c in cells], [c.data for c in cells]
+    ids = torch.as_tensor(np.asarray(gids[0]).view(np.int32).copy(), device="cuda")
+    vals = torch.as_tensor(np.asarray(data[0]), device="cuda")
+    torch.cuda.synchronize()
+    outs = []
+    for refused in (False, True):
+        with vl.Batch(mesh, len(cells), 6 * sum(c.n_blocks for c in cells) + 65536) as b:
+            got = []
+            for unpack in (False, True):
+                b.upload(gids, data)
+                if refused:
+                    with pytest.raises(vl.VlgpuError):
+                        b.capture(0, "accel", [0, 1])
+                if unpack:
+                    b.unpack_cells([1], [len(gids[0])], ids.data_ptr(), vals.data_ptr())
+                    got.append(b.cells())
+                b.adjust()
+                got.append(b.cells())
+            b.sync()
+            outs.append(got)
+    for a, b in zip(*outs):
+        _same(a, b)

@@ -990,6 +990,7 @@ int vlgpu_batch_capture(vlgpu_batch* b, int slot, int kind, uint32_t n_steps, co
                                       b->adj_next, b->turn,    b->trans_turn,  kind == 1,  b->pivot_valid,
                                       false,       0,          0};
    const bool content_valid = b->content_valid;
+   const int st_list = b->st_list;
    const unsigned long long l0 = b->launches, r0 = b->remap_launches;
    VL_CHECK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeRelaxed));
    int st = VLGPU_OK;
@@ -1004,6 +1005,7 @@ int vlgpu_batch_capture(vlgpu_batch* b, int slot, int kind, uint32_t n_steps, co
    b->st_gids = start.st_gids;
    b->st_src = start.st_src;
    b->st_slots = start.st_slots;
+   b->st_list = st_list;
    b->cur = start.cur;
    b->adj_next = start.adj_next;
    b->turn = start.turn;
