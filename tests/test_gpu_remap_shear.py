@@ -147,3 +147,22 @@ def test_right_or_reported(orc_sp, dim, recon):
         assert err <= 1e-5, f"cell {c}: {err:.2e} of the peak, {isect[1:] / isect[1 + dim]}"
     # the test reaches both sides of the ring's limit
     assert clear >= len(cells) // 3 and leaning >= len(cells) // 20 and clear < len(cells)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("recon", ["ppm", "plm"])
+@pytest.mark.parametrize("cells_off", [1000, 2 ** 20, 2 ** 21 + 190, 2 ** 22 + 190, 3e9])
+def test_targets_far_above_are_reported(cells_off, recon):
+    """A column that starts many target cells above the mesh is reported, also where the number of cells times the
+    ring's slot size exceeds 32 bits and where the number itself does."""
+    from vlasiator_b200 import vlgpu
+    dv = float(MESH.dv[2])
+    gids = np.sort(MESH.gid(47, 47, np.arange(46, 49))).astype(np.uint32)
+    data = np.full((3, 64), 1e-13, F)
+    # the first source cell lies cells_off target cells above the one with index zero
+    isect = np.array([[MESH.vmin[2] + 4 * 46 * dv - cells_off * dv, 0.0, 0.0, dv]])
+    with vlgpu.Batch(MESH, 1, 4096, recon=recon) as b:
+        b.upload([gids], [data])
+        b.map_1d(isect, 2)
+        assert b.status()[0] == 3  # at the wall, and out of the ring's range
+        b.sync()

@@ -1134,10 +1134,12 @@ constexpr size_t PAIR_SMEM = (size_t)RING_CELLS * PAIR_SLOT_BYTES;
 // With S + 4 dv / dk <= 20 both are less than the ring's 32, with room for the
 // rounding of the edges.  (A step that turns by 22 degrees has 6.)
 constexpr float PAIR_LEAN = 20.0f;
-// Target cells of a column's start beyond which nothing can be right any more
-// (the mesh has 384): a start above is reported, one below counts as the
-// column's lowest target, and the slot's offset stays far from its 32 bits.
+// A column's start is cut at this many target cells (the mesh has 384): one
+// above is reported when the column ends, one below counts as the column's
+// lowest target, and the slot's offset stays far from its 32 bits.  A start
+// that a 32-bit cell index does not hold is reported on either side.
 constexpr float PAIR_FAR = 1e6f;
+constexpr float PAIR_INDEX = 2147483648.0f;
 
 // The lane's two columns of the block at `row` (data: the lane's first cell of
 // row 0): cells g = 0..3 along the sweep, .x and .y the two columns.
@@ -1367,7 +1369,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, PAIR_CTAS) remap_pair_kernel(
          // each lane's first target: the lowest g with (g+1) dk + im > v_l
          auto first_target = [&](float imc, float& gf, float& uc, uint32_t& so) {
             const float q0 = fd(fs(v_l, imc), dk);
-            range_err |= q0 > PAIR_FAR;
+            range_err |= fabsf(q0) >= PAIR_INDEX;
             int g = __float2int_rz(fminf(fmaxf(q0, -PAIR_FAR), PAIR_FAR));
             float e = fa(fm((float)(g + 1), dk), imc);
 #pragma unroll 1
